@@ -239,72 +239,85 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_bwd(const float* __restri
     }
 }
 
-// Sums the per-block head partials in a fixed order, one CTA per sum: loss ->
-// out_loss, head grads -> grads. Each thread adds the blocks b = t mod 256, then a
-// pairwise tree combines the 256 threads' sums (FP64 adds are slow on this GPU:
-// a chain as long as the block count would dominate the training step).
-constexpr int kHeadReduceThreads = 256;
-__global__ void __launch_bounds__(kHeadReduceThreads) k_head_reduce(const float* __restrict__ part, int nblocks,
-                                                                    float* __restrict__ grads_head,
-                                                                    float* __restrict__ out_loss, float invN)
+// The gradient from its partial sums, one launch: the first kHeadSums CTAs sum the
+// head's per-block partials (loss -> out_loss, head gradients), the others the
+// layers' per-CTA weight-gradient partials. FP64 adds are slow on this GPU, so no
+// chain is long: 256 strided sums and a pairwise tree for the head, four interleaved
+// sums for a weight.
+constexpr int kReduceThreads = 256;
+
+struct ReduceLayer
 {
-    const int k = blockIdx.x;  // gridDim.x == kHeadSums
+    const float* partial;  // [ctas][3 kx][cin + 1][3 ky * cout]
+    int ctas, cin, cout;
+    int block0;            // first CTA of this layer
+    float *dW, *db;        // dW[cout][cin][9], db[cout]
+};
+
+struct ReduceArgs
+{
+    ReduceLayer layer[kNumLayers];
+    const float* headPart;
+    int headBlocks;
+    float* gradsHead;
+    float* loss;
+    float invN;
+};
+
+__device__ __forceinline__ void reduce_head(const ReduceArgs& R, int k)
+{
     double acc = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += kHeadReduceThreads) acc += part[static_cast<size_t>(b) * kHeadSums + k];
-    __shared__ double sum[kHeadReduceThreads];
+    for (int b = threadIdx.x; b < R.headBlocks; b += kReduceThreads)
+        acc += R.headPart[static_cast<size_t>(b) * kHeadSums + k];
+    __shared__ double sum[kReduceThreads];
     sum[threadIdx.x] = acc;
     __syncthreads();
-    for (int h = kHeadReduceThreads / 2; h > 0; h >>= 1)
+    for (int h = kReduceThreads / 2; h > 0; h >>= 1)
     {
         if (threadIdx.x < h) sum[threadIdx.x] += sum[threadIdx.x + h];
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
     if (k == 0)
-        *out_loss = static_cast<float>(sum[0] * invN);
+        *R.loss = static_cast<float>(sum[0] * R.invN);
     else
-        grads_head[k - 1] = static_cast<float>(sum[0]);  // w[4][16], then b[4]
+        R.gradsHead[k - 1] = static_cast<float>(sum[0]);  // w[4][16], then b[4]
 }
 
-// dW[co][ci][t] = sum over CTAs of partial[gy][cta][tt][ci][co] (t = gy * tpg + tt); db from row cin.
-__global__ void k_wgrad_reduce(const float* __restrict__ partial, int gridX, int tpg, int cin, int cinReal, int cout,
-                               float* __restrict__ dW, float* __restrict__ db)
+// One thread per (kx, ci, ky, co) of a layer, co fastest as in the partials (a warp
+// reads whole lines of every partial; the scattered 4-byte writes are a single pass
+// over 120 thousand gradients), ci = cin for the bias.
+__global__ void __launch_bounds__(kReduceThreads) k_grad_reduce(const __grid_constant__ ReduceArgs R)
 {
-    const int nW = cout * cinReal * 9;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nW + cout) return;
-    int co, ci, t;
-    if (i < nW)
+    if (blockIdx.x < kHeadSums) return reduce_head(R, blockIdx.x);
+    int L = 0;
+    while (L + 1 < kNumLayers && static_cast<int>(blockIdx.x) >= R.layer[L + 1].block0) ++L;
+    const ReduceLayer& a = R.layer[L];
+    const int rows = 3 * a.cout, n = 3 * (a.cin + 1) * rows;
+    const int i = (blockIdx.x - a.block0) * kReduceThreads + threadIdx.x;
+    if (i >= n) return;
+    const int row = i % rows, q = i / rows;
+    const int ci = q % (a.cin + 1), kx = q / (a.cin + 1);
+    const int co = row % a.cout, ky = row / a.cout;
+    if (ci == a.cin && (kx != 1 || ky != 1)) return;
+    const float* src = a.partial + i;
+    const size_t stride = static_cast<size_t>(n);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    int c = 0;
+    for (; c + 16 <= a.ctas; c += 16)
     {
-        co = i / (cinReal * 9);
-        const int r = i - co * cinReal * 9;
-        ci = r / 9;
-        t = r - ci * 9;
-    }
-    else
-    {
-        co = i - nW;
-        ci = cin;  // bias row
-        t = 0;
-    }
-    const int gy = t / tpg, tt = t - gy * tpg;
-    // 8 interleaved FP64 sums (CTA bx into sum bx mod 8), then combined pairwise:
-    // a dependent chain of gridX / 8 + 3 adds instead of gridX
-    double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const size_t stride = static_cast<size_t>(tpg) * (cin + 1) * cout;
-    const float* src = partial + ((static_cast<size_t>(gy) * gridX * tpg + tt) * (cin + 1) + ci) * cout + co;
-    int bx = 0;
-    for (; bx + 8 <= gridX; bx += 8)
-    {
+        float v[16];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] += src[(bx + j) * stride];
+        for (int j = 0; j < 16; ++j) v[j] = src[(c + j) * stride];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j & 3] += v[j];
     }
-    for (int j = 0; bx + j < gridX; ++j) acc[j] += src[(bx + j) * stride];
-    const double total = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-    if (i < nW)
-        dW[i] = static_cast<float>(total);
+    for (; c < a.ctas; ++c) acc[c & 3] += src[c * stride];
+    const float total = static_cast<float>((acc[0] + acc[1]) + (acc[2] + acc[3]));
+    if (ci < a.cin)
+        a.dW[(co * a.cin + ci) * 9 + ky * 3 + kx] = total;
     else
-        db[co] = static_cast<float>(total);
+        a.db[co] = total;
 }
 
 // PyTorch's Adam: m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2;
@@ -693,38 +706,79 @@ int conv(fr_aonet* n, const Shape& S, int lv, const uint16_t* in0, int c0, const
     return FR_OK;
 }
 
-// Weight gradient of layer L from its input X (one or two tensors) and its output gradient dY.
-int wgrad(fr_aonet* n, const Shape& S, int L, const uint16_t* x0, const uint16_t* x1, const uint16_t* dY,
-          cudaStream_t st)
+// One layer's part of the weight-gradient launch: X (one or two tensors) and the
+// output gradient dY. Its CTAs and partial sums follow in wgrad_all.
+int wgrad_layer(fr_aonet* n, const Shape& S, int layer, const uint16_t* x0, const uint16_t* x1, const uint16_t* dY,
+                WgradLayer& L)
 {
-    const LayerSpec& s = kLayers[L];
-    const int lv = s.level;
-    const int H = S.h(lv), W = S.w(lv);
-    CUtensorMap mx0, mx1, mdy;
-    if (!make_cp_map(&mx0, x0, s.c0, S.B, H, W, kHaloW, kHaloH) ||
-        (s.c1 > 0 && !make_cp_map(&mx1, x1, s.c1, S.B, H, W, kHaloW, kHaloH)) ||
-        !make_cp_map(&mdy, dY, s.cout, S.B, H, W, kTileW, kTileH))
+    const LayerSpec& s = kLayers[layer];
+    const int H = S.h(s.level), W = S.w(s.level);
+    if (!make_cp_map(&L.mapX0, x0, s.c0, S.B, H, W, kHaloW, kTileH) ||
+        (s.c1 > 0 && !make_cp_map(&L.mapX1, x1, s.c1, S.B, H, W, kHaloW, kTileH)) ||
+        !make_cp_map(&L.mapDY, dY, s.cout, S.B, H, W, kTileW, kTileH))
         return net_fail(n, FR_ERR_CUDA, "tensor map encode");
-    if (s.c1 == 0) mx1 = mx0;
-    WgradArgs a{};
-    a.B = S.B, a.H = H, a.W = W;
-    a.tilesX = (W + kTileW - 1) / kTileW;
-    a.tilesY = (H + kTileH - 1) / kTileH;
-    a.numTiles = S.B * a.tilesX * a.tilesY;
-    a.c0 = s.c0, a.c1 = s.c1, a.cout = s.cout;
-    a.tapsPerGroup = s.cout == 64 ? 5 : 9;
-    const int gridY = (9 + a.tapsPerGroup - 1) / a.tapsPerGroup;
-    const int gridX = std::min(a.numTiles, n->numSMs);
-    const int cin = s.c0 + s.c1;
-    const size_t need = static_cast<size_t>(gridY) * gridX * a.tapsPerGroup * (cin + 1) * s.cout;
-    if (need > n->partialCap) return net_fail(n, FR_ERR_INVALID, "wgrad partial buffer too small");
-    a.partial = n->partial;
-    a.status = n->status;
-    launch_wgrad(mx0, mx1, mdy, a, gridX, gridY, wgrad_smem_bytes(s.cout), st);
-    const int nOut = w_count(L) + s.cout;
-    k_wgrad_reduce<<<blocks_for(nOut, 256), 256, 0, st>>>(n->partial, gridX, a.tapsPerGroup, cin, s.cinReal, s.cout,
-                                                          n->grads + n->paramOff[L],
-                                                          n->grads + n->paramOff[L] + w_count(L));
+    if (s.c1 == 0) L.mapX1 = L.mapX0;
+    L.tilesX = (W + kTileW - 1) / kTileW;
+    L.tilesY = (H + kTileH - 1) / kTileH;
+    L.numTiles = S.B * L.tilesX * L.tilesY;
+    L.c0 = s.c0, L.c1 = s.c1, L.cout = s.cout;
+    const uint32_t stage = wgrad_stage_bytes(s.c0 + s.c1, s.cout), window = wgrad_a_window(s.cout);
+    L.stages = kMaxStages;
+    while (L.stages > 2 && (L.stages - 1) * stage + std::max(stage, window) > kWgradSmem) --L.stages;
+    L.sets = std::min(4, 512 / wgrad_set_cols(s.c0 + s.c1, s.cout));
+    return FR_OK;
+}
+
+// The weight gradients of every layer (k_wgrad, k_grad_reduce) and the head's sums.
+int wgrad_all(fr_aonet* n, const WgradLayer* layers, int headBlocks, float invN, cudaStream_t st)
+{
+    WgradArgs U{};
+    U.nLayers = kNumLayers;
+    U.status = n->status;
+    // A CTA takes an even share of one wave's MMAs, or fewer tiles where its accumulator
+    // sets hold no more than kWgradChain tiles each; the CTAs with the most work first,
+    // so that those beyond the first wave are short.
+    auto blocks = [&](int L) { return (3 * kLayers[L].cout + 127) / 128; };
+    long long work = 0;
+    for (int L = 0; L < kNumLayers; ++L) work += static_cast<long long>(layers[L].numTiles) * blocks(L);
+    const long long share = std::max(1LL, (work + n->numSMs - 1) / n->numSMs);
+    auto tiles = [&](int L) { return std::min(std::max(share / blocks(L), 1LL), 1LL * kWgradChain * layers[L].sets); };
+    int order[kNumLayers];
+    for (int L = 0; L < kNumLayers; ++L) order[L] = L;
+    std::stable_sort(order, order + kNumLayers,
+                     [&](int p, int q) { return tiles(p) * blocks(p) > tiles(q) * blocks(q); });
+    ReduceArgs R{};
+    size_t need = 0;
+    int grid = 0, rblocks = kHeadSums;
+    size_t at[kNumLayers];
+    for (int i = 0; i < kNumLayers; ++i)
+    {
+        const int L = order[i];
+        WgradLayer& w = U.layer[i];
+        w = layers[L];
+        const int cin = w.c0 + w.c1;
+        w.cta0 = grid;
+        w.ctas = static_cast<int>((w.numTiles + tiles(L) - 1) / tiles(L));
+        grid += w.ctas;
+        at[i] = need;
+        need += w.ctas * wgrad_partial_floats(cin, w.cout);
+        R.layer[i] = ReduceLayer{nullptr, w.ctas, cin, w.cout, rblocks, n->grads + n->paramOff[L],
+                                 n->grads + n->paramOff[L] + w_count(L)};
+        rblocks += blocks_for(9LL * (cin + 1) * w.cout, kReduceThreads);
+    }
+    if (need > n->partialCap)
+    {
+        cudaFree(n->partial);  // waits for earlier steps
+        n->partial = nullptr, n->partialCap = 0;
+        NET_CUDA(n, cudaMalloc(&n->partial, sizeof(float) * need));
+        n->partialCap = need;
+    }
+    for (int i = 0; i < kNumLayers; ++i) R.layer[i].partial = U.layer[i].partial = n->partial + at[i];
+    R.headPart = n->headPart, R.headBlocks = headBlocks;
+    R.gradsHead = n->grads + n->paramOff[kNumLayers];
+    R.loss = n->lossDev, R.invN = invN;
+    launch_wgrad(U, grid, st);
+    k_grad_reduce<<<rblocks, kReduceThreads, 0, st>>>(R);
     n->launches += 2;
     return FR_OK;
 }
@@ -862,46 +916,49 @@ int backward_impl(fr_aonet* n, const uint16_t* in, const float* label, const Sha
     k_head_bwd<<<hb, kHeadThreads, 0, st>>>(n->aoTmp, label, reinterpret_cast<const uint4*>(n->a7),
                                             n->params + n->paramOff[kNumLayers], reinterpret_cast<uint4*>(n->g7),
                                             n->headPart, S.B, S.H, S.W, invN);
-    k_head_reduce<<<kHeadSums, kHeadReduceThreads, 0, st>>>(n->headPart, hb, n->grads + n->paramOff[kNumLayers],
-                                                           n->lossDev, invN);
-    n->launches += 2;
+    n->launches++;
+    WgradLayer wg[kNumLayers];
+    auto WG = [&](int L, const uint16_t* x0, const uint16_t* x1, const uint16_t* dy) {
+        return wgrad_layer(n, S, L, x0, x1, dy, wg[L]);
+    };
     // level 0 decoder
-    NET_TRY(wgrad(n, S, 9, n->a6, nullptr, n->g7, st));
+    NET_TRY(WG(9, n->a6, nullptr, n->g7));
     NET_TRY(DG(9, n->g7, n->g6, 16, nullptr, n->a6));
-    NET_TRY(wgrad(n, S, 8, n->u0, n->s0, n->g6, st));
+    NET_TRY(WG(8, n->u0, n->s0, n->g6));
     NET_TRY(DG(8, n->g6, n->gu0, 32, n->gs0c, nullptr));
     k_up_bwd_mask<<<blocks_for((long long)S.B * 4 * S.h(1) * S.w(1), 256), 256, 0, st>>>(
         reinterpret_cast<const uint4*>(n->gu0), reinterpret_cast<const uint4*>(n->a5), reinterpret_cast<uint4*>(n->g5),
         S.B * 4, S.h(1), S.w(1));
     // level 1 decoder
-    NET_TRY(wgrad(n, S, 7, n->a4, nullptr, n->g5, st));
+    NET_TRY(WG(7, n->a4, nullptr, n->g5));
     NET_TRY(DG(7, n->g5, n->g4, 32, nullptr, n->a4));
-    NET_TRY(wgrad(n, S, 6, n->u1, n->s1, n->g4, st));
+    NET_TRY(WG(6, n->u1, n->s1, n->g4));
     NET_TRY(DG(6, n->g4, n->gu1, 64, n->gs1c, nullptr));
     k_up_bwd_mask<<<blocks_for((long long)S.B * 8 * S.h(2) * S.w(2), 256), 256, 0, st>>>(
         reinterpret_cast<const uint4*>(n->gu1), reinterpret_cast<const uint4*>(n->a3), reinterpret_cast<uint4*>(n->g3),
         S.B * 8, S.h(2), S.w(2));
     // bottleneck
-    NET_TRY(wgrad(n, S, 5, n->a2, nullptr, n->g3, st));
+    NET_TRY(WG(5, n->a2, nullptr, n->g3));
     NET_TRY(DG(5, n->g3, n->g2, 64, nullptr, n->a2));
-    NET_TRY(wgrad(n, S, 4, n->p1, nullptr, n->g2, st));
+    NET_TRY(WG(4, n->p1, nullptr, n->g2));
     NET_TRY(DG(4, n->g2, n->gp1, 32, nullptr, nullptr));
     k_pool_bwd_add_mask<<<blocks_for((long long)S.B * 4 * S.h(1) * S.w(1), 256), 256, 0, st>>>(
         reinterpret_cast<const uint4*>(n->gs1c), reinterpret_cast<const uint4*>(n->gp1),
         reinterpret_cast<const uint4*>(n->s1), reinterpret_cast<uint4*>(n->gS1), S.B * 4, S.h(1), S.w(1));
     // level 1 encoder
-    NET_TRY(wgrad(n, S, 3, n->a1, nullptr, n->gS1, st));
+    NET_TRY(WG(3, n->a1, nullptr, n->gS1));
     NET_TRY(DG(3, n->gS1, n->g1, 32, nullptr, n->a1));
-    NET_TRY(wgrad(n, S, 2, n->p0, nullptr, n->g1, st));
+    NET_TRY(WG(2, n->p0, nullptr, n->g1));
     NET_TRY(DG(2, n->g1, n->gp0, 16, nullptr, nullptr));
     k_pool_bwd_add_mask<<<blocks_for((long long)S.B * 2 * S.H * S.W, 256), 256, 0, st>>>(
         reinterpret_cast<const uint4*>(n->gs0c), reinterpret_cast<const uint4*>(n->gp0),
         reinterpret_cast<const uint4*>(n->s0), reinterpret_cast<uint4*>(n->gS0), S.B * 2, S.H, S.W);
     // level 0 encoder
-    NET_TRY(wgrad(n, S, 1, n->a0, nullptr, n->gS0, st));
+    NET_TRY(WG(1, n->a0, nullptr, n->gS0));
     NET_TRY(DG(1, n->gS0, n->g0, 16, nullptr, n->a0));
-    NET_TRY(wgrad(n, S, 0, n->xs, nullptr, n->g0, st));
-    n->launches += 3;
+    NET_TRY(WG(0, n->xs, nullptr, n->g0));
+    n->launches += 4;
+    NET_TRY(wgrad_all(n, wg, hb, invN, st));
     NET_CUDA(n, cudaGetLastError());
     return FR_OK;
 }
@@ -1023,17 +1080,6 @@ fr_aonet* fr_aonet_create(int32_t device, uint64_t seed, char* err, size_t errle
         ok = cudaMalloc(&n->packFwd[L], n->packFwdBytes[L]) == cudaSuccess;
         if (ok && L > 0) ok = cudaMalloc(&n->packBwd[L], 9u * cin * sp.cout * 2u) == cudaSuccess;
     }
-    // wgrad partials: the largest layer's gridY * SMs * taps * (cin + 1) * cout
-    size_t cap = 0;
-    for (int L = 0; L < kNumLayers; ++L)
-    {
-        const LayerSpec& sp = kLayers[L];
-        const int tpg = sp.cout == 64 ? 5 : 9;
-        const int gy = (9 + tpg - 1) / tpg;
-        cap = std::max(cap, static_cast<size_t>(gy) * n->numSMs * tpg * (sp.c0 + sp.c1 + 1) * sp.cout);
-    }
-    if (ok) ok = cudaMalloc(&n->partial, sizeof(float) * cap) == cudaSuccess;
-    n->partialCap = cap;
     if (ok)
         ok = cudaMemcpy(n->params, h.data(), sizeof(float) * kNumParams, cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemset(n->grads, 0, sizeof(float) * kNumParams) == cudaSuccess &&

@@ -529,106 +529,110 @@ __global__ void __launch_bounds__(192, 1) k_unet_fwd(const __grid_constant__ Une
     }
 }
 
-__global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorMap mapX0,
-                                               const __grid_constant__ CUtensorMap mapX1,
-                                               const __grid_constant__ CUtensorMap mapDY, const WgradArgs a)
+// Every layer's weight gradient in one launch (WgradArgs). A tile is 8 x 16 pixels
+// of X rows and output columns: dY is loaded at rows y0 + 1, y0, y0 - 1 (ky = 0, 1,
+// 2; the TMA zero fill stands for pixels outside the image), so rows (ky, co) of
+// the A operand are adjacent planes, and X with one extra pixel on either side, so
+// kx is a start address 16 bytes further. 24 MMAs (48 for 64 output channels) cover
+// the nine taps of a tile; one M = 128 MMA per tap took 72, each mostly fetching
+// rows of zeros. Bound by the MMAs' A fetch (about 40 cycles each). The CTAs are
+// shared out among the layers by their MMA count, so a step needs about one wave and
+// few partial sums: with one launch of 152 CTAs per layer the ten launches took 301 us
+// at 16 x 256 x 256 and left 152 partials per weight to add up (425 us).
+__global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs U)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ SyncState sy;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cin = a.c0 + a.c1;
-    constexpr uint32_t xBytes = kWgradXPlanes * kPlaneBytes;  // 46080 = 45 KiB
-    const uint32_t dyPlane = kTileW * kTileH * 16;            // 2048
-    const uint32_t dyBytes = static_cast<uint32_t>(a.cout / 8) * dyPlane;
-    const uint32_t stageBytes = xBytes + 8 * dyPlane;         // room for cout = 64
-    const int t0 = blockIdx.y * a.tapsPerGroup;
-    const int nt = min(a.tapsPerGroup, 9 - t0);
-    const uint32_t allocCols = tmem_cols(a.tapsPerGroup * a.cout);
+    int L = 0;
+    while (L + 1 < U.nLayers && static_cast<int>(blockIdx.x) >= U.layer[L + 1].cta0) ++L;
+    const WgradLayer& a = U.layer[L];
+    const int k0 = blockIdx.x - a.cta0;
+    const int cin = a.c0 + a.c1, cout = a.cout;
+    const int nCols = cin + 16;                      // X channels, the ones column, padding
+    const int mBlocks = (3 * cout + 127) / 128;
+    const uint32_t yBytes = static_cast<uint32_t>(cout / 8) * kWgradYPlane;  // one dY copy
+    const uint32_t stageBytes = wgrad_stage_bytes(cin, cout);
+    const int setCols = wgrad_set_cols(cin, cout);
+    const uint32_t allocCols = tmem_cols(a.sets * setCols);
 
-    // Planes cin/8 .. 15 of every X stage are constant: plane cin/8 holds 1.0 in
-    // channel 0 (its accumulator row is the bias gradient), the rest are zero.
-    for (int s = 0; s < kWgradStages; ++s)
+    // The planes cin/8 and cin/8 + 1 of every X stage are constant: 1.0 in channel 0
+    // (its accumulator column is the bias gradient), else zero.
+    for (int s = 0; s < a.stages; ++s)
     {
-        uint32_t* p = reinterpret_cast<uint32_t*>(smem + s * stageBytes + (cin / 8) * kPlaneBytes);
-        const int words = (kWgradXPlanes - cin / 8) * kPlaneBytes / 4;
-        for (int i = threadIdx.x; i < words; i += blockDim.x)
-            p[i] = (i < kPlaneBytes / 4 && (i & 3) == 0) ? 0x3F80u : 0u;
+        uint32_t* p = reinterpret_cast<uint32_t*>(smem + s * stageBytes + 3 * yBytes + (cin / 8) * kWgradXPlane);
+        for (int i = threadIdx.x; i < 2 * kWgradXPlane / 4; i += blockDim.x)
+            p[i] = (i < kWgradXPlane / 4 && (i & 3) == 0) ? 0x3F80u : 0u;
     }
     frtc::fence_proxy_async_smem();
-    if (threadIdx.x == 0)
-    {
-        for (int s = 0; s < kMaxStages; ++s)
-        {
-            frtc::mbar_init(&sy.full[s], 1);
-            frtc::mbar_init(&sy.empty[s], 1);
-        }
-        frtc::mbar_init(&sy.done, 1);
-        sy.abort = 0;
-        frtc::fence_mbar_init();
-    }
+    init_sync(sy);
     if (warp == 1) frtc::tmem_alloc(&sy.tmem, allocCols);
     frtc::tc_fence_before();
     __syncthreads();
     frtc::tc_fence_after();
     const uint32_t tmem = sy.tmem;
     volatile int* abortp = &sy.abort;
-    const int ntiles = blockIdx.x < a.numTiles ? (a.numTiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
     if (warp == 0)
     {
         if (lane == 0)
         {
-            const uint32_t loadBytes = static_cast<uint32_t>(cin / 8) * kPlaneBytes + dyBytes;
+            const uint32_t loadBytes = 3 * yBytes + static_cast<uint32_t>(cin / 8) * kWgradXPlane;
             int issued = 0;
-            for (int tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, ++issued)
+            for (int tile = k0; tile < a.numTiles; tile += a.ctas, ++issued)
             {
-                const int s = issued % kWgradStages;
-                const uint32_t ph = (issued / kWgradStages) & 1;
-                if (issued >= kWgradStages && !wait_or_abort(&sy.empty[s], ph ^ 1, abortp, a.status)) break;
+                const int s = issued % a.stages;
+                const uint32_t ph = (issued / a.stages) & 1;
+                if (issued >= a.stages && !wait_or_abort(&sy.empty[s], ph ^ 1, abortp, U.status)) break;
                 int b, tx, ty;
                 decode_tile(tile, a.tilesX, a.tilesY, b, tx, ty);
                 unsigned char* dst = smem + s * stageBytes;
                 frtc::mbar_expect_tx(&sy.full[s], loadBytes);
-                frtc::tma_load_3d(dst, &mapX0, 8 * (tx * kTileW - 1), ty * kTileH - 1, b * (a.c0 / 8), &sy.full[s]);
+                for (int ky = 0; ky < 3; ++ky)
+                    frtc::tma_load_3d(dst + ky * yBytes, &a.mapDY, 8 * tx * kTileW, ty * kTileH + 1 - ky,
+                                      b * (cout / 8), &sy.full[s]);
+                dst += 3 * yBytes;
+                frtc::tma_load_3d(dst, &a.mapX0, 8 * (tx * kTileW - 1), ty * kTileH, b * (a.c0 / 8), &sy.full[s]);
                 if (a.c1)
-                    frtc::tma_load_3d(dst + (a.c0 / 8) * kPlaneBytes, &mapX1, 8 * (tx * kTileW - 1), ty * kTileH - 1,
+                    frtc::tma_load_3d(dst + (a.c0 / 8) * kWgradXPlane, &a.mapX1, 8 * (tx * kTileW - 1), ty * kTileH,
                                       b * (a.c1 / 8), &sy.full[s]);
-                frtc::tma_load_3d(dst + xBytes, &mapDY, 8 * tx * kTileW, ty * kTileH, b * (a.cout / 8), &sy.full[s]);
             }
-            for (int i = issued - kWgradStages; i < issued; ++i)
-                if (i >= 0) frtc::mbar_wait(&sy.full[i % kWgradStages], (i / kWgradStages) & 1, kWaitNs);
+            // every issued copy lands before the CTA exits
+            for (int i = issued - a.stages; i < issued; ++i)
+                if (i >= 0) frtc::mbar_wait(&sy.full[i % a.stages], (i / a.stages) & 1, kWaitNs);
         }
     }
     else if (warp == 1)
     {
         if (lane == 0)
         {
-            const uint32_t idesc = frtc::idesc_bf16_f32(128, a.cout, 1, 1);
+            const uint32_t idesc = frtc::idesc_bf16_f32(128, nCols, 1, 1);
+            // both operands MN-major: K core matrices (8 pixels of a row) one row apart,
+            // groups of 8 rows / columns (channels) one plane apart
+            constexpr uint64_t aHi = frtc::smem_desc_hi(128u, kWgradYPlane);
+            constexpr uint64_t bHi = frtc::smem_desc_hi(kWgradXRowBytes, kWgradXPlane);
             int it = 0;
-            for (int tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x, ++it)
+            for (int tile = k0; tile < a.numTiles; tile += a.ctas, ++it)
             {
-                const int s = it % kWgradStages;
-                if (!wait_or_abort(&sy.full[s], (it / kWgradStages) & 1, abortp, a.status)) break;
+                const int s = it % a.stages;
+                if (!wait_or_abort(&sy.full[s], (it / a.stages) & 1, abortp, U.status)) break;
                 frtc::tc_fence_after();
-                const uint32_t xb = frtc::smem_u32(smem + s * stageBytes);
-                const uint32_t yb = xb + xBytes;
-                constexpr uint64_t aHi = frtc::smem_desc_hi(kRowBytes, kPlaneBytes);
-                const uint64_t bHi = frtc::smem_desc_hi(128u, dyPlane);
-                for (int tt = 0; tt < nt; ++tt)
-                {
-                    const int t = t0 + tt;
-                    const uint32_t d = tmem + static_cast<uint32_t>(tt * a.cout);
-                    const uint32_t aTap = xb + static_cast<uint32_t>(((t / 3) * kHaloW + (t % 3)) * 16);
-#pragma unroll
-                    for (int j = 0; j < kTileH / 2; ++j)
+                const uint32_t yb = frtc::smem_u32(smem + s * stageBytes);
+                const uint32_t xb = yb + 3 * yBytes;
+                const uint32_t set = tmem + static_cast<uint32_t>((it % a.sets) * setCols);
+                const uint32_t more = it >= a.sets;  // the set already holds earlier tiles
+                for (int m = 0; m < mBlocks; ++m)
+                    for (int kx = 0; kx < 3; ++kx)
                     {
-                        // A: rows = input channels (MN-major), K = 16 pixels = halo rows 2j+dy, 2j+1+dy.
-                        const uint64_t ad = aHi | ((aTap + static_cast<uint32_t>(2 * j * kRowBytes)) >> 4);
-                        // B: rows = output channels (MN-major), K = the same 16 output pixels.
-                        const uint64_t bd = bHi | ((yb + static_cast<uint32_t>(2 * j) * 128u) >> 4);
-                        frtc::mma_bf16(d, ad, bd, idesc, (it | j) != 0);
+                        const uint32_t d = set + static_cast<uint32_t>((m * 3 + kx) * nCols);
+                        const uint32_t ya = yb + static_cast<uint32_t>(m * 16 * kWgradYPlane);
+                        const uint32_t xa = xb + static_cast<uint32_t>(kx * 16);
+#pragma unroll
+                        for (int j = 0; j < kTileH / 2; ++j)  // K = 16 pixels: two tile rows
+                            frtc::mma_bf16(d, aHi | ((ya + static_cast<uint32_t>(j * 256)) >> 4),
+                                           bHi | ((xa + static_cast<uint32_t>(j * 2 * kWgradXRowBytes)) >> 4), idesc,
+                                           more | static_cast<uint32_t>(j));
                     }
-                }
                 frtc::mma_commit(&sy.empty[s]);
             }
             frtc::mma_commit(&sy.done);
@@ -638,27 +642,38 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ CUtensorM
     else
     {
         const int q = warp & 3;
-        const int row = q * 32 + lane;  // input channel (row cin: bias)
         int ok = 1;
-        if (lane == 0) ok = wait_or_abort(&sy.done, 0, abortp, a.status);
+        if (lane == 0) ok = wait_or_abort(&sy.done, 0, abortp, U.status);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         frtc::tc_fence_after();
-        const size_t base =
-            ((static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * a.tapsPerGroup) * (cin + 1);
-        for (int tt = 0; tt < nt; ++tt)
-            for (int g = 0; g < a.cout / 16; ++g)
-            {
-                float v[16];
-                frtc::tmem_ld16(tmem + (static_cast<uint32_t>(q * 32) << 16) +
-                                    static_cast<uint32_t>(tt * a.cout + g * 16),
-                                v);
-                if (row <= cin)
+        const int used = min(a.sets, (a.numTiles - 1 - k0) / a.ctas + 1);  // every CTA has a tile
+        float* part = a.partial + static_cast<size_t>(k0) * wgrad_partial_floats(cin, cout);
+        for (int m = 0; m < mBlocks; ++m)
+        {
+            const int row = m * 128 + q * 32 + lane;  // ky * cout + co
+            for (int kx = 0; kx < 3; ++kx)
+                for (int g = 0; g < nCols / 16; ++g)
                 {
-                    float* dst = a.partial + ((base + static_cast<size_t>(tt) * (cin + 1) + row) * a.cout + g * 16);
+                    const uint32_t at = tmem + (static_cast<uint32_t>(q * 32) << 16) +
+                                        static_cast<uint32_t>((m * 3 + kx) * nCols + g * 16);
+                    float v[16];
+                    frtc::tmem_ld16(at, v);
+                    for (int e = 1; e < used; ++e)
+                    {
+                        float w[16];
+                        frtc::tmem_ld16(at + static_cast<uint32_t>(e * setCols), w);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) dst[i] = (ok && ntiles > 0) ? v[i] : 0.f;
+                        for (int i = 0; i < 16; ++i) v[i] += w[i];
+                    }
+                    if (row >= 3 * cout) continue;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                    {
+                        const int ci = g * 16 + i;
+                        if (ci <= cin) part[(static_cast<size_t>(kx) * (cin + 1) + ci) * (3 * cout) + row] = ok ? v[i] : 0.f;
+                    }
                 }
-            }
+        }
     }
     frtc::tc_fence_before();
     __syncthreads();
@@ -682,11 +697,6 @@ uint32_t conv_smem_bytes(int cin, int cout, int stages, bool paired, int mb)
     const uint32_t plane = static_cast<uint32_t>(kHaloW * (kTileH * mb + 2) * 16);
     const uint32_t stage = (static_cast<uint32_t>(cin / 8) * plane + 1023u) & ~1023u;
     return w + stage * stages;
-}
-
-uint32_t wgrad_smem_bytes(int /*cout*/)
-{
-    return kWgradStages * (kWgradXPlanes * kPlaneBytes + 8 * kTileW * kTileH * 16);
 }
 
 void launch_conv3x3(const CUtensorMap& map0, const CUtensorMap& map1, const ConvArgs& a, int grid, uint32_t smem,
@@ -745,8 +755,7 @@ cudaError_t launch_unet_fwd(const UnetArgs& u, int grid, uint32_t smem, cudaStre
     return cudaLaunchKernelEx(&cfg, k_unet_fwd, u);
 }
 
-void launch_wgrad(const CUtensorMap& mapX0, const CUtensorMap& mapX1, const CUtensorMap& mapDY, const WgradArgs& a,
-                  int gridX, int gridY, uint32_t smem, cudaStream_t st)
+void launch_wgrad(const WgradArgs& a, int grid, cudaStream_t st)
 {
     static bool attr = false;
     if (!attr)
@@ -754,7 +763,7 @@ void launch_wgrad(const CUtensorMap& mapX0, const CUtensorMap& mapX1, const CUte
         cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
         attr = true;
     }
-    k_wgrad<<<dim3(gridX, gridY), 192, smem, st>>>(mapX0, mapX1, mapDY, a);
+    k_wgrad<<<grid, 192, kWgradSmem, st>>>(a);
 }
 
 }  // namespace fra

@@ -51,16 +51,52 @@ struct ConvArgs
     int* status;         // bit 1: a pipeline wait timed out
 };
 
+// ---- weight gradients of every layer in one launch -------------------------------
+// dW[co][ci][ky][kx] = sum_p dY[co][p] X[ci][p + (ky - 1, kx - 1)] as one GEMM per
+// layer whose K runs over pixels: the rows are (ky, co) - dY read three times, one
+// row up, level and down - and the columns are input channels, the three kx being
+// three column blocks read from one X tile at three start addresses.
+constexpr int kWgradMaxLayers = 10;
+constexpr int kWgradXRowBytes = kHaloW * 16;                 // 160: an X row of a tile, 10 pixels
+constexpr int kWgradXPlane = kTileH * kWgradXRowBytes;       // 2560: 8 channels of a tile's X
+constexpr int kWgradYPlane = kTileW * kTileH * 16;           // 2048: 8 channels of a tile's dY
+constexpr uint32_t kWgradSmem = 184u * 1024u;                // one CTA per SM, 2..4 stages
+
+struct WgradLayer
+{
+    CUtensorMap mapX0, mapX1, mapDY;
+    int tilesX, tilesY, numTiles;
+    int c0, c1;          // X channels from mapX0 / mapX1; cin = c0 + c1 <= 96
+    int cout;            // dY channels: 16, 32 or 64
+    int stages;          // shared-memory pipeline depth
+    int sets;            // accumulator sets in TMEM: tile i of a CTA adds to set i % sets
+    int cta0, ctas;      // the CTAs [cta0, cta0 + ctas) share this layer's tiles
+    float* partial;      // [ctas][3 kx][cin + 1][3 ky * cout]; row cin: the bias (ky = kx = 1)
+};
+
 struct WgradArgs
 {
-    int B, H, W;
-    int tilesX, tilesY, numTiles;
-    int c0, c1;          // X channels from map0 / map1; cin = c0 + c1 <= 120
-    int cout;            // dY channels: 16, 32 or 64
-    int tapsPerGroup;    // taps handled by one blockIdx.y group
-    float* partial;      // [gridDim.y][gridDim.x][tapsPerGroup][cin + 1][cout]
+    WgradLayer layer[kWgradMaxLayers];
+    int nLayers;
     int* status;
 };
+
+// Bytes of one pipeline stage of a layer (dY three times, X, the ones and zero planes).
+constexpr uint32_t wgrad_stage_bytes(int cin, int cout)
+{
+    return static_cast<uint32_t>(3 * (cout / 8) * kWgradYPlane + (cin / 8 + 2) * kWgradXPlane);
+}
+// The A operand's 128-row blocks (16 planes each) are read whole, past the 3 * cout
+// valid rows: the last stage needs this much shared memory behind its start.
+constexpr uint32_t wgrad_a_window(int cout) { return static_cast<uint32_t>((3 * cout + 127) / 128 * 16 * kWgradYPlane); }
+// TMEM columns of one accumulator set: three kx of (cin + 16) columns, per row block.
+constexpr int wgrad_set_cols(int cin, int cout) { return 3 * ((3 * cout + 127) / 128) * (cin + 16); }
+// The tensor core's FP32 accumulation loses a little in every add, always downwards:
+// at most this many tiles (8 adds each) go into one accumulator, and the sets and
+// the CTAs' partial sums are then added in FP32 and FP64 with rounding to nearest.
+constexpr int kWgradChain = 16;
+// Floats of one CTA's partial sums.
+constexpr size_t wgrad_partial_floats(int cin, int cout) { return static_cast<size_t>(9) * (cin + 1) * cout; }
 
 // ---- fused forward: the whole network in one cooperative launch ------------------
 // Stages run in order with a grid-wide barrier after each: a convolution (its
@@ -112,15 +148,11 @@ int unet_fwd_ctas_per_sm(uint32_t smem);
 
 // Shared-memory bytes of one launch.
 uint32_t conv_smem_bytes(int cin, int cout, int stages, bool paired, int mb);
-uint32_t wgrad_smem_bytes(int cout);
-constexpr int kWgradStages = 2;
-constexpr int kWgradXPlanes = 16;  // M = 128 rows = 16 planes of 8 channels
 
 // programmatic: launch as a programmatic dependent of the stream's previous
 // kernel (the prologue overlaps its tail; outputs are read after griddepcontrol.wait).
 void launch_conv3x3(const CUtensorMap& map0, const CUtensorMap& map1, const ConvArgs& a, int grid,
                     uint32_t smem, cudaStream_t st, bool programmatic);
-void launch_wgrad(const CUtensorMap& mapX0, const CUtensorMap& mapX1, const CUtensorMap& mapDY, const WgradArgs& a,
-                  int gridX, int gridY, uint32_t smem, cudaStream_t st);
+void launch_wgrad(const WgradArgs& a, int grid, cudaStream_t st);
 
 }  // namespace fra

@@ -107,6 +107,43 @@ def test_gradients_match_oracle():
         assert rel < 3e-2, (name, rel)
 
 
+@pytest.mark.parametrize("shape", [(1, 32, 32), (3, 96, 160), (2, 256, 256)])
+def test_weight_gradients_over_shapes(shape):
+    """The one-launch weight gradients where their split changes: a single partial
+    tile per level, ragged tiles on every level, and several tiles per CTA in more
+    accumulator sets than one. Against the oracle as above; and the batch's
+    gradient against the mean of its images' gradients, which (batches of 1, 2 and 4
+    scale by powers of two) round alike up to the FP32 accumulation: at most 16 tiles
+    of 8 adds in one accumulator, each off by at most 2^-23, so 1.6e-5 of the sums;
+    1e-4 leaves room for cancellation."""
+    _need_gpu()
+    import aonet_ref as R
+    from forkerrenderer_gb300.aonet import AONet
+
+    B, H, W = shape
+    rng = np.random.default_rng(B * H + W)
+    net = AONet(0, seed=7)
+    bits, x4 = _batch(rng, B, H, W)
+    label = rng.uniform(0.1, 0.95, (B, H, W)).astype(np.float32)
+    net.backward(_dev(bits.view(np.int16)), _dev(label), B, H, W)
+    g = net.get_grads()
+    ref_net = R.Net(net.get_params())
+    ref_net.forward(x4)
+    _, gref = ref_net.backward(label)
+    for name, sl in _layer_slices():
+        a, b = g[sl].astype(np.float64), gref[sl]
+        rel = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12)
+        assert rel < 3e-2, (name, rel)
+    if B in (2, 4):
+        mean = np.zeros(g.size)
+        for i in range(B):
+            net.backward(_dev(bits[i:i + 1].view(np.int16)), _dev(label[i:i + 1]), 1, H, W)
+            mean += net.get_grads().astype(np.float64) / B
+        for name, sl in _layer_slices():
+            rel = np.linalg.norm(g[sl] - mean[sl]) / max(np.linalg.norm(mean[sl]), 1e-12)
+            assert rel < 1e-4, (name, rel)
+
+
 def test_adam_step_matches_oracle():
     _need_gpu()
     import aonet_ref as R
