@@ -3,7 +3,7 @@
 //
 // Both kernels are persistent and warp-specialised (192 threads):
 //   warp 0      TMA producer (one lane): halo tiles into a shared-memory ring
-//   warp 1      MMA issuer (one lane) and TMEM owner
+//   warp 1      MMA issuer (the warp waits, one elected lane issues) and TMEM owner
 //   warps 2..5  epilogue: TMEM -> registers -> global
 #include <cfloat>
 #include <cuda_bf16.h>
@@ -51,6 +51,12 @@ __device__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abor
         }
     }
     return true;
+}
+
+// The same for a converged warp whose lanes all wait (uniform result).
+__device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort, int* status)
+{
+    return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort, status));
 }
 
 // Barriers of one CTA: the halo ring, the two TMEM buffers, weights, done.
@@ -172,28 +178,28 @@ __device__ __forceinline__ void conv_layer(const CUtensorMap* map0, const CUtens
     }
     else if (warp == 1)
     {
-        if (lane == 0)
+        const uint32_t idesc = frtc::idesc_bf16_f32(128, a.cout, 0, 0);
+        const uint32_t wBase = frtc::smem_u32(R.sW);
+        const uint32_t bLbo = static_cast<uint32_t>(a.cout) * 16u;
+        // Descriptor constants hoisted out of the tile loop: per MMA only the
+        // start addresses change (a few integer ops, so issue keeps up with
+        // the tensor pipe).
+        const uint64_t bHi = frtc::smem_desc_hi(bLbo, 128);
+        const uint64_t aHi = frtc::smem_desc_hi(planeBytes, kRowBytes);
+        const uint32_t bTapStride = static_cast<uint32_t>(cin / 8) * bLbo;
+        const int kc = cin / 16;
+        bool ok = warp_wait_or_abort(&sy.wbar, wParity, abortp, a.status);
+        for (int tile = blockIdx.x; ok && tile < a.numTiles; tile += gridDim.x, ++rc.mma)
         {
-            const uint32_t idesc = frtc::idesc_bf16_f32(128, a.cout, 0, 0);
-            const uint32_t wBase = frtc::smem_u32(R.sW);
-            const uint32_t bLbo = static_cast<uint32_t>(a.cout) * 16u;
-            // Descriptor constants hoisted out of the tile loop: per MMA only the
-            // start addresses change (a few integer ops, so issue keeps up with
-            // the tensor pipe).
-            const uint64_t bHi = frtc::smem_desc_hi(bLbo, 128);
-            const uint64_t aHi = frtc::smem_desc_hi(planeBytes, kRowBytes);
-            const uint32_t bTapStride = static_cast<uint32_t>(cin / 8) * bLbo;
-            const int kc = cin / 16;
-            bool ok = wait_or_abort(&sy.wbar, wParity, abortp, a.status);
-            for (int tile = blockIdx.x; ok && tile < a.numTiles; tile += gridDim.x, ++rc.mma)
+            const int it = rc.mma;
+            const int s = it % R.stages;
+            if (!warp_wait_or_abort(&sy.full[s], (it / R.stages) & 1, abortp, a.status)) break;
+            const int buf = it & 1;
+            if (it >= 2 && !warp_wait_or_abort(&sy.tempty[buf], ((it >> 1) & 1) ^ 1, abortp, a.status)) break;
+            frtc::tc_fence_after();
+            const uint32_t stageAddr = frtc::smem_u32(R.sStage + s * R.stageBytes);
+            if (frtc::elect_one())
             {
-                const int it = rc.mma;
-                const int s = it % R.stages;
-                if (!wait_or_abort(&sy.full[s], (it / R.stages) & 1, abortp, a.status)) break;
-                const int buf = it & 1;
-                if (it >= 2 && !wait_or_abort(&sy.tempty[buf], ((it >> 1) & 1) ^ 1, abortp, a.status)) break;
-                frtc::tc_fence_after();
-                const uint32_t stageAddr = frtc::smem_u32(R.sStage + s * R.stageBytes);
                 for (int mb = 0; mb < MB; ++mb)
                 {
                     const uint32_t d = tmem + static_cast<uint32_t>(buf) * accCols + static_cast<uint32_t>(mb * a.cout);
@@ -231,6 +237,7 @@ __device__ __forceinline__ void conv_layer(const CUtensorMap* map0, const CUtens
                 frtc::mma_commit(&sy.empty[s]);
                 frtc::mma_commit(&sy.tfull[buf]);
             }
+            __syncwarp();
         }
     }
     else
@@ -395,12 +402,16 @@ __global__ void __launch_bounds__(192) k_conv3x3(const __grid_constant__ CUtenso
             if (i >= 0) frtc::mbar_wait(&sy.full[i % R.stages], (i / R.stages) & 1, kWaitNs);
         frtc::mbar_wait(&sy.wbar, 0, kWaitNs);
     }
-    else if (warp == 1 && lane == 0)
+    else if (warp == 1)
     {
-        // All MMAs of this thread complete before TMEM is released.
-        frtc::mma_commit(&sy.done);
-        frtc::mbar_wait(&sy.done, 0, kWaitNs);
-        griddep_launch();
+        // All MMAs of the elected lane complete before TMEM is released.
+        if (frtc::elect_one())
+        {
+            frtc::mma_commit(&sy.done);
+            frtc::mbar_wait(&sy.done, 0, kWaitNs);
+            griddep_launch();
+        }
+        __syncwarp();
     }
     frtc::tc_fence_before();
     __syncthreads();
@@ -515,10 +526,14 @@ __global__ void __launch_bounds__(192, 1) k_unet_fwd(const __grid_constant__ Une
             if (i >= 0) frtc::mbar_wait(&sy.full[i % R.stages], (i / R.stages) & 1, kWaitNs);
         if (convs > 0) frtc::mbar_wait(&sy.wbar, static_cast<uint32_t>((convs - 1) & 1), kWaitNs);
     }
-    else if (warp == 1 && lane == 0)
+    else if (warp == 1)
     {
-        frtc::mma_commit(&sy.done);
-        frtc::mbar_wait(&sy.done, 0, kWaitNs);
+        if (frtc::elect_one())
+        {
+            frtc::mma_commit(&sy.done);
+            frtc::mbar_wait(&sy.done, 0, kWaitNs);
+        }
+        __syncwarp();
     }
     frtc::tc_fence_before();
     __syncthreads();

@@ -170,6 +170,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// One lane of a converged warp (the same one every time). Code that issues MMAs keeps
+// the whole warp in its loops and lets only the elected lane issue: descriptors and
+// addresses then stay in uniform registers, where a loop run by one lane alone moves
+// each of them there again for every MMA.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p)::"memory");
+    return p != 0;
+}
+
 // Arrives on the mbarrier when all previously issued MMAs of this thread complete.
 __device__ __forceinline__ void mma_commit(uint64_t* bar)
 {
