@@ -241,15 +241,17 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_bwd(const float* __restri
 
 // The gradient from its partial sums, one launch: the first kHeadSums CTAs sum the
 // head's per-block partials (loss -> out_loss, head gradients), the others the
-// layers' per-CTA weight-gradient partials. FP64 adds are slow on this GPU, so no
-// chain is long: 256 strided sums and a pairwise tree for the head, four interleaved
-// sums for a weight.
+// layers' weight-gradient chains. FP64 is slow on this GPU (a convert and an add per
+// partial made this kernel 91 us of a 16 x 256 x 256 step), so a weight's sum is
+// compensated FP32: every add's exact rounding error (Knuth's TwoSum) goes into a
+// second float, and the pair rounds to the result, within 2^-40 of the FP64 sum of
+// these at most 152 terms before that rounding.
 constexpr int kReduceThreads = 256;
 
 struct ReduceLayer
 {
-    const float* partial;  // [ctas][3 kx][cin + 1][3 ky * cout]
-    int ctas, cin, cout;
+    const float* partial;  // [chains][3 kx][cout][3 ky * cin + 1]
+    int chains, cin, cout;
     int block0;            // first CTA of this layer
     float *dW, *db;        // dW[cout][cin][9], db[cout]
 };
@@ -284,38 +286,55 @@ __device__ __forceinline__ void reduce_head(const ReduceArgs& R, int k)
         R.gradsHead[k - 1] = static_cast<float>(sum[0]);  // w[4][16], then b[4]
 }
 
-// One thread per (kx, ci, ky, co) of a layer, co fastest as in the partials (a warp
-// reads whole lines of every partial; the scattered 4-byte writes are a single pass
-// over 120 thousand gradients), ci = cin for the bias.
+// (hi, lo) += x: hi the rounded running sum, lo the sum of its rounding errors.
+__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float x)
+{
+    const float s = __fadd_rn(hi, x);
+    const float b = __fsub_rn(s, hi);
+    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b));
+    hi = s;
+    lo = __fadd_rn(lo, e);
+}
+
+// One thread per (kx, co, ky, ci) of a layer, ci fastest as in the partials (a warp
+// reads whole lines of every chain; the scattered 4-byte writes are a single pass
+// over 120 thousand gradients), the last of a row for the bias.
 __global__ void __launch_bounds__(kReduceThreads) k_grad_reduce(const __grid_constant__ ReduceArgs R)
 {
     if (blockIdx.x < kHeadSums) return reduce_head(R, blockIdx.x);
     int L = 0;
     while (L + 1 < kNumLayers && static_cast<int>(blockIdx.x) >= R.layer[L + 1].block0) ++L;
     const ReduceLayer& a = R.layer[L];
-    const int rows = 3 * a.cout, n = 3 * (a.cin + 1) * rows;
+    const int rows = 3 * a.cin + 1, n = 3 * a.cout * rows;
     const int i = (blockIdx.x - a.block0) * kReduceThreads + threadIdx.x;
     if (i >= n) return;
     const int row = i % rows, q = i / rows;
-    const int ci = q % (a.cin + 1), kx = q / (a.cin + 1);
-    const int co = row % a.cout, ky = row / a.cout;
-    if (ci == a.cin && (kx != 1 || ky != 1)) return;
+    const int co = q % a.cout, kx = q / a.cout;
+    if (row == 3 * a.cin && kx != 1) return;
     const float* src = a.partial + i;
     const size_t stride = static_cast<size_t>(n);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    int c = 0;
-    for (; c + 16 <= a.ctas; c += 16)
+    // chain c into sum c mod 4, combined pairwise at the end; 32 loads in flight
+    constexpr int kLoads = 32;
+    float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = 0; c < a.chains; c += kLoads)
     {
-        float v[16];
+        float v[kLoads];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = src[(c + j) * stride];
+        for (int j = 0; j < kLoads; ++j) v[j] = c + j < a.chains ? src[(c + j) * stride] : 0.f;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j & 3] += v[j];
+        for (int j = 0; j < kLoads; ++j) two_sum_add(hi[j & 3], lo[j & 3], v[j]);  // adding 0 is exact
     }
-    for (; c < a.ctas; ++c) acc[c & 3] += src[c * stride];
-    const float total = static_cast<float>((acc[0] + acc[1]) + (acc[2] + acc[3]));
-    if (ci < a.cin)
-        a.dW[(co * a.cin + ci) * 9 + ky * 3 + kx] = total;
+#pragma unroll
+    for (int j = 2; j > 0; j >>= 1)
+#pragma unroll
+        for (int k = 0; k < j; ++k)
+        {
+            two_sum_add(hi[k], lo[k], hi[k + j]);
+            two_sum_add(hi[k], lo[k], lo[k + j]);
+        }
+    const float total = __fadd_rn(hi[0], lo[0]);
+    if (row < 3 * a.cin)
+        a.dW[(co * a.cin + row % a.cin) * 9 + row / a.cin * 3 + kx] = total;
     else
         a.db[co] = total;
 }
@@ -639,10 +658,9 @@ int plan_conv(fr_aonet* n, const Shape& S, int lv, const uint16_t* in0, int c0, 
 {
     const int H = S.h(lv), W = S.w(lv);
     const int cin = c0 + c1;
-    const bool paired = cin == 8;
     const long long tiles1 = static_cast<long long>(S.B) * ((W + kTileW - 1) / kTileW) * ((H + kTileH - 1) / kTileH);
     int mb = (tiles1 >= 16LL * n->numSMs && 2 * 4 * cout <= 512) ? 4 : 1;
-    while (mb > 1 && conv_smem_bytes(cin, cout, 2, paired, mb) > 200u * 1024u) mb >>= 1;
+    while (mb > 1 && conv_smem_bytes(cin, cout, 2, mb) > 200u * 1024u) mb >>= 1;
     const int tileH = kTileH * mb;
     if (!make_cp_map(&P.m0, in0, c0, S.B, H, W, kHaloW, tileH + 2)) return net_fail(n, FR_ERR_CUDA, "tensor map encode");
     if (c1 > 0)
@@ -675,10 +693,10 @@ int plan_conv(fr_aonet* n, const Shape& S, int lv, const uint16_t* in0, int c0, 
     // where that keeps 4 CTAs on an SM (their epilogues overlap: the 48-channel
     // level-0 layer runs 4 CTAs of 2 stages per SM faster than 2 CTAs of 4 stages).
     int stages = kMaxStages;
-    while (stages > 2 && conv_smem_bytes(cin, cout, stages, paired, mb) > 200u * 1024u) --stages;
-    while (stages > 2 && (228u * 1024u) / (conv_smem_bytes(cin, cout, stages, paired, mb) + 2048u) < 4u) --stages;
+    while (stages > 2 && conv_smem_bytes(cin, cout, stages, mb) > 200u * 1024u) --stages;
+    while (stages > 2 && (228u * 1024u) / (conv_smem_bytes(cin, cout, stages, mb) + 2048u) < 4u) --stages;
     a.stages = stages;
-    P.smem = conv_smem_bytes(cin, cout, stages, paired, mb);
+    P.smem = conv_smem_bytes(cin, cout, stages, mb);
     const int cols = 2 * mb * cout;
     const int tmemCols = cols <= 32 ? 32 : cols <= 64 ? 64 : cols <= 128 ? 128 : cols <= 256 ? 256 : 512;
     int perSM = static_cast<int>((228u * 1024u) / (P.smem + 2048u));
@@ -712,9 +730,11 @@ int wgrad_layer(fr_aonet* n, const Shape& S, int layer, const uint16_t* x0, cons
                 WgradLayer& L)
 {
     const LayerSpec& s = kLayers[layer];
-    const int H = S.h(s.level), W = S.w(s.level);
-    if (!make_cp_map(&L.mapX0, x0, s.c0, S.B, H, W, kHaloW, kTileH) ||
-        (s.c1 > 0 && !make_cp_map(&L.mapX1, x1, s.c1, S.B, H, W, kHaloW, kTileH)) ||
+    const int H = S.h(s.level), W = S.w(s.level), cin = s.c0 + s.c1;
+    const bool kyRows = wgrad_ky_rows(cin);
+    const int xRows = kTileH + (kyRows ? 0 : 2);
+    if (!make_cp_map(&L.mapX0, x0, s.c0, S.B, H, W, kHaloW, xRows) ||
+        (s.c1 > 0 && !make_cp_map(&L.mapX1, x1, s.c1, S.B, H, W, kHaloW, xRows)) ||
         !make_cp_map(&L.mapDY, dY, s.cout, S.B, H, W, kTileW, kTileH))
         return net_fail(n, FR_ERR_CUDA, "tensor map encode");
     if (s.c1 == 0) L.mapX1 = L.mapX0;
@@ -722,10 +742,12 @@ int wgrad_layer(fr_aonet* n, const Shape& S, int layer, const uint16_t* x0, cons
     L.tilesY = (H + kTileH - 1) / kTileH;
     L.numTiles = S.B * L.tilesX * L.tilesY;
     L.c0 = s.c0, L.c1 = s.c1, L.cout = s.cout;
-    const uint32_t stage = wgrad_stage_bytes(s.c0 + s.c1, s.cout), window = wgrad_a_window(s.cout);
+    L.kyRows = kyRows;
+    // one chain per SM of the chip: an FP32 accumulator adds up few tiles
+    L.nChains = std::min(L.numTiles, n->numSMs);
+    const uint32_t stage = wgrad_stage_bytes(cin, s.cout, kyRows), window = wgrad_a_window(cin, kyRows);
     L.stages = kMaxStages;
     while (L.stages > 2 && (L.stages - 1) * stage + std::max(stage, window) > kWgradSmem) --L.stages;
-    L.sets = std::min(4, 512 / wgrad_set_cols(s.c0 + s.c1, s.cout));
     return FR_OK;
 }
 
@@ -735,36 +757,53 @@ int wgrad_all(fr_aonet* n, const WgradLayer* layers, int headBlocks, float invN,
     WgradArgs U{};
     U.nLayers = kNumLayers;
     U.status = n->status;
-    // A CTA takes an even share of one wave's MMAs, or fewer tiles where its accumulator
-    // sets hold no more than kWgradChain tiles each; the CTAs with the most work first,
-    // so that those beyond the first wave are short.
-    auto blocks = [&](int L) { return (3 * kLayers[L].cout + 127) / 128; };
+    // A chain's cost in cycles, as measured: its tiles' MMAs (47 each for 128 rows, 33 for
+    // 64; the operand and barrier latency) and storing its accumulators (500 per 16
+    // columns of 128 rows, 350 of 64). The CTAs share the cost of all layers evenly: the
+    // smallest cost per CTA at which they fit one per SM.
+    auto cost = [&](int L) {
+        const WgradLayer& w = layers[L];
+        const int cin = w.c0 + w.c1, units = wgrad_units(cin, w.kyRows != 0);
+        const int half = wgrad_half_last(cin, w.kyRows != 0) ? 1 : 0, full = units - half;
+        const int tile = 3 * (kTileH / 2) * (47 * full + 33 * half) + 110;
+        return (w.numTiles + w.nChains - 1) / w.nChains * tile + 3 * (w.cout / 16) * (500 * full + 350 * half);
+    };
+    auto ctas = [&](int L, long long per) {
+        const int q = static_cast<int>(std::max(1LL, per / cost(L)));  // chains per CTA
+        return (layers[L].nChains + q - 1) / q;
+    };
     long long work = 0;
-    for (int L = 0; L < kNumLayers; ++L) work += static_cast<long long>(layers[L].numTiles) * blocks(L);
-    const long long share = std::max(1LL, (work + n->numSMs - 1) / n->numSMs);
-    auto tiles = [&](int L) { return std::min(std::max(share / blocks(L), 1LL), 1LL * kWgradChain * layers[L].sets); };
-    int order[kNumLayers];
-    for (int L = 0; L < kNumLayers; ++L) order[L] = L;
-    std::stable_sort(order, order + kNumLayers,
-                     [&](int p, int q) { return tiles(p) * blocks(p) > tiles(q) * blocks(q); });
+    for (int L = 0; L < kNumLayers; ++L) work += static_cast<long long>(layers[L].nChains) * cost(L);
+    long long per = std::max(1LL, work / n->numSMs);
+    for (;; per += per / 64 + 1)
+    {
+        int sum = 0;
+        for (int L = 0; L < kNumLayers; ++L) sum += ctas(L, per);
+        if (sum <= n->numSMs) break;
+    }
     ReduceArgs R{};
     size_t need = 0;
     int grid = 0, rblocks = kHeadSums;
     size_t at[kNumLayers];
-    for (int i = 0; i < kNumLayers; ++i)
+    for (int L = 0; L < kNumLayers; ++L)
     {
-        const int L = order[i];
-        WgradLayer& w = U.layer[i];
+        WgradLayer& w = U.layer[L];
         w = layers[L];
         const int cin = w.c0 + w.c1;
         w.cta0 = grid;
-        w.ctas = static_cast<int>((w.numTiles + tiles(L) - 1) / tiles(L));
+        w.ctas = ctas(L, per);
+        // accumulators for all of a CTA's chains where they fit the 512 TMEM columns, else
+        // two halves that are filled and read out in turn
+        const int fit = 512 / (wgrad_units(cin, w.kyRows != 0) * 3 * w.cout);
+        const int q = (w.nChains + w.ctas - 1) / w.ctas;
+        w.bufs = q <= fit || fit < 2 ? 1 : 2;
+        w.sets = std::min(q, fit / w.bufs);
         grid += w.ctas;
-        at[i] = need;
-        need += w.ctas * wgrad_partial_floats(cin, w.cout);
-        R.layer[i] = ReduceLayer{nullptr, w.ctas, cin, w.cout, rblocks, n->grads + n->paramOff[L],
+        at[L] = need;
+        need += w.nChains * wgrad_partial_floats(cin, w.cout);
+        R.layer[L] = ReduceLayer{nullptr, w.nChains, cin, w.cout, rblocks, n->grads + n->paramOff[L],
                                  n->grads + n->paramOff[L] + w_count(L)};
-        rblocks += blocks_for(9LL * (cin + 1) * w.cout, kReduceThreads);
+        rblocks += blocks_for(static_cast<long long>(wgrad_partial_floats(cin, w.cout)), kReduceThreads);
     }
     if (need > n->partialCap)
     {
@@ -773,7 +812,7 @@ int wgrad_all(fr_aonet* n, const WgradLayer* layers, int headBlocks, float invN,
         NET_CUDA(n, cudaMalloc(&n->partial, sizeof(float) * need));
         n->partialCap = need;
     }
-    for (int i = 0; i < kNumLayers; ++i) R.layer[i].partial = U.layer[i].partial = n->partial + at[i];
+    for (int L = 0; L < kNumLayers; ++L) R.layer[L].partial = U.layer[L].partial = n->partial + at[L];
     R.headPart = n->headPart, R.headBlocks = headBlocks;
     R.gradsHead = n->grads + n->paramOff[kNumLayers];
     R.loss = n->lossDev, R.invN = invN;

@@ -95,11 +95,6 @@ __device__ __forceinline__ void decode_tile(int tile, int tilesX, int tilesY, in
     tx = r - ty * tilesX;
 }
 
-__device__ __forceinline__ int tap_offset(int t)  // byte offset of tap t inside a halo plane
-{
-    return ((t / 3) * kHaloW + (t % 3)) * 16;
-}
-
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
 {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -108,12 +103,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-
-// Paired-tap schedule for an 8-channel input: K step p covers taps kPairA[p] and
-// kPairB[p] (the second 8 K-elements read the pixel that tap B reads). The last
-// step repeats tap 7 with zero weights.
-__constant__ int kPairA[5] = {0, 2, 4, 6, 7};
-__constant__ int kPairB[5] = {1, 3, 5, 7, 8};
 
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -139,8 +128,8 @@ struct RoleCounters
     int epi = 0;     // epilogue threads
 };
 
-// One layer's tiles on this CTA: warp 0 lane 0 loads halo tiles, warp 1 lane 0
-// issues the MMAs (after the weights, wbar phase wParity), warps 2..5 run the
+// One layer's tiles on this CTA: warp 0 lane 0 loads halo tiles, warp 1 issues
+// the MMAs (after the weights, wbar phase wParity), warps 2..5 run the
 // epilogue. The weights are already being loaded, bias / head are in shared memory.
 __device__ __forceinline__ void conv_layer(const CUtensorMap* map0, const CUtensorMap* map1, const ConvArgs& a,
                                            const ConvRing& R, SyncState& sy, uint32_t tmem, uint32_t wParity,
@@ -148,7 +137,6 @@ __device__ __forceinline__ void conv_layer(const CUtensorMap* map0, const CUtens
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cin = a.c0 + a.c1;
-    const bool paired = (cin == 8);
     const int MB = a.mb;
     const int tileH = kTileH * MB;
     const uint32_t planeBytes = static_cast<uint32_t>(kHaloW * (tileH + 2) * 16);
@@ -204,33 +192,16 @@ __device__ __forceinline__ void conv_layer(const CUtensorMap* map0, const CUtens
                 {
                     const uint32_t d = tmem + static_cast<uint32_t>(buf) * accCols + static_cast<uint32_t>(mb * a.cout);
                     const uint32_t aBase = stageAddr + static_cast<uint32_t>(mb * kTileH) * kRowBytes;
-                    if (paired)
-                    {
 #pragma unroll
-                        for (int p = 0; p < 5; ++p)
-                        {
-                            constexpr int pa[5] = {0, 2, 4, 6, 7};
-                            constexpr int pb[5] = {1, 3, 5, 7, 8};
-                            const uint32_t oa = ((pa[p] / 3) * kHaloW + pa[p] % 3) * 16;
-                            const uint32_t ob = ((pb[p] / 3) * kHaloW + pb[p] % 3) * 16;
-                            const uint64_t ad = frtc::smem_desc_hi(ob - oa, kRowBytes) | ((aBase + oa) >> 4);
-                            const uint64_t bd = bHi | ((wBase + static_cast<uint32_t>(p * 2) * bLbo) >> 4);
-                            frtc::mma_bf16(d, ad, bd, idesc, p > 0);
-                        }
-                    }
-                    else
+                    for (int t = 0; t < 9; ++t)
                     {
-#pragma unroll
-                        for (int t = 0; t < 9; ++t)
+                        const uint32_t aTap = aBase + static_cast<uint32_t>(((t / 3) * kHaloW + t % 3) * 16);
+                        const uint32_t bTap = wBase + static_cast<uint32_t>(t) * bTapStride;
+                        for (int j = 0; j < kc; ++j)
                         {
-                            const uint32_t aTap = aBase + static_cast<uint32_t>(((t / 3) * kHaloW + t % 3) * 16);
-                            const uint32_t bTap = wBase + static_cast<uint32_t>(t) * bTapStride;
-                            for (int j = 0; j < kc; ++j)
-                            {
-                                const uint64_t ad = aHi | ((aTap + static_cast<uint32_t>(2 * j) * planeBytes) >> 4);
-                                const uint64_t bd = bHi | ((bTap + static_cast<uint32_t>(2 * j) * bLbo) >> 4);
-                                frtc::mma_bf16(d, ad, bd, idesc, (t | j) != 0);
-                            }
+                            const uint64_t ad = aHi | ((aTap + static_cast<uint32_t>(2 * j) * planeBytes) >> 4);
+                            const uint64_t bd = bHi | ((bTap + static_cast<uint32_t>(2 * j) * bLbo) >> 4);
+                            frtc::mma_bf16(d, ad, bd, idesc, (t | j) != 0);
                         }
                     }
                 }
@@ -544,16 +515,39 @@ __global__ void __launch_bounds__(192, 1) k_unet_fwd(const __grid_constant__ Une
     }
 }
 
-// Every layer's weight gradient in one launch (WgradArgs). A tile is 8 x 16 pixels
-// of X rows and output columns: dY is loaded at rows y0 + 1, y0, y0 - 1 (ky = 0, 1,
-// 2; the TMA zero fill stands for pixels outside the image), so rows (ky, co) of
-// the A operand are adjacent planes, and X with one extra pixel on either side, so
-// kx is a start address 16 bytes further. 24 MMAs (48 for 64 output channels) cover
-// the nine taps of a tile; one M = 128 MMA per tap took 72, each mostly fetching
-// rows of zeros. Bound by the MMAs' A fetch (about 40 cycles each). The CTAs are
-// shared out among the layers by their MMA count, so a step needs about one wave and
-// few partial sums: with one launch of 152 CTAs per layer the ten launches took 301 us
-// at 16 x 256 x 256 and left 152 partials per weight to add up (425 us).
+// One tile's MMAs: 8 K steps of 16 pixels (two tile rows), each UNITS x 3 kx, unrolled
+// with constant address steps; the last row block may have M = 64 (idescLast).
+template <int UNITS>
+__device__ __forceinline__ void wgrad_tile_mmas(uint32_t set, uint32_t cout, uint32_t xLo, uint32_t aHi, uint32_t unitStep,
+                                                uint32_t yLo, uint32_t bHi, uint32_t idesc, uint32_t idescLast,
+                                                uint32_t more)
+{
+#pragma unroll
+    for (int j = 0; j < kTileH / 2; ++j)
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u)
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx)  // the next kx: 16 bytes further
+                frtc::mma_bf16_lohi(set + static_cast<uint32_t>(u * 3 + kx) * cout,
+                                    xLo + u * unitStep + static_cast<uint32_t>(j * 2 * kRowBytes / 16 + kx), aHi,
+                                    yLo + static_cast<uint32_t>(j * 16), bHi, u == UNITS - 1 ? idescLast : idesc,
+                                    j == 0 ? more : 1u);
+}
+
+// Every layer's weight gradient in one launch (WgradArgs). Rows of the A operand are
+// input channels, columns output channels, K the tile's pixels. With few input
+// channels the three ky are rows too (X is loaded three times, one row further each
+// time, so rows (ky, ci) are adjacent planes) and kx is a start address 16 bytes
+// further: 24 MMAs cover the nine taps of a tile where one M = 128 MMA per tap took
+// 72, each mostly fetching rows of zeros. K steps are outermost, so consecutive MMAs
+// add to different accumulators. A tile's sums go to the accumulator of its chain
+// (tile mod nChains), in tile order: which pixels meet in one FP32 sum does not
+// depend on how the chains are dealt to CTAs. Bound by the MMAs (47 cycles each for
+// 128 rows, 33 for 64: the operand fetch) and, on the small levels, where a chain is
+// one tile, by storing the accumulators (about 500 cycles per 16 columns). One X copy
+// with the ky rows interleaved in shared memory needs the bias as a fourth
+// accumulator, 32 MMAs instead of 24, and measured 105 us against 84. At 16 x 256 x 256
+// this kernel takes 67 us.
 __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs U)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -563,21 +557,29 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs
     while (L + 1 < U.nLayers && static_cast<int>(blockIdx.x) >= U.layer[L + 1].cta0) ++L;
     const WgradLayer& a = U.layer[L];
     const int k0 = blockIdx.x - a.cta0;
-    const int cin = a.c0 + a.c1, cout = a.cout;
-    const int nCols = cin + 16;                      // X channels, the ones column, padding
-    const int mBlocks = (3 * cout + 127) / 128;
-    const uint32_t yBytes = static_cast<uint32_t>(cout / 8) * kWgradYPlane;  // one dY copy
-    const uint32_t stageBytes = wgrad_stage_bytes(cin, cout);
-    const int setCols = wgrad_set_cols(cin, cout);
-    const uint32_t allocCols = tmem_cols(a.sets * setCols);
+    // the loops' parameters in registers: read again from the parameter bank after
+    // every barrier wait, and with a division for the ring slot, they cost 350 cycles a tile
+    const int cin = a.c0 + a.c1, cout = a.cout, nch = a.nChains, ctas = a.ctas, numTiles = a.numTiles;
+    const int stages = a.stages, sets = a.sets, bufs = a.bufs;
+    const bool kyRows = a.kyRows != 0;
+    const int copies = kyRows ? 3 : 1;                               // X copies, one per ky
+    const int xRows = kTileH + (kyRows ? 0 : 2);                     // rows of a copy
+    const uint32_t plane = static_cast<uint32_t>(xRows * kRowBytes);
+    const uint32_t xBytes = static_cast<uint32_t>(cin / 8) * plane;  // one copy
+    const int units = wgrad_units(cin, kyRows);                      // row blocks, or ky
+    const bool half = wgrad_half_last(cin, kyRows);                  // the last row block has M = 64
+    const uint32_t unitStep = kyRows ? 16u * plane : static_cast<uint32_t>(kRowBytes);
+    const uint32_t constBytes = wgrad_const_bytes(kyRows);
+    const uint32_t stageBytes = wgrad_stage_bytes(cin, cout, kyRows);
+    const int setCols = units * 3 * cout;
+    const uint32_t allocCols = tmem_cols(bufs * sets * setCols);
 
-    // The planes cin/8 and cin/8 + 1 of every X stage are constant: 1.0 in channel 0
-    // (its accumulator column is the bias gradient), else zero.
-    for (int s = 0; s < a.stages; ++s)
+    // The plane after X's is constant in every stage: 1.0 in channel 0 (its accumulator
+    // row is the bias gradient), else zero.
+    for (int s = 0; s < stages; ++s)
     {
-        uint32_t* p = reinterpret_cast<uint32_t*>(smem + s * stageBytes + 3 * yBytes + (cin / 8) * kWgradXPlane);
-        for (int i = threadIdx.x; i < 2 * kWgradXPlane / 4; i += blockDim.x)
-            p[i] = (i < kWgradXPlane / 4 && (i & 3) == 0) ? 0x3F80u : 0u;
+        uint32_t* p = reinterpret_cast<uint32_t*>(smem + s * stageBytes + copies * xBytes);
+        for (int i = threadIdx.x; i < static_cast<int>(plane) / 4; i += blockDim.x) p[i] = (i & 3) == 0 ? 0x3F80u : 0u;
     }
     frtc::fence_proxy_async_smem();
     init_sync(sy);
@@ -587,107 +589,148 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs
     frtc::tc_fence_after();
     const uint32_t tmem = sy.tmem;
     volatile int* abortp = &sy.abort;
+    // this CTA's chains k0, k0 + ctas, ... in groups of `sets`; a group's tiles go
+    // round by round (one tile of each chain), which every role walks alike
+    const int mine = (nch - 1 - k0) / ctas + 1;
+    const int rounds = (numTiles + nch - 1) / nch;
 
     if (warp == 0)
     {
         if (lane == 0)
         {
-            const uint32_t loadBytes = 3 * yBytes + static_cast<uint32_t>(cin / 8) * kWgradXPlane;
-            int issued = 0;
-            for (int tile = k0; tile < a.numTiles; tile += a.ctas, ++issued)
-            {
-                const int s = issued % a.stages;
-                const uint32_t ph = (issued / a.stages) & 1;
-                if (issued >= a.stages && !wait_or_abort(&sy.empty[s], ph ^ 1, abortp, U.status)) break;
-                int b, tx, ty;
-                decode_tile(tile, a.tilesX, a.tilesY, b, tx, ty);
-                unsigned char* dst = smem + s * stageBytes;
-                frtc::mbar_expect_tx(&sy.full[s], loadBytes);
-                for (int ky = 0; ky < 3; ++ky)
-                    frtc::tma_load_3d(dst + ky * yBytes, &a.mapDY, 8 * tx * kTileW, ty * kTileH + 1 - ky,
-                                      b * (cout / 8), &sy.full[s]);
-                dst += 3 * yBytes;
-                frtc::tma_load_3d(dst, &a.mapX0, 8 * (tx * kTileW - 1), ty * kTileH, b * (a.c0 / 8), &sy.full[s]);
-                if (a.c1)
-                    frtc::tma_load_3d(dst + (a.c0 / 8) * kWgradXPlane, &a.mapX1, 8 * (tx * kTileW - 1), ty * kTileH,
-                                      b * (a.c1 / 8), &sy.full[s]);
-            }
+            const uint32_t loadBytes = copies * xBytes + static_cast<uint32_t>(cout / 8) * kWgradYPlane;
+            int issued = 0, s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int c0 = 0; ok && c0 < mine; c0 += sets)
+                for (int r = 0; ok && r < rounds; ++r)
+                    for (int c = c0; c < min(c0 + sets, mine); ++c)
+                    {
+                        const int tile = k0 + c * ctas + r * nch;
+                        if (tile >= numTiles) break;
+                        ok = issued < stages || wait_or_abort(&sy.empty[s], ph ^ 1, abortp, U.status);
+                        if (!ok) break;
+                        int b, tx, ty;
+                        decode_tile(tile, a.tilesX, a.tilesY, b, tx, ty);
+                        unsigned char* dst = smem + s * stageBytes;
+                        frtc::mbar_expect_tx(&sy.full[s], loadBytes);
+                        for (int ky = 0; ky < copies; ++ky, dst += xBytes)
+                        {
+                            frtc::tma_load_3d(dst, &a.mapX0, 8 * (tx * kTileW - 1), ty * kTileH - 1 + ky,
+                                              b * (a.c0 / 8), &sy.full[s]);
+                            if (a.c1)
+                                frtc::tma_load_3d(dst + (a.c0 / 8) * plane, &a.mapX1, 8 * (tx * kTileW - 1),
+                                                  ty * kTileH - 1 + ky, b * (a.c1 / 8), &sy.full[s]);
+                        }
+                        frtc::tma_load_3d(dst + constBytes, &a.mapDY, 8 * tx * kTileW, ty * kTileH, b * (cout / 8),
+                                          &sy.full[s]);
+                        ++issued;
+                        if (++s == stages) s = 0, ph ^= 1;
+                    }
             // every issued copy lands before the CTA exits
-            for (int i = issued - a.stages; i < issued; ++i)
-                if (i >= 0) frtc::mbar_wait(&sy.full[i % a.stages], (i / a.stages) & 1, kWaitNs);
+            for (int i = issued - stages; i < issued; ++i)
+                if (i >= 0) frtc::mbar_wait(&sy.full[i % stages], (i / stages) & 1, kWaitNs);
         }
     }
     else if (warp == 1)
     {
-        if (lane == 0)
+        const uint32_t idesc = frtc::idesc_bf16_f32(128, cout, 1, 1);
+        const uint32_t idescLast = half ? frtc::idesc_bf16_f32(64, cout, 1, 1) : idesc;
+        // both operands MN-major: K core matrices (8 pixels of a row) one row apart,
+        // groups of 8 rows / columns (channels) one plane apart
+        const uint64_t aDesc = frtc::smem_desc_hi(kRowBytes, plane);
+        constexpr uint64_t bDesc = frtc::smem_desc_hi(128u, kWgradYPlane);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int c0 = 0, g = 0; ok && c0 < mine; c0 += sets, ++g)
         {
-            const uint32_t idesc = frtc::idesc_bf16_f32(128, nCols, 1, 1);
-            // both operands MN-major: K core matrices (8 pixels of a row) one row apart,
-            // groups of 8 rows / columns (channels) one plane apart
-            constexpr uint64_t aHi = frtc::smem_desc_hi(128u, kWgradYPlane);
-            constexpr uint64_t bHi = frtc::smem_desc_hi(kWgradXRowBytes, kWgradXPlane);
-            int it = 0;
-            for (int tile = k0; tile < a.numTiles; tile += a.ctas, ++it)
-            {
-                const int s = it % a.stages;
-                if (!wait_or_abort(&sy.full[s], (it / a.stages) & 1, abortp, U.status)) break;
-                frtc::tc_fence_after();
-                const uint32_t yb = frtc::smem_u32(smem + s * stageBytes);
-                const uint32_t xb = yb + 3 * yBytes;
-                const uint32_t set = tmem + static_cast<uint32_t>((it % a.sets) * setCols);
-                const uint32_t more = it >= a.sets;  // the set already holds earlier tiles
-                for (int m = 0; m < mBlocks; ++m)
-                    for (int kx = 0; kx < 3; ++kx)
+            const int buf = bufs == 2 ? g & 1 : 0;
+            const int use = bufs == 2 ? g >> 1 : g;  // earlier groups in this buffer
+            if (use > 0 && !warp_wait_or_abort(&sy.tempty[buf], (use - 1) & 1, abortp, U.status)) break;
+            frtc::tc_fence_after();
+            for (int r = 0; ok && r < rounds; ++r)
+                for (int c = c0; c < min(c0 + sets, mine); ++c)
+                {
+                    if (k0 + c * ctas + r * nch >= numTiles) break;
+                    ok = warp_wait_or_abort(&sy.full[s], ph, abortp, U.status);
+                    if (!ok) break;
+                    frtc::tc_fence_after();
+                    const uint32_t xb = frtc::smem_u32(smem + s * stageBytes);
+                    const uint32_t yb = xb + copies * xBytes + constBytes;
+                    const uint32_t set = tmem + static_cast<uint32_t>((buf * sets + c - c0) * setCols);
+                    if (frtc::elect_one())
                     {
-                        const uint32_t d = set + static_cast<uint32_t>((m * 3 + kx) * nCols);
-                        const uint32_t ya = yb + static_cast<uint32_t>(m * 16 * kWgradYPlane);
-                        const uint32_t xa = xb + static_cast<uint32_t>(kx * 16);
-#pragma unroll
-                        for (int j = 0; j < kTileH / 2; ++j)  // K = 16 pixels: two tile rows
-                            frtc::mma_bf16(d, aHi | ((ya + static_cast<uint32_t>(j * 256)) >> 4),
-                                           bHi | ((xa + static_cast<uint32_t>(j * 2 * kWgradXRowBytes)) >> 4), idesc,
-                                           more | static_cast<uint32_t>(j));
+                        const uint32_t xLo = static_cast<uint32_t>(aDesc) | (xb >> 4);
+                        const uint32_t yLo = static_cast<uint32_t>(bDesc) | (yb >> 4);
+                        const uint32_t aHi = static_cast<uint32_t>(aDesc >> 32), bHi = static_cast<uint32_t>(bDesc >> 32);
+                        if (units == 1)
+                            wgrad_tile_mmas<1>(set, cout, xLo, aHi, 0u, yLo, bHi, idesc, idescLast, r > 0);
+                        else if (units == 2)
+                            wgrad_tile_mmas<2>(set, cout, xLo, aHi, unitStep / 16, yLo, bHi, idesc, idescLast, r > 0);
+                        else
+                            wgrad_tile_mmas<3>(set, cout, xLo, aHi, unitStep / 16, yLo, bHi, idesc, idescLast, r > 0);
+                        frtc::mma_commit(&sy.empty[s]);
                     }
-                frtc::mma_commit(&sy.empty[s]);
-            }
+                    __syncwarp();
+                    if (++s == stages) s = 0, ph ^= 1;
+                }
+            if (frtc::elect_one()) frtc::mma_commit(&sy.tfull[buf]);
+            __syncwarp();
+        }
+        if (frtc::elect_one())
+        {
             frtc::mma_commit(&sy.done);
             frtc::mbar_wait(&sy.done, 0, kWaitNs);
         }
+        __syncwarp();
     }
     else
     {
         const int q = warp & 3;
-        int ok = 1;
-        if (lane == 0) ok = wait_or_abort(&sy.done, 0, abortp, U.status);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        frtc::tc_fence_after();
-        const int used = min(a.sets, (a.numTiles - 1 - k0) / a.ctas + 1);  // every CTA has a tile
-        float* part = a.partial + static_cast<size_t>(k0) * wgrad_partial_floats(cin, cout);
-        for (int m = 0; m < mBlocks; ++m)
+        const int rows = 3 * cin + 1;  // (ky, ci), then the bias
+        for (int c0 = 0, g = 0; c0 < mine; c0 += sets, ++g)
         {
-            const int row = m * 128 + q * 32 + lane;  // ky * cout + co
-            for (int kx = 0; kx < 3; ++kx)
-                for (int g = 0; g < nCols / 16; ++g)
+            const int buf = bufs == 2 ? g & 1 : 0;
+            const int use = bufs == 2 ? g >> 1 : g;
+            int ok = 1;
+            if (lane == 0) ok = wait_or_abort(&sy.tfull[buf], use & 1, abortp, U.status);
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;  // the status word is set: the gradients are not used
+            frtc::tc_fence_after();
+            for (int c = c0; c < min(c0 + sets, mine); ++c)
+            {
+                float* part = a.partial + static_cast<size_t>(k0 + c * ctas) * wgrad_partial_floats(cin, cout);
+                const uint32_t set = tmem + (static_cast<uint32_t>(q * 32) << 16) +
+                                     static_cast<uint32_t>((buf * sets + c - c0) * setCols);
+                for (int u = 0; u < units; ++u)
                 {
-                    const uint32_t at = tmem + (static_cast<uint32_t>(q * 32) << 16) +
-                                        static_cast<uint32_t>((m * 3 + kx) * nCols + g * 16);
-                    float v[16];
-                    frtc::tmem_ld16(at, v);
-                    for (int e = 1; e < used; ++e)
-                    {
-                        float w[16];
-                        frtc::tmem_ld16(at + static_cast<uint32_t>(e * setCols), w);
+                    // this thread's accumulator row: (ky, ci) or, just after the channels, the bias
+                    // (M = 64: 16 rows at the start of each warp's 32 lanes)
+                    const bool h = half && u == units - 1;
+                    const int m = (kyRows ? u * 128 : 0) + (h ? q * 16 : q * 32) + lane;
+                    const int nRows = kyRows ? 3 * cin : cin;
+                    const bool bias = m == nRows && (kyRows || u == 0);
+                    const int row = bias ? 3 * cin : kyRows ? m : u * cin + m;
+                    const bool live = (bias || m < nRows) && (!h || lane < 16);
+                    for (int kx = 0; kx < 3; ++kx)
+                        for (int n0 = 0; n0 < cout; n0 += 16)
+                        {
+                            float v[16];
+                            frtc::tmem_ld16(set + static_cast<uint32_t>((u * 3 + kx) * cout + n0), v);
+                            if (live)
+                            {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] += w[i];
-                    }
-                    if (row >= 3 * cout) continue;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                    {
-                        const int ci = g * 16 + i;
-                        if (ci <= cin) part[(static_cast<size_t>(kx) * (cin + 1) + ci) * (3 * cout) + row] = ok ? v[i] : 0.f;
-                    }
+                                for (int i = 0; i < 16; ++i)
+                                    part[(static_cast<size_t>(kx) * cout + n0 + i) * rows + row] = v[i];
+                            }
+                            __syncwarp();
+                        }
                 }
+            }
+            frtc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) frtc::mbar_arrive(&sy.tempty[buf]);
         }
     }
     frtc::tc_fence_before();
@@ -705,9 +748,9 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs
 // per-block maximum minus room for their static shared memory.
 constexpr int kMaxDynSmem = 220 * 1024;
 
-uint32_t conv_smem_bytes(int cin, int cout, int stages, bool paired, int mb)
+uint32_t conv_smem_bytes(int cin, int cout, int stages, int mb)
 {
-    const uint32_t wbytes = paired ? 5u * 2u * 8u * cout * 2u : 9u * cin * cout * 2u;
+    const uint32_t wbytes = 9u * cin * cout * 2u;
     const uint32_t w = (wbytes + 1023u) & ~1023u;
     const uint32_t plane = static_cast<uint32_t>(kHaloW * (kTileH * mb + 2) * 16);
     const uint32_t stage = (static_cast<uint32_t>(cin / 8) * plane + 1023u) & ~1023u;

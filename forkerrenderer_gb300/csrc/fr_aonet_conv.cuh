@@ -52,15 +52,12 @@ struct ConvArgs
 };
 
 // ---- weight gradients of every layer in one launch -------------------------------
-// dW[co][ci][ky][kx] = sum_p dY[co][p] X[ci][p + (ky - 1, kx - 1)] as one GEMM per
-// layer whose K runs over pixels: the rows are (ky, co) - dY read three times, one
-// row up, level and down - and the columns are input channels, the three kx being
-// three column blocks read from one X tile at three start addresses.
+// dW[co][ci][ky][kx] = sum_p dY[co][p] X[ci][p + (ky - 1, kx - 1)], K running over the
+// pixels of 8 x 16 tiles. The tiles of a layer form nChains chains (tile mod nChains),
+// each summed in one FP32 accumulator in tile order; a CTA runs several chains.
 constexpr int kWgradMaxLayers = 10;
-constexpr int kWgradXRowBytes = kHaloW * 16;                 // 160: an X row of a tile, 10 pixels
-constexpr int kWgradXPlane = kTileH * kWgradXRowBytes;       // 2560: 8 channels of a tile's X
-constexpr int kWgradYPlane = kTileW * kTileH * 16;           // 2048: 8 channels of a tile's dY
-constexpr uint32_t kWgradSmem = 184u * 1024u;                // one CTA per SM, 2..4 stages
+constexpr int kWgradYPlane = kTileW * kTileH * 16;  // 2048: 8 channels of a tile's dY
+constexpr uint32_t kWgradSmem = 184u * 1024u;       // one CTA per SM, 2..4 stages
 
 struct WgradLayer
 {
@@ -68,10 +65,13 @@ struct WgradLayer
     int tilesX, tilesY, numTiles;
     int c0, c1;          // X channels from mapX0 / mapX1; cin = c0 + c1 <= 96
     int cout;            // dY channels: 16, 32 or 64
+    int kyRows;          // 1: rows (ky, ci), X loaded once per ky; 0: rows ci, ky by start address
+    int nChains;
+    int sets, bufs;      // accumulators of chains held at a time, and 2 when the next ones
+                         // are filled while these are read out
     int stages;          // shared-memory pipeline depth
-    int sets;            // accumulator sets in TMEM: tile i of a CTA adds to set i % sets
-    int cta0, ctas;      // the CTAs [cta0, cta0 + ctas) share this layer's tiles
-    float* partial;      // [ctas][3 kx][cin + 1][3 ky * cout]; row cin: the bias (ky = kx = 1)
+    int cta0, ctas;      // CTA cta0 + k runs the chains k, k + ctas, ...
+    float* partial;      // [nChains][3 kx][cout][3 ky * cin + 1 (bias, kx = 1)]
 };
 
 struct WgradArgs
@@ -81,22 +81,43 @@ struct WgradArgs
     int* status;
 };
 
-// Bytes of one pipeline stage of a layer (dY three times, X, the ones and zero planes).
-constexpr uint32_t wgrad_stage_bytes(int cin, int cout)
+// Rows (ky, ci) unless they need three blocks of 128 (a row more for the bias): then
+// rows ci and one MMA per tap is no more work.
+constexpr bool wgrad_ky_rows(int cin) { return 3 * cin + 1 <= 256; }
+// MMAs of a K step are 3 kx times this: row blocks, or the three ky.
+__host__ __device__ constexpr int wgrad_units(int cin, bool kyRows) { return kyRows ? (3 * cin + 1 + 127) / 128 : 3; }
+// Whether the last row block needs at most 64 rows.
+__host__ __device__ constexpr bool wgrad_half_last(int cin, bool kyRows)
 {
-    return static_cast<uint32_t>(3 * (cout / 8) * kWgradYPlane + (cin / 8 + 2) * kWgradXPlane);
+    return kyRows && 3 * cin + 1 - (wgrad_units(cin, true) - 1) * 128 <= 64;
 }
-// The A operand's 128-row blocks (16 planes each) are read whole, past the 3 * cout
-// valid rows: the last stage needs this much shared memory behind its start.
-constexpr uint32_t wgrad_a_window(int cout) { return static_cast<uint32_t>((3 * cout + 127) / 128 * 16 * kWgradYPlane); }
-// TMEM columns of one accumulator set: three kx of (cin + 16) columns, per row block.
-constexpr int wgrad_set_cols(int cin, int cout) { return 3 * ((3 * cout + 127) / 128) * (cin + 16); }
-// The tensor core's FP32 accumulation loses a little in every add, always downwards:
-// at most this many tiles (8 adds each) go into one accumulator, and the sets and
-// the CTAs' partial sums are then added in FP32 and FP64 with rounding to nearest.
-constexpr int kWgradChain = 16;
-// Floats of one CTA's partial sums.
-constexpr size_t wgrad_partial_floats(int cin, int cout) { return static_cast<size_t>(9) * (cin + 1) * cout; }
+__host__ __device__ constexpr uint32_t wgrad_plane_bytes(bool kyRows)
+{
+    return static_cast<uint32_t>((kTileH + (kyRows ? 0 : 2)) * kRowBytes);
+}
+// The constant plane behind X, up to the 128-byte boundary that a TMA copy starts on.
+__host__ __device__ constexpr uint32_t wgrad_const_bytes(bool kyRows)
+{
+    return (wgrad_plane_bytes(kyRows) + 127u) & ~127u;
+}
+// Bytes of one pipeline stage: the X copies, the constant plane, dY.
+__host__ __device__ constexpr uint32_t wgrad_stage_bytes(int cin, int cout, bool kyRows)
+{
+    return static_cast<uint32_t>((kyRows ? 3 : 1) * (cin / 8)) * wgrad_plane_bytes(kyRows) +
+           wgrad_const_bytes(kyRows) + static_cast<uint32_t>(cout / 8) * kWgradYPlane;
+}
+// The A operand's 128-row blocks (16 planes each) are read whole, past the valid
+// rows: the last stage needs this much shared memory behind its start.
+constexpr uint32_t wgrad_a_window(int cin, bool kyRows)
+{
+    return (kyRows ? wgrad_units(cin, true) * 16u * wgrad_plane_bytes(true)
+                   : 16u * wgrad_plane_bytes(false) + 2u * kRowBytes) + 64u;
+}
+// Floats of one chain's sums.
+__host__ __device__ constexpr size_t wgrad_partial_floats(int cin, int cout)
+{
+    return static_cast<size_t>(3) * cout * (3 * cin + 1);
+}
 
 // ---- fused forward: the whole network in one cooperative launch ------------------
 // Stages run in order with a grid-wide barrier after each: a convolution (its
@@ -147,7 +168,7 @@ cudaError_t launch_unet_fwd(const UnetArgs& u, int grid, uint32_t smem, cudaStre
 int unet_fwd_ctas_per_sm(uint32_t smem);
 
 // Shared-memory bytes of one launch.
-uint32_t conv_smem_bytes(int cin, int cout, int stages, bool paired, int mb);
+uint32_t conv_smem_bytes(int cin, int cout, int stages, int mb);
 
 // programmatic: launch as a programmatic dependent of the stream's previous
 // kernel (the prologue overlaps its tail; outputs are read after griddepcontrol.wait).

@@ -170,6 +170,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// The same with the descriptors in halves: the start address is the low 14 bits of the
+// low word, so a loop steps it with one 32-bit add.
+__device__ __forceinline__ void mma_bf16_lohi(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                              uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %6, 0; mov.b64 a, {%1, %2}; mov.b64 b, {%3, %4}; "
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p; }" ::"r"(d_tmem),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate));
+}
+
 // One lane of a converged warp (the same one every time). Code that issues MMAs keeps
 // the whole warp in its loops and lets only the elected lane issue: descriptors and
 // addresses then stay in uniform registers, where a loop run by one lane alone moves
