@@ -253,6 +253,16 @@ FR_HD bool w_fast(float fc, float fbz, float rbz, float& w)
     float q = fdiv_y(fc, fbz, rbz);
     float r = ffma(-q, fbz, fc);
     unsigned int qb = fbits(q);
+    w = q;
+    const float az = fbz < 0.f ? -fbz : fbz, ar = r < 0.f ? -r : r;
+    if (qb & 0x7fffffu)
+    {
+        // Nearly every quotient clears the boundary by far: h = ulp(q) / 2, and |r| below
+        // |bz| (h (1 - 2^-19) - 2^-50) is below |bz| (h - E) whatever the three roundings
+        // (2^-24 each) do.
+        const float h = bitsf((qb & 0x7f800000u) - (24u << 23));
+        if (ar < az * ffma(h, 0.99999809265136718750f, -8.8817841970012523234e-16f)) return true;
+    }
     unsigned int e = qb >> 23;  // q in [2^-24, 1]: e in [103, 127]
     bool below = (r != 0.f) && ((r > 0.f) != (fbz > 0.f));
     bool pow2 = (qb & 0x7fffffu) == 0u;
@@ -262,8 +272,6 @@ FR_HD bool w_fast(float fc, float fbz, float rbz, float& w)
     int mexp = 76 - (int)(he - 24u);                         // log2(E / g) = -51 - log2(g)
     float m = mexp <= 0 ? 1.f : bitsf((unsigned)(127 + mexp) << 23);
     float T = (16777216.f - m) * g;                          // exact: integer < 2^24 times 2^k
-    float az = fbz < 0.f ? -fbz : fbz, ar = r < 0.f ? -r : r;
-    w = q;
     return ffma(az, -T, ar) < 0.f;
 }
 
@@ -532,6 +540,76 @@ FR_HD bool bary(const RTri& t, int px, int py, float& b0, float& b1, float& b2)
     return true;
 }
 
+// ---- the setup kernel's small triangles --------------------------------------------
+// A fast-class triangle with small coordinates as three affine edge functions of the
+// pixel's offset (lx, ly) in its box, all multiplied by the sign of bz so that they are
+// >= 0 inside: e1 = |ex|, e2 = |ey|, c = |bz| - e1 - e2. The true values of all three
+// fit int32 (products of factors below 2^15), so wrapped 32-bit arithmetic gives them
+// exactly, and weights from the magnitudes are bary()'s: every step of it is symmetric
+// in the common sign.
+struct SmallEdges
+{
+    int a1, bx1, by1;  // e1 = a1 + bx1 lx + by1 ly
+    int a2, bx2, by2;  // e2
+    int B;             // |bz|, 1 .. 2^24 - 1
+};
+
+FR_HD SmallEdges small_edges(const RTri& t, int X0, int Y0)
+{
+    const int s = t.bz < 0 ? -1 : 1;
+    const int s0x = t.x[1] - t.x[0], s0y = t.x[2] - t.x[0], s0z = t.x[0] - X0;
+    const int s1x = t.y[1] - t.y[0], s1y = t.y[2] - t.y[0], s1z = t.y[0] - Y0;
+    SmallEdges e;
+    e.a1 = s * (s0y * s1z - s0z * s1y), e.bx1 = s * s1y, e.by1 = -s * s0y;
+    e.a2 = s * (s0z * s1x - s0x * s1z), e.bx2 = -s * s1x, e.by2 = s * s0x;
+    e.B = s * (int)t.bz;
+    return e;
+}
+
+FR_HD int affine_wrapped(int a, int bx, int by, int lx, int ly)
+{
+    return (int)((unsigned)a + (unsigned)bx * (unsigned)lx + (unsigned)by * (unsigned)ly);
+}
+
+// Row floor(l / w) of pixel l of a box of width w: rw = RN(1 / w), l < 2^22. (l + 0.5) / w
+// is at least 0.5 / w from an integer, the rounded product off by less than l 2^-22 / w.
+FR_HD int box_row(int l, float rw)
+{
+#ifdef __CUDA_ARCH__
+    // l + 0.5 and the floor through the float format, off the conversion unit
+    const float f = __fsub_rn(__int_as_float(0x4b000000 | l), 8388607.5f);
+    return __float_as_int(__fadd_rd(__fmul_rn(f, rw), 8388608.f)) - 0x4b000000;
+#else
+    return (int)floorf(((float)l + 0.5f) * rw);
+#endif
+}
+
+// bary<.., false> from the edge values of a covered pixel off edge BC (c > 0).
+FR_HD bool bary_off_edge(int e1, int e2, int B, float rB, float& b0, float& b1, float& b2)
+{
+    const float fB = (float)B;
+    b1 = fdiv_y((float)e1, fB, rB);
+    b2 = fdiv_y((float)e2, fB, rB);
+    if (!w_fast((float)(B - e1 - e2), fB, rB, b0))
+    {
+        float d0, d1, d2;  // near a rounding boundary: the double path decides
+        if (!bary_from_ints_double(e1, e2, B, d0, d1, d2)) return false;
+        b0 = d0;
+    }
+    return true;
+}
+
+// The same on edge BC (c == 0), with the triangle's RN53(1 / B) = m53 2^-s53.
+FR_HD bool bary_on_edge(int e1, int e2, int B, float rB, unsigned long long m53, int s53, float& b0, float& b1,
+                        float& b2)
+{
+    const float fB = (float)B;
+    b1 = fdiv_y((float)e1, fB, rB);
+    b2 = fdiv_y((float)e2, fB, rB);
+    b0 = w_on_edge((unsigned)e1, (unsigned)e2, m53, s53);
+    return !(b0 < 0.f);
+}
+
 // (float)(c * (double)p) for a positive normal double constant c with 53-bit
 // significand cm and exponent ce (c = cm * 2^ce), computed exactly in integers:
 // the 77-bit product is rounded to 53 bits, then to 24 bits, both to nearest
@@ -586,13 +664,17 @@ FR_HD float mul_f_d_round(float p, double c, unsigned long long cm, int ce)
 }
 
 // Dot(bary, depths) (geometry.h:881-889): accumulated from 0.f in order.
-FR_HD float depth_of(const RTri& t, float b0, float b1, float b2)
+FR_HD float depth_dot(float d0, float d1, float d2, float b0, float b1, float b2)
 {
     float r = 0.f;
-    r += b0 * t.d[0];
-    r += b1 * t.d[1];
-    r += b2 * t.d[2];
+    r += b0 * d0;
+    r += b1 * d1;
+    r += b2 * d2;
     return r;
+}
+FR_HD float depth_of(const RTri& t, float b0, float b1, float b2)
+{
+    return depth_dot(t.d[0], t.d[1], t.d[2], b0, b1, b2);
 }
 
 // 64-bit visibility key: order-preserving depth bits above the draw index, so

@@ -175,16 +175,25 @@ int setup_group(int tris)
 // Five CTAs per SM (at most 51 registers a thread; 48 without spills): with the two
 // queues, an unbounded allocation took 52 and four CTAs, and in the concurrent frame
 // the extra resident warps let the shadow setup overlap the camera chain better.
+//
+// The pixel loop's integer work (box division, three edge values) was the kernel's
+// bound (ALU pipe 59 %, issue 74 %): the edges are affine functions on the
+// multiply-add pipe, the row comes from the float format, and the queues carry the
+// edge values so that the exact weights start from them.
 __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const int4* __restrict__ scr, RasterParams rp,
                                                          RasterScratch rs, int group)
 {
     // the warp's small triangles, compacted in draw order (slot = rank among them)
-    __shared__ frx::RTri sh[kSetupThreads];
-    __shared__ int4 shb[kSetupThreads];  // (x0, y0, w, triangle)
-    __shared__ float shr[kSetupThreads]; // 1 / w
-    __shared__ int shs[kSetupThreads];   // first pixel in the warp's flattened pixel list
-    __shared__ int shq[2][kSetupThreads / 32][64];  // per-warp queues of covered pixels (slot, y, x):
-                                                    // off edge BC, on edge BC
+    __shared__ int4 shE0[kSetupThreads];    // edge functions: a1, bx1, by1, a2
+    __shared__ int4 shE1[kSetupThreads];    // bx2, by2, |bz|, box width
+    __shared__ int4 shD[kSetupThreads];     // first pixel in the warp's flattened list, box origin's
+                                            // index in the target, 1 / width, triangle
+    __shared__ float4 shF[kSetupThreads];   // RN(1 / |bz|), the vertex depths
+    __shared__ unsigned long long shM[kSetupThreads];  // RN53(1 / |bz|): significand
+    __shared__ int shS[kSetupThreads];                 // and exponent
+    // per-warp queues of covered pixels, off edge BC and on it: slot and pixel, e1 and e2
+    __shared__ int shq[2][kSetupThreads / 32][64];
+    __shared__ int2 she[2][kSetupThreads / 32][64];
     const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
     const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * group + lane;
     int area = 0;
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
             int x0, x1, y0, y1;
             bbox(r, rp.W, rp.H, x0, x1, y0, y1);
             long long a = (long long)(x1 - x0 + 1) * (y1 - y0 + 1);
-            if (r.cls == frx::kTriFast && a <= rp.smallArea && rp.W <= 8192 && rp.H <= 8192)
+            if (r.cls == frx::kTriFast && r.small && a <= rp.smallArea && rp.W <= 8192 && rp.H <= 8192)
             {
                 area = (int)a;
                 sx0 = x0, sy0 = y0, sw = x1 - x0 + 1;
@@ -242,10 +251,14 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
     const int slot = __popc(__ballot_sync(0xffffffffu, area > 0) & ((1u << lane) - 1u));
     if (area > 0)
     {
-        sh[wbase + slot] = r;
-        shb[wbase + slot] = make_int4(sx0, sy0, sw, t);
-        shr[wbase + slot] = 1.f / (float)sw;
-        shs[wbase + slot] = incl - area;
+        const frx::SmallEdges e = frx::small_edges(r, sx0, sy0);
+        const int k = wbase + slot;
+        shE0[k] = make_int4(e.a1, e.bx1, e.by1, e.a2);
+        shE1[k] = make_int4(e.bx2, e.by2, e.B, sw);
+        shD[k] = make_int4(incl - area, sy0 * rp.W + sx0, __float_as_int(1.f / (float)sw), t);
+        shF[k] = make_float4(fabsf(r.rbz), r.d[0], r.d[1], r.d[2]);
+        shM[k] = r.m53;
+        shS[k] = r.s53;
     }
     __syncwarp();
     // Pixels that pass the cheap integer coverage pre-test are queued (per warp,
@@ -253,8 +266,27 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
     // so the expensive path never idles lanes on uncovered pixels. Pixels on edge
     // BC (whose weight takes the exact on-edge path) have a queue of their own, so
     // neither batch form carries the other's code path.
-    int* queue = shq[0][threadIdx.x >> 5];
-    int* queueE = shq[1][threadIdx.x >> 5];
+    int *queue = shq[0][threadIdx.x >> 5], *queueE = shq[1][threadIdx.x >> 5];
+    int2 *edges = she[0][threadIdx.x >> 5], *edgesE = she[1][threadIdx.x >> 5];
+    // the exact weights, depth and key of one queued pixel
+    auto off_edge = [&](int entry, int2 e) {
+        const int k = wbase + (entry >> 26);
+        const float4 f = shF[k];
+        float b0, b1, b2;
+        if (!frx::bary_off_edge(e.x, e.y, shE1[k].z, f.x, b0, b1, b2)) return;
+        const float d = frx::depth_dot(f.y, f.z, f.w, b0, b1, b2);
+        if (!frx::depth_passes_clear(d)) return;
+        atomicMin(rs.keys + (entry & 0x3ffffff), frx::make_key(d, (unsigned)shD[k].w));  // result unused: RED.MIN
+    };
+    auto on_edge = [&](int entry, int2 e) {
+        const int k = wbase + (entry >> 26);
+        const float4 f = shF[k];
+        float b0, b1, b2;
+        if (!frx::bary_on_edge(e.x, e.y, shE1[k].z, f.x, shM[k], shS[k], b0, b1, b2)) return;
+        const float d = frx::depth_dot(f.y, f.z, f.w, b0, b1, b2);
+        if (!frx::depth_passes_clear(d)) return;
+        atomicMin(rs.keys + (entry & 0x3ffffff), frx::make_key(d, (unsigned)shD[k].w));
+    };
     int qn = 0, qe = 0;
     // The owner of pixel p of the flattened list is the last triangle that starts
     // at or before p: one OR-reduction marks the triangles starting in this
@@ -262,6 +294,7 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
     // starts up to the lane (slots follow the start order).
     int owner = -1;
     const int rel0 = incl - area;
+    const unsigned lt = (1u << lane) - 1u;
     for (int base = 0; base < total; base += 32)
     {
         const int p = base + lane;
@@ -269,60 +302,57 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
         const unsigned starts = __reduce_or_sync(0xffffffffu, (area > 0 && (unsigned)rel < 32u) ? 1u << rel : 0u);
         const int j = owner + __popc(starts & ((2u << lane) - 1u));
         owner += __popc(starts);
-        int kind = 0;
-        int px = 0, py = 0;
+        int e1 = -1, e2 = 0, c = 0, entry = 0;
         if (p < total)
         {
-            int local = p - shs[wbase + j];
-            int4 b = shb[wbase + j];
-            int q = (int)((float)local * shr[wbase + j]);
-            int rem = local - q * b.z;
-            if (rem < 0) --q, rem += b.z;
-            else if (rem >= b.z) ++q, rem -= b.z;
-            px = b.x + rem, py = b.y + q;
-            kind = frx::pretest_kind(sh[wbase + j], px, py);
+            const int4 E0 = shE0[wbase + j], E1 = shE1[wbase + j], D = shD[wbase + j];
+            const int l = p - D.x;
+            const int ly = frx::box_row(l, __int_as_float(D.z));
+            const int lx = l - ly * E1.w;
+            e1 = frx::affine_wrapped(E0.x, E0.y, E0.z, lx, ly);
+            e2 = frx::affine_wrapped(E0.w, E1.x, E1.y, lx, ly);
+            c = E1.z - e1 - e2;
+            entry = (j << 26) | (D.y + ly * rp.W + lx);
         }
-        const unsigned lt = (1u << lane) - 1u;
-        const unsigned m = __ballot_sync(0xffffffffu, kind == 1), me = __ballot_sync(0xffffffffu, kind == 2);
-        const int entry = (j << 26) | (py << 13) | px;
-        if (kind == 1) queue[qn + __popc(m & lt)] = entry;
-        if (kind == 2) queueE[qe + __popc(me & lt)] = entry;
+        const bool cov = (e1 | e2 | c) >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, cov && c != 0), me = __ballot_sync(0xffffffffu, cov && c == 0);
+        if (cov && c != 0)
+        {
+            const int at = qn + __popc(m & lt);
+            queue[at] = entry;
+            edges[at] = make_int2(e1, e2);
+        }
         qn += __popc(m);
-        qe += __popc(me);
+        if (me)  // uniform
+        {
+            if (cov && c == 0)
+            {
+                const int at = qe + __popc(me & lt);
+                queueE[at] = entry;
+                edgesE[at] = make_int2(e1, e2);
+            }
+            qe += __popc(me);
+        }
         __syncwarp();
         if (qn >= 32)
         {
-            int e = queue[lane];
-            int jj = e >> 26;
-            fragment_key<1>(sh[wbase + jj], shb[wbase + jj].w, e & 8191, (e >> 13) & 8191, rp.W, rs.keys);
+            off_edge(queue[lane], edges[lane]);
             __syncwarp();
-            if (lane < qn - 32) queue[lane] = queue[32 + lane];
+            if (lane < qn - 32) queue[lane] = queue[32 + lane], edges[lane] = edges[32 + lane];
             qn -= 32;
             __syncwarp();
         }
         if (qe >= 32)
         {
-            int e = queueE[lane];
-            int jj = e >> 26;
-            fragment_key<2>(sh[wbase + jj], shb[wbase + jj].w, e & 8191, (e >> 13) & 8191, rp.W, rs.keys);
+            on_edge(queueE[lane], edgesE[lane]);
             __syncwarp();
-            if (lane < qe - 32) queueE[lane] = queueE[32 + lane];
+            if (lane < qe - 32) queueE[lane] = queueE[32 + lane], edgesE[lane] = edgesE[32 + lane];
             qe -= 32;
             __syncwarp();
         }
     }
-    if (lane < qn)
-    {
-        int e = queue[lane];
-        int jj = e >> 26;
-        fragment_key<1>(sh[wbase + jj], shb[wbase + jj].w, e & 8191, (e >> 13) & 8191, rp.W, rs.keys);
-    }
-    if (lane < qe)
-    {
-        int e = queueE[lane];
-        int jj = e >> 26;
-        fragment_key<2>(sh[wbase + jj], shb[wbase + jj].w, e & 8191, (e >> 13) & 8191, rp.W, rs.keys);
-    }
+    if (lane < qn) off_edge(queue[lane], edges[lane]);
+    if (lane < qe) on_edge(queueE[lane], edgesE[lane]);
 }
 
 // Medium triangles: the grid's warps are shared out among them, each triangle's box
