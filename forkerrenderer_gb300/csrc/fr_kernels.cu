@@ -157,7 +157,9 @@ __global__ void k_transform_light(DevScene S, FrameConst F, int4* scrL)
 // triangle. Triangles whose clamped bounding box has at most smallArea pixels
 // are drawn right here, cooperatively by the warp: the 32 boxes are flattened
 // (warp prefix sum of their areas) and dealt out pixel by pixel to the lanes,
-// so every lane stays busy whatever the mix of triangle sizes. Larger fast
+// so every lane stays busy whatever the mix of triangle sizes; a lane takes two
+// neighbouring pixels of a row, the second one step further along the edge functions
+// (one pixel a lane: 73 us for 409,602 triangles in a 2048^2 map, two: 66). Larger fast
 // triangles go to the medium list (one or more warps each), the rest to the tile bins.
 constexpr int kSetupThreads = 256;
 
@@ -186,14 +188,14 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
     // the warp's small triangles, compacted in draw order (slot = rank among them)
     __shared__ int4 shE0[kSetupThreads];    // edge functions: a1, bx1, by1, a2
     __shared__ int4 shE1[kSetupThreads];    // bx2, by2, |bz|, box width
-    __shared__ int4 shD[kSetupThreads];     // first pixel in the warp's flattened list, box origin's
-                                            // index in the target, 1 / width, triangle
+    __shared__ int4 shD[kSetupThreads];     // first pair in the warp's flattened list, box origin's
+                                            // index in the target, 1 / pairs a row, triangle
     __shared__ float4 shF[kSetupThreads];   // RN(1 / |bz|), the vertex depths
     __shared__ unsigned long long shM[kSetupThreads];  // RN53(1 / |bz|): significand
     __shared__ int shS[kSetupThreads];                 // and exponent
     // per-warp queues of covered pixels, off edge BC and on it: slot and pixel, e1 and e2
-    __shared__ int shq[2][kSetupThreads / 32][64];
-    __shared__ int2 she[2][kSetupThreads / 32][64];
+    __shared__ int shq[2][kSetupThreads / 32][96];
+    __shared__ int2 she[2][kSetupThreads / 32][96];
     const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
     const int t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * group + lane;
     int area = 0;
@@ -211,8 +213,8 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
             long long a = (long long)(x1 - x0 + 1) * (y1 - y0 + 1);
             if (r.cls == frx::kTriFast && r.small && a <= rp.smallArea && rp.W <= 8192 && rp.H <= 8192)
             {
-                area = (int)a;
                 sx0 = x0, sy0 = y0, sw = x1 - x0 + 1;
+                area = ((sw + 1) >> 1) * (y1 - y0 + 1);  // pixel pairs
             }
             else if (r.cls == frx::kTriFast && a <= rp.mediumArea)
             {
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
         const int k = wbase + slot;
         shE0[k] = make_int4(e.a1, e.bx1, e.by1, e.a2);
         shE1[k] = make_int4(e.bx2, e.by2, e.B, sw);
-        shD[k] = make_int4(incl - area, sy0 * rp.W + sx0, __float_as_int(1.f / (float)sw), t);
+        shD[k] = make_int4(incl - area, sy0 * rp.W + sx0, __float_as_int(1.f / (float)((sw + 1) >> 1)), t);
         shF[k] = make_float4(fabsf(r.rbz), r.d[0], r.d[1], r.d[2]);
         shM[k] = r.m53;
         shS[k] = r.s53;
@@ -288,9 +290,9 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
         atomicMin(rs.keys + (entry & 0x3ffffff), frx::make_key(d, (unsigned)shD[k].w));
     };
     int qn = 0, qe = 0;
-    // The owner of pixel p of the flattened list is the last triangle that starts
+    // The owner of pair p of the flattened list is the last triangle that starts
     // at or before p: one OR-reduction marks the triangles starting in this
-    // 32-pixel step, and the owner is the previous step's last owner plus the
+    // 32-pair step, and the owner is the previous step's last owner plus the
     // starts up to the lane (slots follow the start order).
     int owner = -1;
     const int rel0 = incl - area;
@@ -302,20 +304,25 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
         const unsigned starts = __reduce_or_sync(0xffffffffu, (area > 0 && (unsigned)rel < 32u) ? 1u << rel : 0u);
         const int j = owner + __popc(starts & ((2u << lane) - 1u));
         owner += __popc(starts);
-        int e1 = -1, e2 = 0, c = 0, entry = 0;
+        int e1 = -1, e2 = 0, c = 0, entry = 0, f1 = -1, f2 = 0, g = 0;
         if (p < total)
         {
             const int4 E0 = shE0[wbase + j], E1 = shE1[wbase + j], D = shD[wbase + j];
             const int l = p - D.x;
             const int ly = frx::box_row(l, __int_as_float(D.z));
-            const int lx = l - ly * E1.w;
+            const int lx = 2 * (l - ly * ((E1.w + 1) >> 1));
             e1 = frx::affine_wrapped(E0.x, E0.y, E0.z, lx, ly);
             e2 = frx::affine_wrapped(E0.w, E1.x, E1.y, lx, ly);
             c = E1.z - e1 - e2;
             entry = (j << 26) | (D.y + ly * rp.W + lx);
+            // the pair's second pixel, one step in x (none past the box)
+            f1 = lx + 1 < E1.w ? (int)((unsigned)e1 + (unsigned)E0.y) : -1;
+            f2 = (int)((unsigned)e2 + (unsigned)E1.x);
+            g = E1.z - f1 - f2;
         }
-        const bool cov = (e1 | e2 | c) >= 0;
-        const unsigned m = __ballot_sync(0xffffffffu, cov && c != 0), me = __ballot_sync(0xffffffffu, cov && c == 0);
+        const bool cov = (e1 | e2 | c) >= 0, cov2 = (f1 | f2 | g) >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, cov && c != 0), m2 = __ballot_sync(0xffffffffu, cov2 && g != 0);
+        const unsigned me = __ballot_sync(0xffffffffu, (cov && c == 0) || (cov2 && g == 0));
         if (cov && c != 0)
         {
             const int at = qn + __popc(m & lt);
@@ -323,33 +330,43 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
             edges[at] = make_int2(e1, e2);
         }
         qn += __popc(m);
+        if (cov2 && g != 0)
+        {
+            const int at = qn + __popc(m2 & lt);
+            queue[at] = entry + 1;
+            edges[at] = make_int2(f1, f2);
+        }
+        qn += __popc(m2);
         if (me)  // uniform
         {
+            const unsigned ma = __ballot_sync(0xffffffffu, cov && c == 0), mb = __ballot_sync(0xffffffffu, cov2 && g == 0);
             if (cov && c == 0)
             {
-                const int at = qe + __popc(me & lt);
+                const int at = qe + __popc(ma & lt);
                 queueE[at] = entry;
                 edgesE[at] = make_int2(e1, e2);
             }
-            qe += __popc(me);
+            qe += __popc(ma);
+            if (cov2 && g == 0)
+            {
+                const int at = qe + __popc(mb & lt);
+                queueE[at] = entry + 1;
+                edgesE[at] = make_int2(f1, f2);
+            }
+            qe += __popc(mb);
         }
         __syncwarp();
-        if (qn >= 32)
+        while (qn >= 32)  // the newest 32, so that nothing moves
         {
-            off_edge(queue[lane], edges[lane]);
-            __syncwarp();
-            if (lane < qn - 32) queue[lane] = queue[32 + lane], edges[lane] = edges[32 + lane];
             qn -= 32;
-            __syncwarp();
+            off_edge(queue[qn + lane], edges[qn + lane]);
         }
-        if (qe >= 32)
+        while (qe >= 32)
         {
-            on_edge(queueE[lane], edgesE[lane]);
-            __syncwarp();
-            if (lane < qe - 32) queueE[lane] = queueE[32 + lane], edgesE[lane] = edgesE[32 + lane];
             qe -= 32;
-            __syncwarp();
+            on_edge(queueE[qe + lane], edgesE[qe + lane]);
         }
+        __syncwarp();
     }
     if (lane < qn) off_edge(queue[lane], edges[lane]);
     if (lane < qe) on_edge(queueE[lane], edgesE[lane]);
