@@ -61,7 +61,8 @@ bool alloc_raster(Alloc& A, frk::RasterScratch& rs, int W, int H, int T, long lo
     rs.largeTris = A.get<frx::RTri>(rs.triCap);
     rs.largeIdx = A.get<int>(rs.triCap);
     rs.largeAux = A.get<float4>(rs.triCap);
-    rs.counters = A.get<int>(4);
+    rs.counters = A.get<int>(5);
+    rs.ticket = reinterpret_cast<unsigned*>(rs.counters + 4);
     rs.tileCount = A.get<int>(tiles);
     rs.tileStart = A.get<int>(tiles + 1);
     rs.tileFill = A.get<int>(tiles);
@@ -190,17 +191,17 @@ int record(fr_batch* b)
     for (auto& L : b->lights)
     {
         cudaStream_t s = b->br[next++ % kBranches];
-        frk::launch_transform_light(L.S, L.F, L.scrL, s);
         frk::RasterParams rp = base;
         rp.W = L.F.SW, rp.H = L.F.SH;
+        frk::launch_transform_light(L.S, L.F, L.scrL, rp, L.rs, s);
         frk::launch_raster(L.S, L.scrL, rp, L.rs, s, launches, false);
     }
     for (auto& V : b->views)
     {
         cudaStream_t s = b->br[next++ % kBranches];
-        frk::launch_transform_camera(b->viewScene, V.F, V.vo, s);
         frk::RasterParams rp = base;
         rp.W = V.F.W, rp.H = V.F.H;
+        frk::launch_transform_camera(b->viewScene, V.F, V.vo, rp, V.rs, s);
         frk::launch_raster(b->viewScene, V.vo.scr, rp, V.rs, s, launches, false);
     }
     for (int i = 0; i < kBranches; ++i)

@@ -146,13 +146,14 @@ int ensure_frame(fr_ctx* ctx, int W, int H, int SW, int SH)
     ctx->keysCap = P;
     FR_TRY(falloc(ctx, ctx->keys, P));
     FR_TRY(falloc(ctx, ctx->keysShadow, SP > 0 ? SP : 1));
-    FR_TRY(falloc(ctx, ctx->counters, 8));
-    auto scratch = [&](frk::RasterScratch& rs, unsigned long long* keys, int tiles, int* counters) -> int {
+    FR_TRY(falloc(ctx, ctx->counters, 10));
+    auto scratch = [&](frk::RasterScratch& rs, unsigned long long* keys, int tiles, int* counters, int* ticket) -> int {
         const long long binCap =
             ctx->cfg.bin_capacity > 0 ? ctx->cfg.bin_capacity : (long long)tiles * 16 + (1 << 22);
         rs = frk::RasterScratch{};
         rs.keys = keys;
         rs.counters = counters;
+        rs.ticket = reinterpret_cast<unsigned*>(ticket);
         rs.triCap = T > 0 ? T : 1;
         rs.binCap = binCap;
         FR_TRY(falloc(ctx, rs.mediumTris, rs.triCap));
@@ -166,10 +167,11 @@ int ensure_frame(fr_ctx* ctx, int W, int H, int SW, int SH)
         FR_TRY(falloc(ctx, rs.binTri, (size_t)binCap));
         return FR_OK;
     };
-    FR_TRY(scratch(ctx->rsShadow, ctx->keysShadow, tiles_of(SW, SH) > 0 ? tiles_of(SW, SH) : 1, ctx->counters));
+    FR_TRY(scratch(ctx->rsShadow, ctx->keysShadow, tiles_of(SW, SH) > 0 ? tiles_of(SW, SH) : 1, ctx->counters,
+                   ctx->counters + 8));
     // the shadow map's fused resolve reads each winning triangle's record (one load round trip)
     FR_TRY(falloc(ctx, ctx->rsShadow.triRec, 2 * (size_t)ctx->rsShadow.triCap));
-    FR_TRY(scratch(ctx->rsCam, ctx->keys, tiles_of(W, H), ctx->counters + 4));
+    FR_TRY(scratch(ctx->rsCam, ctx->keys, tiles_of(W, H), ctx->counters + 4, ctx->counters + 9));
     FR_TRY(falloc(ctx, ctx->gb.a, P));
     FR_TRY(falloc(ctx, ctx->gb.b, P));
     FR_TRY(falloc(ctx, ctx->gb.c, P));
@@ -182,7 +184,7 @@ int ensure_frame(fr_ctx* ctx, int W, int H, int SW, int SH)
     FR_TRY(falloc(ctx, ctx->ssaoBg16, 16));
     if (ctx->cfg.keep_float_frame) FR_TRY(falloc(ctx, ctx->frameF, 3 * P));
     else ctx->frameF = nullptr;
-    FR_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(int) * 8, ctx->stream));
+    FR_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(int) * 10, ctx->stream));
     FR_CUDA(cudaMemsetAsync(ctx->shadow, 0, sizeof(float) * SP, ctx->stream));
     // frames may run on a caller's stream and on the second stream: the cleared
     // buffers are ready before either sees them
@@ -295,8 +297,8 @@ int begin_frame(fr_ctx* ctx, const fr_frame_params* params)
 int do_shadow(fr_ctx* ctx, cudaStream_t st)
 {
     if (!ctx->info.shadow_on) return FR_OK;
-    frk::launch_transform_light(ctx->S, ctx->fc, ctx->scrL, st);
     frk::RasterParams rp{ctx->SW, ctx->SH, ctx->cfg.small_tri_area, ctx->cfg.medium_tri_area};
+    frk::launch_transform_light(ctx->S, ctx->fc, ctx->scrL, rp, ctx->rsShadow, st);
     frk::launch_raster(ctx->S, ctx->scrL, rp, ctx->rsShadow, st, ctx->launches, true, ctx->shadow);
     ctx->launches += 1;
     FR_CUDA(cudaGetLastError());
@@ -305,8 +307,8 @@ int do_shadow(fr_ctx* ctx, cudaStream_t st)
 
 int do_camera(fr_ctx* ctx, cudaStream_t st, bool forwardPass)
 {
-    frk::launch_transform_camera(ctx->S, ctx->fc, ctx->vo, st);
     frk::RasterParams rp{ctx->W, ctx->H, ctx->cfg.small_tri_area, ctx->cfg.medium_tri_area};
+    frk::launch_transform_camera(ctx->S, ctx->fc, ctx->vo, rp, ctx->rsCam, st);
     frk::launch_raster(ctx->S, ctx->vo.scr, rp, ctx->rsCam, st, ctx->launches);
     if (forwardPass)
         frk::launch_forward_shade(ctx->S, ctx->fc, ctx->vo, ctx->keys, ctx->shadow, ctx->gb.depth, ctx->frame8,

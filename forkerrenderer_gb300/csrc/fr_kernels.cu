@@ -93,11 +93,34 @@ __device__ __forceinline__ void fragment_key(const frx::RTri& r, int t, int px, 
 
 // ---- vertex stages ------------------------------------------------------------------------
 
+// The raster scratch a vertex stage clears beside its own work (three memset launches
+// less in front of every pass).
+struct RasterClear
+{
+    unsigned long long* keys;
+    long long numKeys;
+    int *counters, *tileCount;
+    unsigned* ticket;
+    int tiles;
+};
+
+__device__ __forceinline__ void clear_raster(const RasterClear& c)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)gridDim.x * blockDim.x;
+    const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);  // two empty keys
+    for (long long i = t; i < c.numKeys / 2; i += n) reinterpret_cast<uint4*>(c.keys)[i] = ones;
+    if (t == 0 && (c.numKeys & 1)) c.keys[c.numKeys - 1] = frx::kEmptyKey;
+    for (long long i = t; i < c.tiles; i += n) c.tileCount[i] = 0;
+    if (t < 4) c.counters[t] = 0;
+    if (t == 0) *c.ticket = 0u;
+}
+
 // Camera vertex shader (gshader.h:41-92 / phongshader.h:35-85 / pbrshader.h:35-85)
 // per unique vertex, then the viewport transform and int snap of DrawTriangle
 // (forkergl.cpp:244-249). Normals are transformed per unique normal.
-__global__ void k_transform_camera(DevScene S, FrameConst F, VertexOut vo)
+__global__ void k_transform_camera(DevScene S, FrameConst F, VertexOut vo, RasterClear rc)
 {
+    clear_raster(rc);
     int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < S.numVerts)
     {
@@ -139,8 +162,9 @@ __global__ void k_transform_camera(DevScene S, FrameConst F, VertexOut vo)
 
 // DepthShader::ProcessVertex (depthshader.h:21-28): (L * M) * v, / w, then the
 // shadow viewport. .w keeps NDC z for the shadow-map value.
-__global__ void k_transform_light(DevScene S, FrameConst F, int4* scrL)
+__global__ void k_transform_light(DevScene S, FrameConst F, int4* scrL, RasterClear rc)
 {
+    clear_raster(rc);
     int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= S.numVerts) return;
     const DevModel& Md = S.models[S.vmodel[v]];
@@ -377,7 +401,12 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
 // left a box of 8,192 pixels to 256 dependent steps: 61 us for the ground's two triangles
 // in a 161 x 97 frame (now 6 us), 86 us for the medium triangles of a 4096^2 shadow map
 // of 2.05 million (now 67 us).
-__global__ void k_raster_medium(RasterParams rp, RasterScratch rs)
+__device__ __noinline__ void medium_general(const frx::RTri& r, int t, int px, int py, int W, unsigned long long* keys)
+{
+    fragment_key(r, t, px, py, W, keys);
+}
+
+__device__ __forceinline__ void raster_medium(const RasterParams& rp, const RasterScratch& rs)
 {
     const int n = min(rs.counters[0], rs.triCap);
     if (n == 0) return;
@@ -393,16 +422,42 @@ __global__ void k_raster_medium(RasterParams rp, RasterScratch rs)
         int x0, x1, y0, y1;
         bbox(r, rp.W, rp.H, x0, x1, y0, y1);
         const int w = x1 - x0 + 1, area = w * (y1 - y0 + 1);
-        for (int p = part * 32 + lane; p < area; p += per * 32) fragment_key(r, t, x0 + p % w, y0 + p / w, rp.W, rs.keys);
+        if (!r.small)
+        {
+            for (int p = part * 32 + lane; p < area; p += per * 32)
+                medium_general(r, t, x0 + p % w, y0 + p / w, rp.W, rs.keys);
+            continue;
+        }
+        // the setup kernel's edge functions and weights (box_row: area <= 2^20)
+        const frx::SmallEdges e = frx::small_edges(r, x0, y0);
+        const float rw = 1.f / (float)w, rB = fabsf(r.rbz);
+        for (int p = part * 32 + lane; p < area; p += per * 32)
+        {
+            const int ly = frx::box_row(p, rw), lx = p - ly * w;
+            const int e1 = frx::affine_wrapped(e.a1, e.bx1, e.by1, lx, ly);
+            const int e2 = frx::affine_wrapped(e.a2, e.bx2, e.by2, lx, ly);
+            const int c = e.B - e1 - e2;
+            if ((e1 | e2 | c) < 0) continue;
+            if (c == 0)
+            {
+                medium_general(r, t, x0 + lx, y0 + ly, rp.W, rs.keys);
+                continue;
+            }
+            float b0, b1, b2;
+            if (!frx::bary_off_edge(e1, e2, e.B, rB, b0, b1, b2)) continue;
+            const float d = frx::depth_of(r, b0, b1, b2);
+            if (!frx::depth_passes_clear(d)) continue;
+            atomicMin(rs.keys + (size_t)(y0 + ly) * rp.W + x0 + lx, frx::make_key(d, (unsigned)t));
+        }
     }
 }
 
-// Tile binning of large triangles: pass 0 counts (triangle, tile) pairs, pass 1
-// scatters triangle list indices into the per-tile ranges. Work items are
-// (triangle, tile row) pairs, one warp each, so a triangle spanning thousands
-// of tiles is binned by many warps at once. With at most kDirectLarge large
+// Tile binning of large triangles: (triangle, tile) pairs are counted per tile, the
+// counts scanned and the triangle list indices scattered into the per-tile ranges.
+// Work items are (triangle, tile row) pairs, one warp each, so a triangle spanning
+// thousands of tiles is binned by many warps at once. With at most kDirectLarge large
 // triangles the fine raster takes them all (each gated by its box per pixel,
-// the same pixels the bins would give it) and the binning kernels do nothing.
+// the same pixels the bins would give it) and there is no binning.
 constexpr int kDirectLarge = 8;
 
 __device__ __forceinline__ bool large_direct(const RasterScratch& rs)
@@ -410,9 +465,10 @@ __device__ __forceinline__ bool large_direct(const RasterScratch& rs)
     return min(rs.counters[1], rs.triCap) <= kDirectLarge;
 }
 
-__global__ void k_bin(RasterParams rp, RasterScratch rs, int scatter)
+// fn(large triangle, tile) for every pair of this warp's items.
+template <typename Fn>
+__device__ __forceinline__ void for_large_tiles(const RasterParams& rp, const RasterScratch& rs, Fn fn)
 {
-    if (large_direct(rs)) return;
     int n = min(rs.counters[1], rs.triCap);
     int lane = threadIdx.x & 31;
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -429,52 +485,26 @@ __global__ void k_bin(RasterParams rp, RasterScratch rs, int scatter)
         int ty = y0 / kTile + row;
         if (ty > y1 / kTile) continue;
         int tx0 = x0 / kTile, tx1 = x1 / kTile;
-        for (int tx = tx0 + lane; tx <= tx1; tx += 32)
-        {
-            int tile = ty * ntx + tx;
-            if (!scatter)
-                atomicAdd(&rs.tileCount[tile], 1);
-            else
-            {
-                long long pos = (long long)rs.tileStart[tile] + atomicAdd(&rs.tileFill[tile], 1);
-                if (pos < rs.binCap) rs.binTri[pos] = i;
-            }
-        }
+        for (int tx = tx0 + lane; tx <= tx1; tx += 32) fn(i, ty * ntx + tx);
     }
 }
 
-// Exclusive scan of the tile counts: one CTA walks the array in coalesced
-// chunks of 1024, scanning each chunk with warp shuffles and carrying the total.
-__global__ void __launch_bounds__(1024) k_bin_scan(RasterScratch rs, int tiles)
+// Exclusive scan of the tile counts by one CTA of kMediumThreads: it walks the array
+// in coalesced chunks, scanning each with warp shuffles and carrying the total.
+constexpr int kMediumThreads = 256;
+__device__ __forceinline__ void bin_scan(const RasterScratch& rs, int tiles)
 {
-    if (large_direct(rs)) return;  // uniform across the block
-    // Each thread scans kScanPer consecutive tiles in registers, so one pass of
-    // the block covers 16,384 tiles (a 2048^2 map) with one block-wide scan.
-    constexpr int kScanPer = 16;
-    __shared__ long long warpSum[32];
-    __shared__ long long carry;
+    // Each thread scans kScanPer consecutive tiles in registers: 4,096 tiles a pass.
+    constexpr int kScanPer = 16, kWarps = kMediumThreads / 32;
+    __shared__ long long warpSum[kWarps];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < tiles; base += 1024 * kScanPer)
+    long long carry = 0;
+    for (int base = 0; base < tiles; base += kMediumThreads * kScanPer)
     {
         const int i0 = base + tid * kScanPer;
         int v[kScanPer];
-        if (i0 + kScanPer <= tiles)
-        {
-            const int4* src = reinterpret_cast<const int4*>(rs.tileCount + i0);  // 64-byte aligned
 #pragma unroll
-            for (int q = 0; q < kScanPer / 4; ++q)
-            {
-                const int4 w = src[q];
-                v[4 * q] = w.x, v[4 * q + 1] = w.y, v[4 * q + 2] = w.z, v[4 * q + 3] = w.w;
-            }
-        }
-        else
-        {
-#pragma unroll
-            for (int k = 0; k < kScanPer; ++k) v[k] = i0 + k < tiles ? rs.tileCount[i0 + k] : 0;
-        }
+        for (int k = 0; k < kScanPer; ++k) v[k] = i0 + k < tiles ? __ldcg(rs.tileCount + i0 + k) : 0;
         long long local = 0;
 #pragma unroll
         for (int k = 0; k < kScanPer; ++k) local += v[k];
@@ -487,57 +517,54 @@ __global__ void __launch_bounds__(1024) k_bin_scan(RasterScratch rs, int tiles)
         }
         if (lane == 31) warpSum[wid] = x;
         __syncthreads();
-        if (wid == 0)
+        long long run = carry + (x - local);
+        for (int w = 0; w < kWarps; ++w)
         {
-            long long w = warpSum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                long long y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warpSum[lane] = w;  // inclusive
+            if (w < wid) run += warpSum[w];
+            carry += warpSum[w];
         }
-        __syncthreads();
-        long long run = carry + (wid ? warpSum[wid - 1] : 0) + (x - local);
-        if (i0 + kScanPer <= tiles)
+        for (int k = 0; k < kScanPer && i0 + k < tiles; ++k)
         {
-            int st[kScanPer];
-#pragma unroll
-            for (int k = 0; k < kScanPer; ++k)
-            {
-                st[k] = (int)min(run, (long long)0x7fffffff);
-                run += v[k];
-            }
-            int4* dst = reinterpret_cast<int4*>(rs.tileStart + i0);
-            int4* fill = reinterpret_cast<int4*>(rs.tileFill + i0);
-#pragma unroll
-            for (int q = 0; q < kScanPer / 4; ++q)
-            {
-                dst[q] = make_int4(st[4 * q], st[4 * q + 1], st[4 * q + 2], st[4 * q + 3]);
-                fill[q] = make_int4(0, 0, 0, 0);
-            }
+            rs.tileStart[i0 + k] = (int)min(run, (long long)0x7fffffff);
+            rs.tileFill[i0 + k] = 0;
+            run += v[k];
         }
-        else
-        {
-            for (int k = 0; k < kScanPer && i0 + k < tiles; ++k)
-            {
-                rs.tileStart[i0 + k] = (int)min(run, (long long)0x7fffffff);
-                rs.tileFill[i0 + k] = 0;
-                run += v[k];
-            }
-        }
-        __syncthreads();
-        if (tid == 0) carry += warpSum[31];
         __syncthreads();
     }
     if (tid == 0)
     {
-        long long total = carry;
-        rs.tileStart[tiles] = (int)min(total, (long long)0x7fffffff);
-        rs.counters[2] = (int)min(total, (long long)0x7fffffff);
-        if (total > rs.binCap) atomicOr(&rs.counters[3], kStatusBinOverflow);
+        rs.tileStart[tiles] = (int)min(carry, (long long)0x7fffffff);
+        rs.counters[2] = (int)min(carry, (long long)0x7fffffff);
+        if (carry > rs.binCap) atomicOr(&rs.counters[3], kStatusBinOverflow);
     }
+}
+
+// The medium triangles, and the counting and scan of the large ones' tile pairs (the
+// last CTA to finish counting scans): one launch where there were three, two of which
+// had nothing to do in most frames.
+__global__ void __launch_bounds__(kMediumThreads) k_raster_medium(RasterParams rp, RasterScratch rs, int tiles)
+{
+    raster_medium(rp, rs);
+    if (large_direct(rs)) return;  // uniform over the grid
+    for_large_tiles(rp, rs, [&](int, int tile) { atomicAdd(&rs.tileCount[tile], 1); });
+    __shared__ bool last;
+    __threadfence();  // this thread's counts are visible before its CTA's ticket
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(rs.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    bin_scan(rs, tiles);
+}
+
+// The large triangles' list indices into their tiles' ranges.
+__global__ void k_bin(RasterParams rp, RasterScratch rs)
+{
+    if (large_direct(rs)) return;
+    for_large_tiles(rp, rs, [&](int i, int tile) {
+        long long pos = (long long)rs.tileStart[tile] + atomicAdd(&rs.tileFill[tile], 1);
+        if (pos < rs.binCap) rs.binTri[pos] = i;
+    });
 }
 
 // One CTA per 16 x 16 tile: the tile's triangles are staged in shared memory
@@ -2136,24 +2163,43 @@ inline int blocks(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 }  // namespace
 
 // ---- launchers -------------------------------------------------------------------------------
-void launch_transform_camera(const DevScene& S, const FrameConst& F, VertexOut vo, cudaStream_t st)
+namespace
 {
-    int n = max(S.numVerts, S.numNormals);
-    if (n > 0) k_transform_camera<<<blocks(n, 256), 256, 0, st>>>(S, F, vo);
+
+int raster_tiles(const RasterParams& rp) { return ((rp.W + kTile - 1) / kTile) * ((rp.H + kTile - 1) / kTile); }
+
+RasterClear raster_clear(const RasterParams& rp, const RasterScratch& rs)
+{
+    return RasterClear{rs.keys, (long long)rp.W * rp.H, rs.counters, rs.tileCount, rs.ticket, raster_tiles(rp)};
 }
 
-void launch_transform_light(const DevScene& S, const FrameConst& F, int4* scrL, cudaStream_t st)
+// CTAs of a vertex stage: one thread a vertex, and enough of them for the clear (16 keys
+// a thread up to two CTAs per SM).
+int transform_blocks(int n, const RasterClear& c)
 {
-    if (S.numVerts > 0) k_transform_light<<<blocks(S.numVerts, 256), 256, 0, st>>>(S, F, scrL);
+    return std::max(blocks(n, 256), std::min(blocks(c.numKeys, 256 * 16), 2 * 152));
+}
+
+}  // namespace
+
+void launch_transform_camera(const DevScene& S, const FrameConst& F, VertexOut vo, const RasterParams& rp,
+                             const RasterScratch& rs, cudaStream_t st)
+{
+    const RasterClear c = raster_clear(rp, rs);
+    k_transform_camera<<<transform_blocks(max(S.numVerts, S.numNormals), c), 256, 0, st>>>(S, F, vo, c);
+}
+
+void launch_transform_light(const DevScene& S, const FrameConst& F, int4* scrL, const RasterParams& rp,
+                            const RasterScratch& rs, cudaStream_t st)
+{
+    const RasterClear c = raster_clear(rp, rs);
+    k_transform_light<<<transform_blocks(S.numVerts, c), 256, 0, st>>>(S, F, scrL, c);
 }
 
 void launch_raster(const DevScene& S, const int4* scr, const RasterParams& rp, RasterScratch& rs, cudaStream_t st,
                    int& launches, bool tileRaster, float* shadowOut)
 {
-    const int tiles = ((rp.W + kTile - 1) / kTile) * ((rp.H + kTile - 1) / kTile);
-    cudaMemsetAsync(rs.keys, 0xff, sizeof(unsigned long long) * (size_t)rp.W * rp.H, st);
-    cudaMemsetAsync(rs.counters, 0, sizeof(int) * 4, st);
-    cudaMemsetAsync(rs.tileCount, 0, sizeof(int) * tiles, st);
+    const int tiles = raster_tiles(rp);
     if (S.numTris <= 0)
     {
         if (shadowOut) cudaMemsetAsync(shadowOut, 0, sizeof(float) * (size_t)rp.W * rp.H, st);
@@ -2162,13 +2208,11 @@ void launch_raster(const DevScene& S, const int4* scr, const RasterParams& rp, R
     const int group = setup_group(S.numTris);
     k_setup<<<blocks(S.numTris, kSetupThreads / 32 * group), kSetupThreads, 0, st>>>(S, scr, rp, rs, group);
     int sms = 152;
-    k_raster_medium<<<sms * 8, 256, 0, st>>>(rp, rs);
-    k_bin<<<sms * 4, 256, 0, st>>>(rp, rs, 0);
-    k_bin_scan<<<1, 1024, 0, st>>>(rs, tiles);
-    k_bin<<<sms * 4, 256, 0, st>>>(rp, rs, 1);
+    k_raster_medium<<<sms * 8, kMediumThreads, 0, st>>>(rp, rs, tiles);
+    k_bin<<<sms * 4, 256, 0, st>>>(rp, rs);
     if (tileRaster && shadowOut) k_tile_raster_shadow<<<tiles, 256, 0, st>>>(rp, rs, S, scr, shadowOut);
     else if (tileRaster) k_tile_raster<<<tiles, 256, 0, st>>>(rp, rs);
-    launches += tileRaster ? 6 : 5;
+    launches += tileRaster ? 4 : 3;
 }
 
 void launch_tile_raster_views(const ViewRaster* vr, const int* itemStart, int nEntries, int total, int* queue,

@@ -21,6 +21,7 @@ struct RasterScratch
     float4* largeAux;          // [cap] the large triangles' per-vertex .w screen data
     int4* triRec;              // [2 * triangles] resolve records (tri_record), or null
     int* counters;             // [0] medium count, [1] large count, [2] bin pairs, [3] status bits
+    unsigned* ticket;          // CTAs of the medium raster that have counted their tile pairs
     int* tileCount;            // [tiles]
     int* tileStart;            // [tiles + 1]
     int* tileFill;             // [tiles]
@@ -73,12 +74,14 @@ struct ViewShade
                           // vertex as the reference does), or -1: projected per pixel
 };
 
-// Vertex stages.
+// Vertex stages; each also clears the raster scratch of its pass (the keys of a W x H
+// target, the counters and tile counts), which launch_raster expects cleared.
 void launch_transform_camera(const frd::DevScene& S, const frd::FrameConst& F, frd::VertexOut vo,
-                             cudaStream_t st);
-void launch_transform_light(const frd::DevScene& S, const frd::FrameConst& F, int4* scrL, cudaStream_t st);
+                             const RasterParams& rp, const RasterScratch& rs, cudaStream_t st);
+void launch_transform_light(const frd::DevScene& S, const frd::FrameConst& F, int4* scrL, const RasterParams& rp,
+                            const RasterScratch& rs, cudaStream_t st);
 
-// Visibility raster: clears keys, classifies and draws every triangle.
+// Visibility raster: classifies and draws every triangle into cleared scratch.
 // scr: per-vertex (sx, sy, depth bits, *) screen data of this pass.
 // shadowOut (a shadow pass): the fine raster also writes the shadow map (the
 // resolve of launch_resolve_shadow fused in).
