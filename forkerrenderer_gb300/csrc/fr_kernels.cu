@@ -1351,17 +1351,24 @@ __device__ __forceinline__ void ssao_background_cta(const FrameConst& F, const f
     }
 }
 
+// Programmatic dependent launch: the dependent may start now; it waits in
+// griddep_wait where it needs this kernel's results.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __global__ void __launch_bounds__(1024) k_ssao_background(FrameConst F, const float* __restrict__ depth,
                                                            const float* __restrict__ table, float* __restrict__ out16,
                                                            const int* __restrict__ gate)
 {
+    griddep_launch();
     if (gate && *gate == 0) return;
     extern __shared__ float rcb[];
     ssao_background_cta(F, depth, table, rcb, out16);
 }
 
 // 512-thread CTAs, three per SM (40 registers a thread; the 16-cell sample table
-// is 49 KB at 64 samples).
+// is 49 KB at 64 samples). Launched as a programmatic dependent of the background
+// kernel (one CTA, 5 us): only the background pixels wait for its values.
 constexpr int kSsaoThreads = 512;
 
 __global__ void __launch_bounds__(kSsaoThreads, 3) k_ssao(FrameConst F, GBuffer gb, const float* __restrict__ table,
@@ -1382,12 +1389,14 @@ __global__ void __launch_bounds__(kSsaoThreads, 3) k_ssao(FrameConst F, GBuffer 
         const float fragDepth = gb.depth[p];
         if (!(fragDepth < FLT_MAX))
         {
-            gb.ao[p] = bg16[cell];
+            griddep_wait();
+            gb.ao[p] = __ldcg(bg16 + cell);
             continue;
         }
         float4 A = gb.a[p], B = gb.b[p];
         gb.ao[p] = ssao_pixel_filtered(F, gb.depth, tbl4 + cell * stride, ld3(A), ld3(B), fragDepth);
     }
+    griddep_wait();  // this kernel ends after the background kernel, whatever its pixels
 }
 
 // ---- learned AO: network input and probe -----------------------------------------------------
@@ -2296,7 +2305,15 @@ void launch_ssao(const FrameConst& F, GBuffer gb, const float* table, float* bg1
     // gated (learned-AO fallback): a small grid-stride grid, so a skipped pass costs little
     const int grid = gate ? std::min(blocks((long long)F.W * F.H, kSsaoThreads), 2 * 152)
                           : blocks((long long)F.W * F.H, kSsaoThreads);
-    k_ssao<<<grid, kSsaoThreads, smem, st>>>(F, gb, table, bg16, gate);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kSsaoThreads);
+    cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = withBackground ? 1 : 0;
+    const float* bg = bg16;
+    cudaLaunchKernelEx(&cfg, k_ssao, F, gb, table, bg, gate);
 }
 
 void launch_ssao_background(const FrameConst& F, const float* depth, const float* table, float* bg16, cudaStream_t st)
