@@ -9,6 +9,8 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "fr_aonet.h"
@@ -45,6 +47,32 @@ struct Alloc
         for (void* p : ptrs) cudaFree(p);
     }
 };
+
+// dst = src, large copies by up to four threads (a fresh destination's page faults are
+// most of its time).
+void copy_bytes(unsigned char* dst, const unsigned char* src, size_t n)
+{
+    const size_t parts = std::min<size_t>(4, n >> 20);
+    if (parts < 2)
+    {
+        std::memcpy(dst, src, n);
+        return;
+    }
+    std::vector<std::thread> ts;
+    const size_t step = ((n / parts) + 65535) & ~(size_t)65535;
+    size_t at = step;
+    try
+    {
+        for (; at < n; at += step)
+            ts.emplace_back([=] { std::memcpy(dst + at, src + at, std::min(step, n - at)); });
+    }
+    catch (const std::system_error&)  // no thread to be had: the rest here
+    {
+        std::memcpy(dst + at, src + at, n - at);
+    }
+    std::memcpy(dst, src, std::min(step, n));
+    for (auto& t : ts) t.join();
+}
 
 int tiles_of(int w, int h, int t) { return ((w + t - 1) / t) * ((h + t - 1) / t); }
 
@@ -119,6 +147,7 @@ struct fr_batch
     frk::BatchLight* dLights = nullptr;
     int* dQueues = nullptr;
     float4* ssaoTblGlobal = nullptr;
+    uint8_t *rgb = nullptr, *rgbDev = nullptr;  // pinned: a packed 8-bit frame of any view, for downloads
 
     fr_batch_tuning tuning{16, 64, 2};
     cudaStream_t br[kBranches] = {};
@@ -470,6 +499,14 @@ fr_batch* fr_batch_create(fr_ctx* ctx, const fr_view_desc* views, int32_t n_view
     b->dShadeStart = A.get<int>(n_views + 1);
     b->dLights = A.get<frk::BatchLight>(bl.size());
     b->dQueues = A.get<int>(2);
+    size_t maxPix = 0;
+    for (auto& X : b->views) maxPix = std::max(maxPix, (size_t)X.F.W * X.F.H);
+    if (cudaHostAlloc(reinterpret_cast<void**>(&b->rgb), 3 * maxPix, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->rgbDev), b->rgb, 0) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return fr_batch_destroy(b), bail("out of pinned host memory");
+    }
     if (A.err != cudaSuccess) return fr_batch_destroy(b), bail("out of device memory");
     cudaMemcpy(b->dRaster, vr.data(), sizeof(frk::ViewRaster) * vr.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(b->dRasterStart, rstart.data(), sizeof(int) * rstart.size(), cudaMemcpyHostToDevice);
@@ -499,6 +536,7 @@ void fr_batch_destroy(fr_batch* b)
         if (b->joinEv[i]) cudaEventDestroy(b->joinEv[i]);
     }
     if (b->forkEv) cudaEventDestroy(b->forkEv);
+    if (b->rgb) cudaFreeHost(b->rgb);
     for (auto& e : b->tev)
         if (e) cudaEventDestroy(e);
     delete b;
@@ -634,22 +672,34 @@ int64_t fr_batch_download(fr_batch* b, int32_t view, int32_t id, void* dst, size
     }
     if (!dst) return (int64_t)need;
     if (bytes < need) return bfail(b, FR_ERR_INVALID, "destination too small");
-    B_CUDA(b, cudaStreamSynchronize(b->ctx->stream));
     if (src)
     {
+        B_CUDA(b, cudaStreamSynchronize(b->ctx->stream));
         B_CUDA(b, cudaMemcpy(dst, src, need, cudaMemcpyDeviceToHost));
         return FR_OK;
     }
-    // packed r | g << 8 | b << 16 -> RGB8
-    std::vector<unsigned> tmp(need / 3);
-    B_CUDA(b, cudaMemcpy(tmp.data(), rgba, sizeof(unsigned) * tmp.size(), cudaMemcpyDeviceToHost));
-    unsigned char* o = static_cast<unsigned char*>(dst);
-    for (size_t i = 0; i < tmp.size(); ++i)
+    // Packed to R, G, B bytes by the device, into the caller's pinned memory where the
+    // device can address it, else into the batch's pinned buffer and copied from there. (A
+    // 4-byte copy and a scalar loop on the host took as long as rendering the views; the
+    // device writing pageable memory itself is faster while its pages stay mapped, but
+    // costs milliseconds a pass when the caller's buffers come fresh from the system.)
+    const int n = (int)(need / 3);
+    cudaStream_t st = b->ctx->stream;
+    cudaPointerAttributes pa{};
+    const cudaError_t ae = cudaPointerGetAttributes(&pa, dst);
+    if (ae != cudaSuccess) cudaGetLastError();  // this call's own error: copy below
+    if (ae == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer && pa.device == b->ctx->cfg.device)
+        frk::launch_pack_rgb(rgba, static_cast<uint8_t*>(pa.devicePointer), n, st);
+    else
     {
-        o[3 * i] = tmp[i] & 0xff;
-        o[3 * i + 1] = (tmp[i] >> 8) & 0xff;
-        o[3 * i + 2] = (tmp[i] >> 16) & 0xff;
+        frk::launch_pack_rgb(rgba, b->rgbDev, n, st);
+        B_CUDA(b, cudaGetLastError());
+        B_CUDA(b, cudaStreamSynchronize(st));
+        copy_bytes(static_cast<unsigned char*>(dst), b->rgb, need);
+        return FR_OK;
     }
+    B_CUDA(b, cudaGetLastError());
+    B_CUDA(b, cudaStreamSynchronize(st));
     return FR_OK;
 }
 
