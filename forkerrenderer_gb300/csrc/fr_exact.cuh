@@ -32,6 +32,7 @@
 #pragma once
 
 #include <stdint.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define FR_HD __host__ __device__ __forceinline__
@@ -143,6 +144,20 @@ FR_HD float bitsf(unsigned int u)
 #endif
 }
 
+FR_HD unsigned long long dbits(double d)
+{
+    unsigned long long u;
+    memcpy(&u, &d, 8);
+    return u;
+}
+
+FR_HD double bitsd(unsigned long long u)
+{
+    double d;
+    memcpy(&d, &u, 8);
+    return d;
+}
+
 // Per-triangle raster setup: int-snapped screen vertices and viewport depths.
 struct RTri
 {
@@ -154,7 +169,7 @@ struct RTri
     int s53;                  // RN53(1 / |bz|) = m53 * 2^-s53 (class kTriFast)
     int small;                // all coordinates within +-kSmallLimit: edge functions fit int32
     long long bz;             // integer edge determinant (classes kTriFast / kTriIntDouble)
-    unsigned long long m53;
+    unsigned long long m53;   // (class kTriIntDouble: the bits of 1.0 / bz in double, 0 = not set)
 };
 
 FR_HD bool coords_in_range(const int* X, const int* Y)
@@ -190,6 +205,7 @@ FR_HD void classify(RTri& t, bool withRecip = true)
         t.rbz = t.cls == kTriFast ? frcp_rn(t.fbz) : 0.f;
         t.m53 = 0, t.s53 = 0;
         if (t.cls == kTriFast && withRecip) recip53((unsigned long long)(bz < 0 ? -bz : bz), t.m53, t.s53);
+        if (t.cls == kTriIntDouble && withRecip) t.m53 = dbits(1.0 / (double)bz);
         t.small = 1;
         for (int k = 0; k < 3; ++k)
             if (t.x[k] < -kSmallLimit || t.x[k] > kSmallLimit || t.y[k] < -kSmallLimit || t.y[k] > kSmallLimit)
@@ -228,15 +244,18 @@ FR_HD bool bary_reference(const int* X, const int* Y, int px, int py, float& b0,
 }
 
 // Double-path weights from exact integer edge values (|ex|,|ey|,|bz| < 2^53).
-FR_HD bool bary_from_ints_double(long long ex, long long ey, long long bz, float& b0, float& b1,
-                                 float& b2)
+FR_HD bool bary_from_ints_inv(long long ex, long long ey, double inv, float& b0, float& b1, float& b2)
 {
-    double inv = 1.0 / (double)bz;
     double u = (double)ex * inv, v = (double)ey * inv;
     float r0 = (float)(1.0 - (u + v)), r1 = (float)u, r2 = (float)v;
     if (r0 < 0.f || r1 < 0.f || r2 < 0.f) return false;
     b0 = r0, b1 = r1, b2 = r2;
     return true;
+}
+
+FR_HD bool bary_from_ints_double(long long ex, long long ey, long long bz, float& b0, float& b1, float& b2)
+{
+    return bary_from_ints_inv(ex, ey, 1.0 / (double)bz, b0, b1, b2);
 }
 
 // float(1 - (u + v)) of the double path for a covered fast-class pixel with
@@ -506,7 +525,8 @@ FR_HD bool bary(const RTri& t, int px, int py, float& b0, float& b1, float& b2)
     if (c != 0 && ((c > 0) != pos)) return false;
     if (t.cls == kTriIntDouble)
     {
-        if (!bary_from_ints_double(ex, ey, bz, b0, b1, b2)) return false;
+        // the division once per triangle where classify() kept it
+        if (!bary_from_ints_inv(ex, ey, t.m53 ? bitsd(t.m53) : 1.0 / (double)bz, b0, b1, b2)) return false;
     }
     else
     {
@@ -608,6 +628,31 @@ FR_HD bool bary_on_edge(int e1, int e2, int B, float rB, unsigned long long m53,
     b2 = fdiv_y((float)e2, fB, rB);
     b0 = w_on_edge((unsigned)e1, (unsigned)e2, m53, s53);
     return !(b0 < 0.f);
+}
+
+// Whether any pixel of the box [x0, x1] x [y0, y1] may be covered, for every class:
+// false only if bary() rejects them all. The reference's edge values (bary_reference;
+// the integer classes compute the same exact values) are products and one difference
+// of float differences that are monotonic in px and py, and every rounding is
+// monotonic, so their extremes over the box come from its sides. u < 0 or v < 0
+// rejects where the edge's largest value is negative (edge values are integers and
+// |Z| < 2^70, so no tiny quotient rounds to zero), w < 0 where the smallest u + v is
+// above 1 by far more than its roundings.
+FR_HD bool box_may_be_covered(const RTri& t, int x0, int x1, int y0, int y1)
+{
+    const float ax = (float)t.x[0], ay = (float)t.y[0], bx = (float)t.x[1], by = (float)t.y[1];
+    const float cx = (float)t.x[2], cy = (float)t.y[2];
+    double s0x = bx - ax, s0y = cx - ax, s1x = by - ay, s1y = cy - ay;
+    const double zx0 = ax - (float)x0, zx1 = ax - (float)x1, zy0 = ay - (float)y0, zy1 = ay - (float)y1;
+    double Z = s0x * s1y - s0y * s1x;
+    if (Z < 0.0) Z = -Z, s0x = -s0x, s0y = -s0y, s1x = -s1x, s1y = -s1y;
+    // X = s0y s1z - s0z s1y, Y = s0z s1x - s0x s1z, times the sign of Z
+    const double a0 = s0y * zy0, a1 = s0y * zy1, b0 = s1y * zx0, b1 = s1y * zx1;
+    const double c0 = s1x * zx0, c1 = s1x * zx1, d0 = s0x * zy0, d1 = s0x * zy1;
+    const double xmax = fmax(a0, a1) - fmin(b0, b1), ymax = fmax(c0, c1) - fmin(d0, d1);
+    if (xmax < 0.0 || ymax < 0.0) return false;
+    const double xmin = fmin(a0, a1) - fmax(b0, b1), ymin = fmin(c0, c1) - fmax(d0, d1);
+    return !(xmin + ymin > Z * 1.000000001);
 }
 
 // (float)(c * (double)p) for a positive normal double constant c with 53-bit

@@ -572,49 +572,94 @@ __global__ void k_bin(RasterParams rp, RasterScratch rs)
 // publishes it once. The body is shared by the single-view launch (one CTA per
 // tile) and the persistent multi-view launch ((view, tile) work queue).
 constexpr int kTileBatch = 64;
+constexpr int kTileThreads = kTile * kTile;
 
-template <int CAP>
-__device__ __forceinline__ void tile_raster_body(const RasterParams& rp, const RasterScratch& rs, int tile,
-                                                 frx::RTri* sh, int* shIdx, int4* shBox)
+// Barrier `id` of one tile's kTileThreads threads (a CTA may hold several tiles).
+__device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTileThreads) : "memory"); }
+
+// The tile's pixel of thread tid against triangles 0 .. cnt - 1 of shared memory: the
+// smaller of `best` and their keys. Every thread of the tile runs the loop (ballots).
+__device__ __forceinline__ unsigned long long tile_min_key(const frx::RTri* sh, const int* shIdx, const int4* shBox, int cnt,
+                                                           bool inside, int px, int py, unsigned long long best)
 {
-    const bool direct = large_direct(rs);
+    for (int j = 0; j < cnt; ++j)
+    {
+        int4 bb = shBox[j];
+        bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
+        if (__ballot_sync(0xffffffffu, inb) == 0u) continue;
+        if (!inb) continue;
+        float b0, b1, b2;
+        if (!frx::bary<0, false>(sh[j], px, py, b0, b1, b2)) continue;
+        float d = frx::depth_of(sh[j], b0, b1, b2);
+        if (!frx::depth_passes_clear(d)) continue;
+        unsigned long long key = frx::make_key(d, (unsigned)shIdx[j]);
+        best = key < best ? key : best;
+    }
+    return best;
+}
+
+__device__ __forceinline__ void stage_large(const RasterParams& rp, const RasterScratch& rs, int li, int i, frx::RTri* sh,
+                                            int* shIdx, int4* shBox)
+{
+    frx::RTri r = rs.largeTris[li];
+    sh[i] = r;
+    shIdx[i] = rs.largeIdx[li];
+    int x0, x1, y0, y1;
+    bbox(r, rp.W, rp.H, x0, x1, y0, y1);
+    shBox[i] = make_int4(x0, x1, y0, y1);
+}
+
+// (out of line: its FP64 registers would spill the callers')
+__device__ __noinline__ bool edges_meet_tile(const frx::RTri* r, int tx0, int ty0)
+{
+    return frx::box_may_be_covered(*r, tx0, tx0 + kTile - 1, ty0, ty0 + kTile - 1);
+}
+
+// One tile with threads tid = 0 .. kTileThreads - 1 (barrier `bar`). staged: the pass'
+// large triangles (large_direct) are in shared memory already. A binned triangle whose
+// edges miss the tile is not staged (bins hold every tile of its box: 3.4 million pairs
+// for a few views beside a sphere, most of them slivers through the camera plane that
+// run 256 FP64 evaluations a tile). cntSh: a counter of the tile in shared memory.
+template <int CAP>
+__device__ __forceinline__ void tile_raster_body(const RasterParams& rp, const RasterScratch& rs, int tile, int tid, int bar,
+                                                 bool direct, bool staged, frx::RTri* sh, int* shIdx, int4* shBox,
+                                                 int* cntSh)
+{
     long long start = direct ? 0 : rs.tileStart[tile];
     long long end = direct ? min(rs.counters[1], rs.triCap) : min((long long)rs.tileStart[tile + 1], rs.binCap);
-    if (start >= end) return;  // uniform across the CTA
+    if (start >= end) return;  // uniform across the tile
     int ntx = (rp.W + kTile - 1) / kTile;
-    int px = (tile % ntx) * kTile + (threadIdx.x & 15);
-    int py = (tile / ntx) * kTile + (threadIdx.x >> 4);
+    const int tx0 = (tile % ntx) * kTile, ty0 = (tile / ntx) * kTile;
+    int px = tx0 + (tid & 15);
+    int py = ty0 + (tid >> 4);
     bool inside = px < rp.W && py < rp.H;
     unsigned long long best = frx::kEmptyKey;
     for (long long base = start; base < end; base += CAP)
     {
         int cnt = (int)min((long long)CAP, end - base);
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+        if (!staged)
         {
-            int li = direct ? (int)(base + i) : rs.binTri[base + i];
-            frx::RTri r = rs.largeTris[li];
-            sh[i] = r;
-            shIdx[i] = rs.largeIdx[li];
-            int x0, x1, y0, y1;
-            bbox(r, rp.W, rp.H, x0, x1, y0, y1);
-            shBox[i] = make_int4(x0, x1, y0, y1);
+            if (direct)
+            {
+                for (int i = tid; i < cnt; i += kTileThreads) stage_large(rp, rs, (int)(base + i), i, sh, shIdx, shBox);
+                tile_sync(bar);
+            }
+            else
+            {
+                if (tid == 0) *cntSh = 0;
+                tile_sync(bar);
+                for (int i = tid; i < cnt; i += kTileThreads)
+                {
+                    const int li = rs.binTri[base + i];
+                    if (edges_meet_tile(rs.largeTris + li, tx0, ty0))
+                        stage_large(rp, rs, li, atomicAdd(cntSh, 1), sh, shIdx, shBox);
+                }
+                tile_sync(bar);
+                cnt = *cntSh;
+            }
         }
-        __syncthreads();
-        // every thread runs the loop so the warp-wide ballot sees full warps
-        for (int j = 0; j < cnt; ++j)
-        {
-            int4 bb = shBox[j];
-            bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
-            if (__ballot_sync(0xffffffffu, inb) == 0u) continue;
-            if (!inb) continue;
-            float b0, b1, b2;
-            if (!frx::bary<0, false>(sh[j], px, py, b0, b1, b2)) continue;
-            float d = frx::depth_of(sh[j], b0, b1, b2);
-            if (!frx::depth_passes_clear(d)) continue;
-            unsigned long long key = frx::make_key(d, (unsigned)shIdx[j]);
-            best = key < best ? key : best;
-        }
-        __syncthreads();
+        best = tile_min_key(sh, shIdx, shBox, cnt, inside, px, py, best);
+        if (!staged) tile_sync(bar);
     }
     if (inside && best != frx::kEmptyKey) atomicMin(rs.keys + (size_t)py * rp.W + px, best);
 }
@@ -624,7 +669,8 @@ __global__ void __launch_bounds__(256) k_tile_raster(RasterParams rp, RasterScra
     __shared__ frx::RTri sh[kTileBatch];
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
-    tile_raster_body<kTileBatch>(rp, rs, blockIdx.x, sh, shIdx, shBox);
+    __shared__ int cntSh;
+    tile_raster_body<kTileBatch>(rp, rs, blockIdx.x, threadIdx.x, 0, large_direct(rs), false, sh, shIdx, shBox, &cntSh);
 }
 
 // Shadow-map value of texel p from its visibility key: the winning triangle's
@@ -680,10 +726,12 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
     __shared__ float4 shZ[kTileBatch];
+    __shared__ int cntSh;
     const int tile = blockIdx.x;
     const int ntx = (rp.W + kTile - 1) / kTile;
-    const int px = (tile % ntx) * kTile + (threadIdx.x & 15);
-    const int py = (tile / ntx) * kTile + (threadIdx.x >> 4);
+    const int tx0 = (tile % ntx) * kTile, ty0 = (tile / ntx) * kTile;
+    const int px = tx0 + (threadIdx.x & 15);
+    const int py = ty0 + (threadIdx.x >> 4);
     const bool inside = px < rp.W && py < rp.H;
     const size_t p = inside ? (size_t)py * rp.W + px : 0;
     const unsigned long long k0 = inside ? __ldcg(rs.keys + p) : frx::kEmptyKey;
@@ -696,19 +744,25 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
     const long long end = direct ? min(rs.counters[1], rs.triCap) : min((long long)rs.tileStart[tile + 1], rs.binCap);
     for (long long base = start; base < end; base += kTileBatch)
     {
-        const int cnt = (int)min((long long)kTileBatch, end - base);
+        int cnt = (int)min((long long)kTileBatch, end - base);
+        if (threadIdx.x == 0) cntSh = 0;
+        __syncthreads();
         for (int i = threadIdx.x; i < cnt; i += blockDim.x)
         {
             const int li = direct ? (int)(base + i) : rs.binTri[base + i];
+            // (a binned triangle whose edges miss the tile is not staged)
+            if (!direct && !edges_meet_tile(rs.largeTris + li, tx0, ty0)) continue;
             const frx::RTri r = rs.largeTris[li];
-            sh[i] = r;
-            shIdx[i] = rs.largeIdx[li];
-            shZ[i] = rs.largeAux[li];
+            const int k = atomicAdd(&cntSh, 1);
+            sh[k] = r;
+            shIdx[k] = rs.largeIdx[li];
+            shZ[k] = rs.largeAux[li];
             int x0, x1, y0, y1;
             bbox(r, rp.W, rp.H, x0, x1, y0, y1);
-            shBox[i] = make_int4(x0, x1, y0, y1);
+            shBox[k] = make_int4(x0, x1, y0, y1);
         }
         __syncthreads();
+        cnt = cntSh;
         // every thread runs the loop so the warp-wide ballot sees full warps
         for (int j = 0; j < cnt; ++j)
         {
@@ -740,6 +794,12 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
         shadow[p] = out0;
 }
 
+// Shared-memory bytes of CAP staged triangles.
+__host__ __device__ constexpr size_t tile_stage_bytes(int cap)
+{
+    return ((size_t)cap * (sizeof(frx::RTri) + sizeof(int) + sizeof(int4)) + 15) / 16 * 16;
+}
+
 // Index of the work-queue entry holding item `it`: the last e with start[e] <= it.
 __device__ __forceinline__ int queue_entry(const int* __restrict__ start, int n, int it)
 {
@@ -754,34 +814,57 @@ __device__ __forceinline__ int queue_entry(const int* __restrict__ start, int n,
 }
 
 // Persistent fine raster of many views (camera views and shadow maps): CTAs
-// take (view, tile) items from one atomic queue until it runs dry. CAP
-// triangles are staged in shared memory per batch.
+// take chunks of (view, tile) items from one atomic queue until it runs dry. A CTA
+// holds two tiles at a time (kTileThreads threads each), CAP triangles staged in
+// shared memory per tile and batch; a pass' few large triangles (large_direct) are
+// staged once and kept while the items stay in that pass.
+constexpr int kViewTiles = 2;    // tiles a CTA holds
+constexpr int kViewChunk = 16;   // items a queue access takes
+
 template <int CAP>
-__global__ void __launch_bounds__(256) k_tile_raster_views(const ViewRaster* __restrict__ vr,
+__global__ void __launch_bounds__(kViewTiles * kTileThreads) k_tile_raster_views(const ViewRaster* __restrict__ vr,
                                                            const int* __restrict__ itemStart, int nEntries, int total,
                                                            int* __restrict__ queue)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
-    frx::RTri* sh = reinterpret_cast<frx::RTri*>(dsm);
-    int* shIdx = reinterpret_cast<int*>(sh + CAP);
-    int4* shBox = reinterpret_cast<int4*>(shIdx + CAP);
-    __shared__ int sItem, sEntry;
+    const int g = threadIdx.x / kTileThreads, tid = threadIdx.x % kTileThreads;  // this thread's tile slot
+    frx::RTri* sh = reinterpret_cast<frx::RTri*>(dsm + g * tile_stage_bytes(CAP));
+    int4* shBox = reinterpret_cast<int4*>(sh + CAP);
+    int* shIdx = reinterpret_cast<int*>(shBox + CAP);
+    __shared__ int sItem, cntSh[kViewTiles];
+    RasterParams rp{};
+    RasterScratch rs{};
+    int cur = -1;         // the pass of rp, rs
+    bool direct = false;
     for (;;)
     {
-        if (threadIdx.x == 0)
-        {
-            int it = atomicAdd(queue, 1);
-            sItem = it;
-            sEntry = it < total ? queue_entry(itemStart, nEntries, it) : 0;
-        }
+        if (threadIdx.x == 0) sItem = atomicAdd(queue, kViewChunk);
         __syncthreads();
-        const int it = sItem;
-        if (it >= total) break;
-        const int e = sEntry;
-        const RasterParams rp = vr[e].rp;
-        const RasterScratch rs = vr[e].rs;
-        tile_raster_body<CAP>(rp, rs, it - itemStart[e], sh, shIdx, shBox);
+        const int base = sItem;
         __syncthreads();  // sItem is rewritten next
+        if (base >= total) break;
+        const int last = min(base + kViewChunk, total);
+        int e = base + g < total ? queue_entry(itemStart, nEntries, base + g) : 0;
+        for (int it = base + g; it < last; it += kViewTiles)
+        {
+            while (e + 1 < nEntries && itemStart[e + 1] <= it) ++e;
+            if (e != cur)
+            {
+                cur = e;
+                rp = vr[e].rp;
+                rs = vr[e].rs;
+                direct = large_direct(rs);
+                if (direct)
+                {
+                    tile_sync(1 + g);  // the slot's previous triangles are done with
+                    const int n = min(rs.counters[1], rs.triCap);
+                    if (tid < n) stage_large(rp, rs, tid, tid, sh, shIdx, shBox);
+                    tile_sync(1 + g);
+                }
+            }
+            tile_raster_body<CAP>(rp, rs, it - itemStart[e], tid, 1 + g, direct, direct, sh, shIdx, shBox,
+                                  cntSh + g);
+        }
     }
 }
 
@@ -1060,39 +1143,45 @@ __device__ __forceinline__ unsigned shade_batch_pixel(const DevScene& S, const V
     return quantize_rgb(c);
 }
 
+// CTAs of 512 threads, two per SM (64 registers), take kLightThreads pixels of the
+// queue's T x T tiles at a time. With 256 threads of 92 registers the two CTAs per SM
+// of the default tuning left the gathers' latency open (11.3 ms for 43.6 Mpixel under
+// four lights, 25 PCF taps each).
+constexpr int kLightThreads = 512;
+
 template <int T, bool kLinear>
-__global__ void __launch_bounds__(256) k_lighting_views(DevScene S, const ViewShade* __restrict__ views,
+__global__ void __launch_bounds__(kLightThreads, 2) k_lighting_views(DevScene S, const ViewShade* __restrict__ views,
                                                         const int* __restrict__ itemStart, int nViews, int total,
                                                         const BatchLight* __restrict__ lights, int nLights,
                                                         int* __restrict__ queue)
 {
-    __shared__ int sItem, sView;
+    constexpr int kItems = kLightThreads >= T * T ? kLightThreads / (T * T) : 1;  // tiles a queue access takes
+    __shared__ int sItem, sView[kItems];
     for (;;)
     {
-        if (threadIdx.x == 0)
-        {
-            int it = atomicAdd(queue, 1);
-            sItem = it;
-            sView = it < total ? queue_entry(itemStart, nViews, it) : 0;
-        }
+        if (threadIdx.x == 0) sItem = atomicAdd(queue, kItems);
         __syncthreads();
-        const int it = sItem;
-        if (it >= total) break;
-        const ViewShade& VS = views[sView];
-        const int W = VS.F.W, H = VS.F.H;
-        const int tile = it - itemStart[sView];
-        const int ntx = (W + T - 1) / T;
-        const int x0 = (tile % ntx) * T, y0 = (tile / ntx) * T;
-        for (int k = threadIdx.x; k < T * T; k += blockDim.x)
+        const int base = sItem;
+        if (base >= total) break;
+        if (threadIdx.x < kItems && base + threadIdx.x < total)
+            sView[threadIdx.x] = queue_entry(itemStart, nViews, base + threadIdx.x);
+        __syncthreads();
+        for (int k = threadIdx.x; k < kItems * T * T; k += kLightThreads)
         {
-            const int px = x0 + k % T, py = y0 + k / T;
+            const int i = k / (T * T), q = k % (T * T);
+            if (base + i >= total) break;
+            const ViewShade& VS = views[sView[i]];
+            const int W = VS.F.W, H = VS.F.H;
+            const int tile = base + i - itemStart[sView[i]];
+            const int ntx = (W + T - 1) / T;
+            const int px = (tile % ntx) * T + q % T, py = (tile / ntx) * T + q / T;
             if (px < W && py < H)
             {
                 const int p = py * W + px;
                 VS.frame8[p] = shade_batch_pixel<kLinear>(S, VS, p, lights, nLights);
             }
         }
-        __syncthreads();
+        __syncthreads();  // sItem and sView are rewritten next
     }
 }
 
@@ -2233,11 +2322,12 @@ void launch_tile_raster_views(const ViewRaster* vr, const int* itemStart, int nE
         cudaFuncSetAttribute(k_tile_raster_views<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr = true;
     }
-    const size_t smem = (size_t)cap * (sizeof(frx::RTri) + sizeof(int) + sizeof(int4));
+    const size_t smem = kViewTiles * tile_stage_bytes(cap >= 1024 ? 1024 : cap >= 256 ? 256 : 64);
+    constexpr int threads = kViewTiles * kTileThreads;
     cudaMemsetAsync(queue, 0, sizeof(int), st);
-    if (cap >= 1024) k_tile_raster_views<1024><<<grid, 256, smem, st>>>(vr, itemStart, nEntries, total, queue);
-    else if (cap >= 256) k_tile_raster_views<256><<<grid, 256, smem, st>>>(vr, itemStart, nEntries, total, queue);
-    else k_tile_raster_views<64><<<grid, 256, smem, st>>>(vr, itemStart, nEntries, total, queue);
+    if (cap >= 1024) k_tile_raster_views<1024><<<grid, threads, smem, st>>>(vr, itemStart, nEntries, total, queue);
+    else if (cap >= 256) k_tile_raster_views<256><<<grid, threads, smem, st>>>(vr, itemStart, nEntries, total, queue);
+    else k_tile_raster_views<64><<<grid, threads, smem, st>>>(vr, itemStart, nEntries, total, queue);
 }
 
 template <bool kLinear>
@@ -2245,11 +2335,11 @@ void launch_lighting_views_t(const DevScene& S, const ViewShade* views, const in
                              const BatchLight* lights, int nLights, int* queue, int T, int grid, cudaStream_t st)
 {
     if (T <= 8)
-        k_lighting_views<8, kLinear><<<grid, 256, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
+        k_lighting_views<8, kLinear><<<grid, kLightThreads, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
     else if (T <= 16)
-        k_lighting_views<16, kLinear><<<grid, 256, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
+        k_lighting_views<16, kLinear><<<grid, kLightThreads, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
     else
-        k_lighting_views<32, kLinear><<<grid, 256, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
+        k_lighting_views<32, kLinear><<<grid, kLightThreads, 0, st>>>(S, views, itemStart, nViews, total, lights, nLights, queue);
 }
 
 void launch_lighting_views(const DevScene& S, const ViewShade* views, const int* itemStart, int nViews, int total,

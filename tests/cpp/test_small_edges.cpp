@@ -1,6 +1,7 @@
 // Host check of the setup kernel's small-triangle path (fr_exact.cuh: small_edges,
 // box_row, bary_off_edge, bary_on_edge) against bary<0, false> on every pixel of the
-// clamped box: same coverage, same weights. Exit status 0 = no difference.
+// clamped box: same coverage, same weights; and that box_may_be_covered never drops a
+// tile with a covered pixel, for triangles of every class. Exit status 0 = no difference.
 // Usage: test_small_edges <num_triangles> <seed>
 #include <algorithm>
 #include <cstdio>
@@ -67,6 +68,34 @@ int main(int argc, char** argv)
             }
         }
     }
+    // 16 x 16 tiles against triangles of every class, many of them with far vertices
+    long tiles = 0, kept = 0;
+    for (long it = 0; it < n / 2; ++it)
+    {
+        frx::RTri t;
+        const long span = (const long[]){12, 60, 400, 5000, 100000, 9000000, 2000000000}[rng() % 7];
+        const int tx = (int)(rng() % 128) * 16, ty = (int)(rng() % 128) * 16;
+        for (int k = 0; k < 3; ++k)
+        {
+            const long s2 = rng() % 3 ? span : 40;
+            t.x[k] = (int)std::max(-2147483647l, std::min(2147483647l, tx + (long)(rng() % (2 * s2 + 1)) - s2));
+            t.y[k] = (int)std::max(-2147483647l, std::min(2147483647l, ty + (long)(rng() % (2 * s2 + 1)) - s2));
+            t.d[k] = 0.f;
+        }
+        if (rng() % 8 == 0) t.y[1] = t.y[0];
+        frx::classify(t);
+        if (t.cls == frx::kTriEmpty) continue;
+        bool any = false;
+        for (int q = 0; q < 256; ++q)
+        {
+            float b0, b1, b2;
+            any = any || frx::bary<0, false>(t, tx + q % 16, ty + q / 16, b0, b1, b2);
+        }
+        const bool keep = frx::box_may_be_covered(t, tx, tx + 15, ty, ty + 15);
+        ++tiles, kept += keep;
+        if (any && !keep && bad++ < 10) std::printf("TILE DROPPED class %d\n", t.cls);
+    }
+    std::printf("tiles %ld kept %ld\n", tiles, kept);
     // every row of every box width a small triangle can have
     for (int w = 1; w <= 8192; w = w < 300 ? w + 1 : w + 61)
         for (int l = 0; l < 65536; l += w < 8 ? 1 : 7, ++rows)
