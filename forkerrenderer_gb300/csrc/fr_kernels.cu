@@ -1129,7 +1129,7 @@ __device__ __forceinline__ unsigned shade_batch_pixel(const DevScene& S, const V
                 const F4 q = mul4(Lk.S.L, F4{pos.x, pos.y, pos.z, 1.f});
                 l = F3{q.x / q.w, q.y / q.w, q.z / q.w};
             }
-            vis = shadow_visibility(Lk.S, Lk.shadow, l, n, L);
+            vis = shadow_visibility<true>(Lk.S, Lk.shadow, l, n, L);
         }
         if (pbrMat)
         {
