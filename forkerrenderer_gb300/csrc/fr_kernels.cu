@@ -1097,13 +1097,13 @@ __device__ __forceinline__ unsigned shade_batch_pixel(const DevScene& S, const V
                                                       const BatchLight* __restrict__ lights, int nLights)
 {
     const FrameConst& F = VS.F;
-    const uint4 C = VS.gb.c[p];
+    const uint4 C = __ldcs(VS.gb.c + p);
     if (!((C.y >> 24) & kGCovered)) return 0u;  // background: black, as the reference's lit frame
-    const float4 A = VS.gb.a[p], B = VS.gb.b[p];
+    const float4 A = __ldcs(VS.gb.a + p), B = __ldcs(VS.gb.b + p);
     GDecoded g = decode_gbuffer_t<kLinear>(S, C);
     const F3 pos = ld3(A), n = ld3(B), lg{A.w, B.w, __uint_as_float(C.x)};
     F3 param = g.param;
-    param.x *= VS.gb.ao[p];
+    param.x *= __ldcs(VS.gb.ao + p);
     const F3 eye{F.eye[0], F.eye[1], F.eye[2]};
     const F3 Vd = normalize(eye - pos);
     const bool pbrMat = g.type >= 0.5f;
@@ -1178,7 +1178,7 @@ __global__ void __launch_bounds__(kLightThreads, 2) k_lighting_views(DevScene S,
             if (px < W && py < H)
             {
                 const int p = py * W + px;
-                VS.frame8[p] = shade_batch_pixel<kLinear>(S, VS, p, lights, nLights);
+                __stcs(VS.frame8 + p, shade_batch_pixel<kLinear>(S, VS, p, lights, nLights));
             }
         }
         __syncthreads();  // sItem and sView are rewritten next
