@@ -169,7 +169,7 @@ struct RTri
     int s53;                  // RN53(1 / |bz|) = m53 * 2^-s53 (class kTriFast)
     int small;                // all coordinates within +-kSmallLimit: edge functions fit int32
     long long bz;             // integer edge determinant (classes kTriFast / kTriIntDouble)
-    unsigned long long m53;   // (class kTriIntDouble: the bits of 1.0 / bz in double, 0 = not set)
+    unsigned long long m53;   // (kTriIntDouble, kTriReference: the bits of 1.0 / bz in double, 0 = not set)
 };
 
 FR_HD bool coords_in_range(const int* X, const int* Y)
@@ -220,7 +220,22 @@ FR_HD void classify(RTri& t, bool withRecip = true)
         t.small = 0;
         double bzd = bz_reference(t.x, t.y);
         t.cls = (bzd > 1e-2 || bzd < -1e-2) ? kTriReference : kTriEmpty;
+        if (t.cls == kTriReference && withRecip) t.m53 = dbits(1.0 / bzd);
     }
+}
+
+// Reference Barycentric with inv = 1.0 / Z_ of bary_reference (one triangle's constant).
+FR_HD bool bary_reference_inv(const int* X, const int* Y, double inv, int px, int py, float& b0, float& b1, float& b2)
+{
+    const float ax = (float)X[0], ay = (float)Y[0], bx = (float)X[1], by = (float)Y[1];
+    const float cx = (float)X[2], cy = (float)Y[2], fx = (float)px, fy = (float)py;
+    const double s0x = bx - ax, s0y = cx - ax, s0z = ax - fx;
+    const double s1x = by - ay, s1y = cy - ay, s1z = ay - fy;
+    const double u = (s0y * s1z - s0z * s1y) * inv, v = (s0z * s1x - s0x * s1z) * inv;
+    const float r0 = (float)(1.0 - (u + v)), r1 = (float)u, r2 = (float)v;
+    if (r0 < 0.f || r1 < 0.f || r2 < 0.f) return false;
+    b0 = r0, b1 = r1, b2 = r2;
+    return true;
 }
 
 // Literal reference Barycentric for any coordinates (geometry.cpp:20-56).
@@ -510,7 +525,9 @@ FR_HD bool bary_small(const RTri& t, int px, int py, float& b0, float& b1, float
 template <int kOnly = 0, bool kZeroSigns = true>
 FR_HD bool bary(const RTri& t, int px, int py, float& b0, float& b1, float& b2)
 {
-    if (t.cls == kTriReference) return bary_reference(t.x, t.y, px, py, b0, b1, b2);
+    if (t.cls == kTriReference)
+        return t.m53 ? bary_reference_inv(t.x, t.y, bitsd(t.m53), px, py, b0, b1, b2)
+                     : bary_reference(t.x, t.y, px, py, b0, b1, b2);
     if (t.cls == kTriEmpty) return false;
     if (t.cls == kTriFast && t.small && small_pixel(px, py))
         return bary_small<kOnly, kZeroSigns>(t, px, py, b0, b1, b2);

@@ -579,13 +579,13 @@ __device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, %
 
 // The tile's pixel of thread tid against triangles 0 .. cnt - 1 of shared memory: the
 // smaller of `best` and their keys. Every thread of the tile runs the loop (ballots).
-__device__ __forceinline__ unsigned long long tile_min_key(const frx::RTri* sh, const int* shIdx, const int4* shBox, int cnt,
-                                                           bool inside, int px, int py, unsigned long long best)
+__device__ __forceinline__ unsigned long long tile_min_key(const frx::RTri* sh, const int* shIdx, const int4* shBox,
+                                                           int cnt, bool inside, int px, int py, unsigned long long best)
 {
     for (int j = 0; j < cnt; ++j)
     {
-        int4 bb = shBox[j];
-        bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
+        const int4 bb = shBox[j];
+        const bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
         if (__ballot_sync(0xffffffffu, inb) == 0u) continue;
         if (!inb) continue;
         float b0, b1, b2;
@@ -726,12 +726,10 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
     __shared__ float4 shZ[kTileBatch];
-    __shared__ int cntSh;
     const int tile = blockIdx.x;
     const int ntx = (rp.W + kTile - 1) / kTile;
-    const int tx0 = (tile % ntx) * kTile, ty0 = (tile / ntx) * kTile;
-    const int px = tx0 + (threadIdx.x & 15);
-    const int py = ty0 + (threadIdx.x >> 4);
+    const int px = (tile % ntx) * kTile + (threadIdx.x & 15);
+    const int py = (tile / ntx) * kTile + (threadIdx.x >> 4);
     const bool inside = px < rp.W && py < rp.H;
     const size_t p = inside ? (size_t)py * rp.W + px : 0;
     const unsigned long long k0 = inside ? __ldcg(rs.keys + p) : frx::kEmptyKey;
@@ -744,25 +742,19 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
     const long long end = direct ? min(rs.counters[1], rs.triCap) : min((long long)rs.tileStart[tile + 1], rs.binCap);
     for (long long base = start; base < end; base += kTileBatch)
     {
-        int cnt = (int)min((long long)kTileBatch, end - base);
-        if (threadIdx.x == 0) cntSh = 0;
-        __syncthreads();
+        const int cnt = (int)min((long long)kTileBatch, end - base);
         for (int i = threadIdx.x; i < cnt; i += blockDim.x)
         {
             const int li = direct ? (int)(base + i) : rs.binTri[base + i];
-            // (a binned triangle whose edges miss the tile is not staged)
-            if (!direct && !edges_meet_tile(rs.largeTris + li, tx0, ty0)) continue;
             const frx::RTri r = rs.largeTris[li];
-            const int k = atomicAdd(&cntSh, 1);
-            sh[k] = r;
-            shIdx[k] = rs.largeIdx[li];
-            shZ[k] = rs.largeAux[li];
+            sh[i] = r;
+            shIdx[i] = rs.largeIdx[li];
+            shZ[i] = rs.largeAux[li];
             int x0, x1, y0, y1;
             bbox(r, rp.W, rp.H, x0, x1, y0, y1);
-            shBox[k] = make_int4(x0, x1, y0, y1);
+            shBox[i] = make_int4(x0, x1, y0, y1);
         }
         __syncthreads();
-        cnt = cntSh;
         // every thread runs the loop so the warp-wide ballot sees full warps
         for (int j = 0; j < cnt; ++j)
         {
@@ -819,7 +811,7 @@ __device__ __forceinline__ int queue_entry(const int* __restrict__ start, int n,
 // shared memory per tile and batch; a pass' few large triangles (large_direct) are
 // staged once and kept while the items stay in that pass.
 constexpr int kViewTiles = 2;    // tiles a CTA holds
-constexpr int kViewChunk = 16;   // items a queue access takes
+constexpr int kViewChunk = 8;     // items a queue access takes
 
 template <int CAP>
 __global__ void __launch_bounds__(kViewTiles * kTileThreads) k_tile_raster_views(const ViewRaster* __restrict__ vr,
