@@ -1325,8 +1325,9 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
-// The frame kernel's table: per (cell, sample) three float4: (k, Q.w), (Q.xyz, 0),
-// (o, 0), with o built as in ssao_build_table and Q = VP (o, 0) (frx::ssao_q).
+// The frame kernel's table: per (cell, sample) three float4: (Q'x, Q'y, Q'z, Q.w),
+// (k, 0), (o, 0), with o built as in ssao_build_table, Q = VP (o, 0) (frx::ssao_q) and
+// Q' its rows times the viewport's diagonal (frx::ssao_ends).
 // Cells are 3N + 1 float4 apart: the four cells a warp row reads start 4 banks apart.
 __host__ __device__ constexpr int ssao_q_stride(int N) { return 3 * N + 1; }
 __device__ __forceinline__ void ssao_build_table_q(const FrameConst& F, const float* __restrict__ table, float4* tbl,
@@ -1340,44 +1341,49 @@ __device__ __forceinline__ void ssao_build_table_q(const FrameConst& F, const fl
         float Q[4];
         frx::ssao_q(F.VP, o.x, o.y, o.z, Q);
         int cell = e / N, s = e % N;
-        tbl[cell * stride + 3 * s] = make_float4(k.x, k.y, k.z, Q[3]);
-        tbl[cell * stride + 3 * s + 1] = make_float4(Q[0], Q[1], Q[2], 0.f);
+        tbl[cell * stride + 3 * s] = make_float4(__fmul_rn(F.VPort[0], Q[0]), __fmul_rn(F.VPort[5], Q[1]),
+                                                 __fmul_rn(F.VPort[10], Q[2]), Q[3]);
+        tbl[cell * stride + 3 * s + 1] = make_float4(k.x, k.y, k.z, 0.f);
         tbl[cell * stride + 3 * s + 2] = make_float4(o.x, o.y, o.z, 0.f);
     }
 }
 
-// One pixel's SSAO through the estimate (frx::ssao_plane): a sample whose
-// estimated pixel and depth comparison lie outside the error bound of every
-// rounding boundary is decided by the estimate; the others (about 1 % on the
-// benchmark frame) are marked and evaluated exactly afterwards. The result is
-// the exact path's for every sample.
+// One pixel's SSAO through the estimate (frx::ssao_ends): a sample whose interval lies
+// in one pixel and on one side of the depth comparison is decided by the estimate; the
+// others (about 1 % on the benchmark frame) are marked and evaluated exactly
+// afterwards. The result is the exact path's for every sample.
 __device__ __forceinline__ float ssao_pixel_filtered(const FrameConst& F, const float* __restrict__ depth,
                                                      const float4* k, F3 pos, F3 nrm, float fragDepth)
 {
-    const frx::SsaoPlane q = frx::ssao_plane(F.VP, F.VPort, F.vportSimple != 0, F.ssaoRadius, pos.x, pos.y, pos.z);
+    const frx::SsaoEnds q = frx::ssao_ends(F.VP, F.VPort, F.vportSimple != 0, F.ssaoRadius, F.W, pos.x, pos.y, pos.z);
     const int N = F.ssaoN;
     int hits = 0;
     if (!q.ok)
     {
-        for (int s = 0; s < N; ++s) hits += ssao_sample(F, depth, k[3 * s], k[3 * s + 2], pos, nrm, fragDepth) > 0.f;
+        for (int s = 0; s < N; ++s)
+            hits += ssao_sample(F, depth, k[3 * s + 1], k[3 * s + 2], pos, nrm, fragDepth) > 0.f;
         return ssao_result(F, hits);
     }
-    const float V0 = F.VPort[0], V3 = F.VPort[3], V5 = F.VPort[5], V7 = F.VPort[7], V10 = F.VPort[10],
-                V11 = F.VPort[11];
+    const unsigned n = (unsigned)(F.W * F.H);
     // one sample by the estimate: adds its hit when decided, else marks it
     auto fast = [&](int s, unsigned bit, unsigned& unsure) {
-        const float4 kq = k[3 * s], qq = k[3 * s + 1];
-        const float sg = ssao_flip(kq, nrm);
-        const float r = rcp_approx(__fmaf_rn(sg, kq.w, q.P[3]));
-        const float ex = __fmaf_rn(V0, __fmul_rn(__fmaf_rn(sg, qq.x, q.P[0]), r), V3);
-        const float ey = __fmaf_rn(V5, __fmul_rn(__fmaf_rn(sg, qq.y, q.P[1]), r), V7);
-        const float ez = __fmaf_rn(V10, __fmul_rn(__fmaf_rn(sg, qq.z, q.P[2]), r), V11);
-        const int ix = frx::f2i_sat(ex - q.dx), iy = frx::f2i_sat(ey - q.dy);
-        const bool xyok = (ix == frx::f2i_sat(ex + q.dx)) & (iy == frx::f2i_sat(ey + q.dy));
-        const float cached = ssao_cached(F, depth, ix, iy);
+        const float4 Q = k[3 * s], kk = k[3 * s + 1];
+        // the flip's sign from a fused dot product: |k| < 1 and |n| <= 1 (rounded), so both
+        // it and the reference's rounded dot are within 3 2^-24 of the real one
+        const float dt = __fmaf_rn(kk.z, nrm.z, __fmaf_rn(kk.y, nrm.y, __fmul_rn(kk.x, nrm.x)));
+        const float sg = dt > 0.f ? 1.f : -1.f;
+        const float r = rcp_approx(__fmaf_rn(sg, Q.w, q.P[3]));
+        const float cx = __fmaf_rn(sg, Q.x, q.P[0]), cy = __fmaf_rn(sg, Q.y, q.P[1]), cz = __fmaf_rn(sg, Q.z, q.P[2]);
+        const int ix = frx::f2i_sat(__fmaf_rn(cx, r, q.lo[0])), iy = frx::f2i_sat(__fmaf_rn(cy, r, q.lo[1]));
+        const bool xyok = (ix == frx::f2i_sat(__fmaf_rn(cx, r, q.hi[0]))) & (iy == frx::f2i_sat(__fmaf_rn(cy, r, q.hi[1])));
+        // unchecked DepthBuffer.GetValue(x, y) (render.cpp:255): the linear index reads
+        // wherever it lands inside the buffer; outside, nothing occludes
+        const int li = iy * F.W + ix;
+        float cached = FLT_MAX;
+        if ((unsigned)li < n) cached = __ldg(depth + li);
         const float thr = cached + F.ssaoBias;
-        const bool above = ez - q.dz >= thr, below = ez + q.dz < thr;
-        const bool sure = xyok & (above | below);
+        const bool above = __fmaf_rn(cz, r, q.lo[2]) >= thr, below = __fmaf_rn(cz, r, q.hi[2]) < thr;
+        const bool sure = xyok & (above | below) & (fabsf(dt) > 1e-6f);
         hits += (int)(sure & above & (fabsf(fragDepth - cached) < F.ssaoRange));
         unsure |= sure ? 0u : bit;
     };
@@ -1401,7 +1407,7 @@ __device__ __forceinline__ float ssao_pixel_filtered(const FrameConst& F, const 
         {
             const int s = base + __ffs(unsure) - 1;
             unsure &= unsure - 1u;
-            hits += ssao_sample(F, depth, k[3 * s], k[3 * s + 2], pos, nrm, fragDepth) > 0.f;
+            hits += ssao_sample(F, depth, k[3 * s + 1], k[3 * s + 2], pos, nrm, fragDepth) > 0.f;
         }
     }
     return ssao_result(F, hits);
@@ -1447,12 +1453,12 @@ __global__ void __launch_bounds__(1024) k_ssao_background(FrameConst F, const fl
     ssao_background_cta(F, depth, table, rcb, out16);
 }
 
-// 512-thread CTAs, three per SM (40 registers a thread; the 16-cell sample table
+// 512-thread CTAs, two per SM without spills (three at 40 registers: 95 us against 92; the 16-cell sample table
 // is 49 KB at 64 samples). Launched as a programmatic dependent of the background
 // kernel (one CTA, 5 us): only the background pixels wait for its values.
 constexpr int kSsaoThreads = 512;
 
-__global__ void __launch_bounds__(kSsaoThreads, 3) k_ssao(FrameConst F, GBuffer gb, const float* __restrict__ table,
+__global__ void __launch_bounds__(kSsaoThreads, 2) k_ssao(FrameConst F, GBuffer gb, const float* __restrict__ table,
                                                const float* __restrict__ bg16, const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;
@@ -1460,10 +1466,13 @@ __global__ void __launch_bounds__(kSsaoThreads, 3) k_ssao(FrameConst F, GBuffer 
     const int stride = ssao_q_stride(F.ssaoN);
     ssao_build_table_q(F, table, tbl4, stride);
     __syncthreads();
-    const int n = F.W * F.H;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
+    // tiles of 32 x 16 pixels, a warp a row: the gathers of a CTA's samples overlap in L1
+    const int tw = (F.W + 31) / 32, tiles = tw * ((F.H + kSsaoThreads / 32 - 1) / (kSsaoThreads / 32));
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
     {
-        int x = p % F.W, y = p / F.W;
+        const int x = tile % tw * 32 + (threadIdx.x & 31), y = tile / tw * (kSsaoThreads / 32) + (threadIdx.x >> 5);
+        if (x >= F.W || y >= F.H) continue;
+        const int p = y * F.W + x;
         int cell = (y & 3) * 4 + (x & 3);
         // a covered pixel's depth passed the depth test (< FLT_MAX); the resolve
         // writes FLT_MAX everywhere else, so the depth stands in for the covered flag
@@ -2385,8 +2394,8 @@ void launch_ssao(const FrameConst& F, GBuffer gb, const float* table, float* bg1
     if (withBackground)
         k_ssao_background<<<1, 1024, sizeof(float) * 16 * F.ssaoN, st>>>(F, gb.depth, table, bg16, gate);
     // gated (learned-AO fallback): a small grid-stride grid, so a skipped pass costs little
-    const int grid = gate ? std::min(blocks((long long)F.W * F.H, kSsaoThreads), 2 * 152)
-                          : blocks((long long)F.W * F.H, kSsaoThreads);
+    const int tiles = blocks(F.W, 32) * blocks(F.H, kSsaoThreads / 32);
+    const int grid = gate ? std::min(tiles, 2 * 152) : tiles;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kSsaoThreads);
     cfg.dynamicSmemBytes = smem, cfg.stream = st;

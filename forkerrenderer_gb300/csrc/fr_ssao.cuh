@@ -146,6 +146,39 @@ FR_HD SsaoPlane ssao_plane(const float* M, const float* Vp, bool vportSimple, fl
     return q;
 }
 
+// The form the kernels use: the ends of the test interval straight from fused
+// multiply-adds. With P'_r = RN(Vp_rr P_r) per pixel and Q'_r = RN(Vp_rr Q_r) per table
+// entry (rows x, y, z; row w unscaled) the ends are fma(fma(+-1, Q'_r, P'_r), rcp(c'.w),
+// Vp_r3 -+ d_r). Against the exact value: 5u A_r and 2u, 4u as above; here 10u |Vp_rr| A_r
+// in the numerator (P 4u, Q 3u, the two scalings and the sum u each), 8u A_w in the
+// denominator, 4u for the reciprocal, u each for the end's constant and the last fma. So
+// |exact - end's middle| <= E = 16u |Vp_rr| (A_r + nh_r A_w) / w_lo + 11u (|Vp_rr| nh_r +
+// |Vp_r3|), and the ends lie 2E away (tests/cpp/test_ssao_ends.cpp). ok also bounds the
+// linear pixel index: every sample's int32 x + y W is exact.
+struct SsaoEnds
+{
+    float P[4];             // P'x, P'y, P'z, P.w
+    float lo[3], hi[3];     // Vp_r3 -+ d_r
+    bool ok;
+};
+
+FR_HD SsaoEnds ssao_ends(const float* M, const float* Vp, bool vportSimple, float radius, int W, float px, float py,
+                         float pz)
+{
+    const SsaoPlane q = ssao_plane(M, Vp, vportSimple, radius, px, py, pz);
+    const float s[3] = {Vp[0], Vp[5], Vp[10]}, t[3] = {Vp[3], Vp[7], Vp[11]};
+    // 16 / 14 of ssao_plane's half-widths covers the larger first term
+    const float d[3] = {q.dx * 1.15f, q.dy * 1.15f, q.dz * 1.15f};
+    SsaoEnds e;
+    for (int r = 0; r < 3; ++r) e.P[r] = fmul_x(s[r], q.P[r]), e.lo[r] = t[r] - d[r], e.hi[r] = t[r] + d[r];
+    e.P[3] = q.P[3];
+    // |x|, |y| <= |Vp_rr| nh_r + |Vp_r3| + d: recover the bound from E >= 11u of it
+    const float u11 = 6.5565109252929688e-07f;  // 11 * 2^-24
+    const float bx = q.dx / (2.f * u11), by = q.dy / (2.f * u11);
+    e.ok = q.ok && d[0] <= 0.25f && d[1] <= 0.25f && (by + 4.f) * (float)W + bx < 2.0e9f;
+    return e;
+}
+
 // Per-table-entry part: Q = VP (o, 0), rows x, y, z, w.
 FR_HD void ssao_q(const float* M, float ox, float oy, float oz, float* Q)
 {
