@@ -647,6 +647,27 @@ FR_HD bool bary_on_edge(int e1, int e2, int B, float rB, unsigned long long m53,
     return !(b0 < 0.f);
 }
 
+// bary<0, false> at a pixel the triangle is known to cover, for a fast-class triangle
+// with small coordinates (a resolve's winner): no coverage tests, the edge values as
+// magnitudes.
+FR_HD void bary_covered(const RTri& t, int px, int py, float& b0, float& b1, float& b2)
+{
+    const int s0x = t.x[1] - t.x[0], s0y = t.x[2] - t.x[0], s0z = t.x[0] - px;
+    const int s1x = t.y[1] - t.y[0], s1y = t.y[2] - t.y[0], s1z = t.y[0] - py;
+    const int ex = s0y * s1z - s0z * s1y, ey = s0z * s1x - s0x * s1z, bz = (int)t.bz;
+    const int e1 = ex < 0 ? -ex : ex, e2 = ey < 0 ? -ey : ey, B = bz < 0 ? -bz : bz;
+    const float rB = t.rbz < 0.f ? -t.rbz : t.rbz;
+    if (e1 + e2 != B)
+        bary_off_edge(e1, e2, B, rB, b0, b1, b2);
+    else
+    {
+        unsigned long long m53;
+        int s53;
+        recip53((unsigned long long)B, m53, s53);
+        bary_on_edge(e1, e2, B, rB, m53, s53, b0, b1, b2);
+    }
+}
+
 // Whether any pixel of the box [x0, x1] x [y0, y1] may be covered, for every class:
 // false only if bary() rejects them all. The reference's edge values (bary_reference;
 // the integer classes compute the same exact values) are products and one difference

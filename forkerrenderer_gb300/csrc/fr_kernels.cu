@@ -577,19 +577,46 @@ constexpr int kTileThreads = kTile * kTile;
 // Barrier `id` of one tile's kTileThreads threads (a CTA may hold several tiles).
 __device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTileThreads) : "memory"); }
 
+// A pass' few large triangles (large_direct) also as edge functions of the absolute
+// pixel: E[2j] = (a1, bx1, by1, a2), E[2j + 1] = (bx2, by2, |bz|, 1), or 0 in the last
+// where the triangle or the target is outside the int32 form.
+__device__ __forceinline__ void stage_edges(const frx::RTri& r, const RasterParams& rp, int4* E)
+{
+    const bool ok = r.cls == frx::kTriFast && r.small && rp.W <= frx::kSmallLimit + 1 && rp.H <= frx::kSmallLimit + 1;
+    const frx::SmallEdges e = ok ? frx::small_edges(r, 0, 0) : frx::SmallEdges{};
+    E[0] = make_int4(e.a1, e.bx1, e.by1, e.a2);
+    E[1] = make_int4(e.bx2, e.by2, e.B, ok);
+}
+
+// Coverage and weights of pixel (px, py) in a staged large triangle: by its edges where
+// it has them (E not null), else by its box and the general form.
+__device__ __forceinline__ bool large_fragment(const frx::RTri& t, const int4* E, int4 box, int px, int py, float& b0,
+                                               float& b1, float& b2)
+{
+    if (E && E[1].w)
+    {
+        const int4 E0 = E[0], E1 = E[1];
+        const int e1 = frx::affine_wrapped(E0.x, E0.y, E0.z, px, py);
+        const int e2 = frx::affine_wrapped(E0.w, E1.x, E1.y, px, py);
+        const int c = E1.z - e1 - e2;
+        if ((e1 | e2 | c) < 0) return false;
+        if (c != 0) return frx::bary_off_edge(e1, e2, E1.z, fabsf(t.rbz), b0, b1, b2);
+    }
+    else if (px < box.x || px > box.y || py < box.z || py > box.w)
+        return false;
+    return frx::bary<0, false>(t, px, py, b0, b1, b2);
+}
+
 // The tile's pixel of thread tid against triangles 0 .. cnt - 1 of shared memory: the
-// smaller of `best` and their keys. Every thread of the tile runs the loop (ballots).
+// smaller of `best` and their keys. shE: their edges (large_direct), or null.
 __device__ __forceinline__ unsigned long long tile_min_key(const frx::RTri* sh, const int* shIdx, const int4* shBox,
-                                                           int cnt, bool inside, int px, int py, unsigned long long best)
+                                                           const int4* shE, int cnt, int px, int py,
+                                                           unsigned long long best)
 {
     for (int j = 0; j < cnt; ++j)
     {
-        const int4 bb = shBox[j];
-        const bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
-        if (__ballot_sync(0xffffffffu, inb) == 0u) continue;
-        if (!inb) continue;
         float b0, b1, b2;
-        if (!frx::bary<0, false>(sh[j], px, py, b0, b1, b2)) continue;
+        if (!large_fragment(sh[j], shE ? shE + 2 * j : nullptr, shBox[j], px, py, b0, b1, b2)) continue;
         float d = frx::depth_of(sh[j], b0, b1, b2);
         if (!frx::depth_passes_clear(d)) continue;
         unsigned long long key = frx::make_key(d, (unsigned)shIdx[j]);
@@ -623,7 +650,7 @@ __device__ __noinline__ bool edges_meet_tile(const frx::RTri* r, int tx0, int ty
 template <int CAP>
 __device__ __forceinline__ void tile_raster_body(const RasterParams& rp, const RasterScratch& rs, int tile, int tid, int bar,
                                                  bool direct, bool staged, frx::RTri* sh, int* shIdx, int4* shBox,
-                                                 int* cntSh)
+                                                 int4* shE, int* cntSh)
 {
     long long start = direct ? 0 : rs.tileStart[tile];
     long long end = direct ? min(rs.counters[1], rs.triCap) : min((long long)rs.tileStart[tile + 1], rs.binCap);
@@ -641,7 +668,11 @@ __device__ __forceinline__ void tile_raster_body(const RasterParams& rp, const R
         {
             if (direct)
             {
-                for (int i = tid; i < cnt; i += kTileThreads) stage_large(rp, rs, (int)(base + i), i, sh, shIdx, shBox);
+                if (tid < cnt)  // at most kDirectLarge
+                {
+                    stage_large(rp, rs, (int)(base + tid), tid, sh, shIdx, shBox);
+                    stage_edges(sh[tid], rp, shE + 2 * tid);
+                }
                 tile_sync(bar);
             }
             else
@@ -658,7 +689,7 @@ __device__ __forceinline__ void tile_raster_body(const RasterParams& rp, const R
                 cnt = *cntSh;
             }
         }
-        best = tile_min_key(sh, shIdx, shBox, cnt, inside, px, py, best);
+        if (inside) best = tile_min_key(sh, shIdx, shBox, direct ? shE : nullptr, cnt, px, py, best);
         if (!staged) tile_sync(bar);
     }
     if (inside && best != frx::kEmptyKey) atomicMin(rs.keys + (size_t)py * rp.W + px, best);
@@ -669,8 +700,9 @@ __global__ void __launch_bounds__(256) k_tile_raster(RasterParams rp, RasterScra
     __shared__ frx::RTri sh[kTileBatch];
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
+    __shared__ int4 shE[2 * kDirectLarge];
     __shared__ int cntSh;
-    tile_raster_body<kTileBatch>(rp, rs, blockIdx.x, threadIdx.x, 0, large_direct(rs), false, sh, shIdx, shBox, &cntSh);
+    tile_raster_body<kTileBatch>(rp, rs, blockIdx.x, threadIdx.x, 0, large_direct(rs), false, sh, shIdx, shBox, shE, &cntSh);
 }
 
 // Shadow-map value of texel p from its visibility key: the winning triangle's
@@ -687,13 +719,11 @@ __device__ __forceinline__ float shadow_texel(const DevScene& S, const int4* __r
         {
             frx::RTri r;
             int4 wv;
-            if (load_tri_record(rec, t, r, wv))
+            if (load_tri_record(rec, t, r, wv) && frx::small_pixel(px, py))
             {
                 float b0, b1, b2;
-                if (frx::bary<0, false>(r, px, py, b0, b1, b2))
-                    out = interp(__int_as_float(wv.x), __int_as_float(wv.y), __int_as_float(wv.z), b0, b1, b2) * 0.5f +
-                          0.5f;
-                return out;
+                frx::bary_covered(r, px, py, b0, b1, b2);
+                return interp(__int_as_float(wv.x), __int_as_float(wv.y), __int_as_float(wv.z), b0, b1, b2) * 0.5f + 0.5f;
             }
         }
         int4 tv = S.triV[t];
@@ -726,6 +756,7 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
     __shared__ float4 shZ[kTileBatch];
+    __shared__ int4 shE[2 * kDirectLarge];
     const int tile = blockIdx.x;
     const int ntx = (rp.W + kTile - 1) / kTile;
     const int px = (tile % ntx) * kTile + (threadIdx.x & 15);
@@ -750,20 +781,16 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
             sh[i] = r;
             shIdx[i] = rs.largeIdx[li];
             shZ[i] = rs.largeAux[li];
+            if (direct) stage_edges(r, rp, shE + 2 * i);
             int x0, x1, y0, y1;
             bbox(r, rp.W, rp.H, x0, x1, y0, y1);
             shBox[i] = make_int4(x0, x1, y0, y1);
         }
         __syncthreads();
-        // every thread runs the loop so the warp-wide ballot sees full warps
-        for (int j = 0; j < cnt; ++j)
+        for (int j = 0; inside && j < cnt; ++j)
         {
-            const int4 bb = shBox[j];
-            const bool inb = inside && px >= bb.x && px <= bb.y && py >= bb.z && py <= bb.w;
-            if (__ballot_sync(0xffffffffu, inb) == 0u) continue;
-            if (!inb) continue;
             float b0, b1, b2;
-            if (!frx::bary<0, false>(sh[j], px, py, b0, b1, b2)) continue;
+            if (!large_fragment(sh[j], direct ? shE + 2 * j : nullptr, shBox[j], px, py, b0, b1, b2)) continue;
             const float d = frx::depth_of(sh[j], b0, b1, b2);
             if (!frx::depth_passes_clear(d)) continue;
             const unsigned long long key = frx::make_key(d, (unsigned)shIdx[j]);
@@ -824,6 +851,7 @@ __global__ void __launch_bounds__(kViewTiles * kTileThreads) k_tile_raster_views
     int4* shBox = reinterpret_cast<int4*>(sh + CAP);
     int* shIdx = reinterpret_cast<int*>(shBox + CAP);
     __shared__ int sItem, cntSh[kViewTiles];
+    __shared__ int4 shE[kViewTiles][2 * kDirectLarge];
     RasterParams rp{};
     RasterScratch rs{};
     int cur = -1;         // the pass of rp, rs
@@ -850,12 +878,16 @@ __global__ void __launch_bounds__(kViewTiles * kTileThreads) k_tile_raster_views
                 {
                     tile_sync(1 + g);  // the slot's previous triangles are done with
                     const int n = min(rs.counters[1], rs.triCap);
-                    if (tid < n) stage_large(rp, rs, tid, tid, sh, shIdx, shBox);
+                    if (tid < n)
+                    {
+                        stage_large(rp, rs, tid, tid, sh, shIdx, shBox);
+                        stage_edges(sh[tid], rp, shE[g] + 2 * tid);
+                    }
                     tile_sync(1 + g);
                 }
             }
             tile_raster_body<CAP>(rp, rs, it - itemStart[e], tid, 1 + g, direct, direct, sh, shIdx, shBox,
-                                  cntSh + g);
+                                  shE[g], cntSh + g);
         }
     }
 }
@@ -877,7 +909,9 @@ __device__ bool fragment_inputs(const DevScene& S, const FrameConst& F, const Ve
     frx::RTri r;
     load_rtri(vo.scr, tv, r, false);
     float b0, b1, b2;
-    if (!frx::bary<0, false>(r, px, py, b0, b1, b2)) return false;
+    // the key's triangle covers its pixel
+    if (r.cls == frx::kTriFast && r.small && frx::small_pixel(px, py)) frx::bary_covered(r, px, py, b0, b1, b2);
+    else if (!frx::bary<0, false>(r, px, py, b0, b1, b2)) return false;
     f.material = tt.w;
     f.model = tn.w;
     float4 A0 = vo.pw[tv.x], A1 = vo.pw[tv.y], A2 = vo.pw[tv.z];

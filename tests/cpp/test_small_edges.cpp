@@ -58,6 +58,17 @@ int main(int argc, char** argv)
             const bool want = frx::bary<0, false>(t, x0 + lx, y0 + ly, r0, r1, r2);
             ++pixels;
             covered += want;
+            if (want)
+            {
+                // a resolve's form, and the edges of the absolute pixel
+                float h0, h1, h2;
+                frx::bary_covered(t, x0 + lx, y0 + ly, h0, h1, h2);
+                const frx::SmallEdges z = frx::small_edges(t, 0, 0);
+                if (h0 != r0 || h1 != r1 || h2 != r2 ||
+                    frx::affine_wrapped(z.a1, z.bx1, z.by1, x0 + lx, y0 + ly) != e1 ||
+                    frx::affine_wrapped(z.a2, z.bx2, z.by2, x0 + lx, y0 + ly) != e2)
+                    ++bad;
+            }
             // a zero weight's sign is not part of the form (kZeroSigns = false)
             auto same = [](float a, float b) { return std::memcmp(&a, &b, 4) == 0 || (a == 0.f && b == 0.f); };
             if (got != want || (want && !(same(g0, r0) && same(g1, r1) && same(g2, r2))))
