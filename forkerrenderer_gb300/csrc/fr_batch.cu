@@ -248,7 +248,7 @@ int record(fr_batch* b)
     for (int i = 0; i < kBranches; ++i) B_CUDA(b, cudaStreamWaitEvent(b->br[i], b->forkEv, 0));
     next = 0;
     for (auto& L : b->lights)
-        frk::launch_resolve_shadow(L.S, L.scrL, L.rs.keys, L.F.SW, L.F.SH, L.shadow, b->br[next++ % kBranches]);
+        frk::launch_resolve_shadow(L.S, L.scrL, L.rs, L.F.SW, L.F.SH, L.shadow, b->br[next++ % kBranches]);
     for (auto& V : b->views)
     {
         const bool learned = V.aoMode == FR_AO_LEARNED;
@@ -393,6 +393,10 @@ fr_batch* fr_batch_create(fr_ctx* ctx, const fr_view_desc* views, int32_t n_view
         L.shadow = A.get<float>((size_t)LD.shadow_size * LD.shadow_size);
         if (!alloc_raster(A, L.rs, LD.shadow_size, LD.shadow_size, T, ctx->cfg.bin_capacity))
             return fr_batch_destroy(b), bail("out of device memory");
+        // the resolve reads each winning triangle's record (cleared: a scene without triangles)
+        L.rs.triRec = A.get<int4>(2 * (size_t)L.rs.triCap);
+        if (!L.rs.triRec) return fr_batch_destroy(b), bail("out of device memory");
+        cudaMemset(L.rs.triRec, 0, 2 * sizeof(int4) * L.rs.triCap);
         b->lights.push_back(L);
     }
     // views

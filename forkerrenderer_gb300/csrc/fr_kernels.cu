@@ -52,11 +52,9 @@ __device__ __forceinline__ void store_tri_record(int4* rec, int t, const frx::RT
     rec[2 * (size_t)t + 1] = make_int4(w0, w1, w2, __float_as_int(r.rbz));
 }
 
-// The RTri of a record (false: the triangle has none). d[] is not restored.
-__device__ __forceinline__ bool load_tri_record(const int4* __restrict__ rec, int t, frx::RTri& r, int4& wv)
+// The RTri of a record (a, wv) (false: the triangle has none). d[] is not restored.
+__device__ __forceinline__ bool unpack_tri_record(int4 a, int4 wv, frx::RTri& r)
 {
-    const int4 a = __ldg(rec + 2 * (size_t)t);
-    wv = __ldg(rec + 2 * (size_t)t + 1);
     if (a.w == 0) return false;
     r.x[0] = (a.x << 16) >> 16, r.y[0] = a.x >> 16;
     r.x[1] = (a.y << 16) >> 16, r.y[1] = a.y >> 16;
@@ -707,23 +705,21 @@ __global__ void __launch_bounds__(256) k_tile_raster(RasterParams rp, RasterScra
 
 // Shadow-map value of texel p from its visibility key: the winning triangle's
 // interpolated NDC z mapped to [0, 1] (render.cpp:83-93), 0 where nothing covers it.
-// rec: the pass's resolve records, or null.
-__device__ __forceinline__ float shadow_texel(const DevScene& S, const int4* __restrict__ scrL,
-                                              const int4* __restrict__ rec, unsigned long long key, int px, int py)
+// (ra, rb): the triangle's resolve record (all 0: none).
+__device__ __forceinline__ float shadow_texel(const DevScene& S, const int4* __restrict__ scrL, int4 ra, int4 rb,
+                                              unsigned long long key, int px, int py)
 {
     float out = 0.f;
     if (key != frx::kEmptyKey)
     {
         int t = (int)(key & 0xffffffffu);
-        if (rec)
         {
             frx::RTri r;
-            int4 wv;
-            if (load_tri_record(rec, t, r, wv) && frx::small_pixel(px, py))
+            if (unpack_tri_record(ra, rb, r) && frx::small_pixel(px, py))
             {
                 float b0, b1, b2;
                 frx::bary_covered(r, px, py, b0, b1, b2);
-                return interp(__int_as_float(wv.x), __int_as_float(wv.y), __int_as_float(wv.z), b0, b1, b2) * 0.5f + 0.5f;
+                return interp(__int_as_float(rb.x), __int_as_float(rb.y), __int_as_float(rb.z), b0, b1, b2) * 0.5f + 0.5f;
             }
         }
         int4 tv = S.triV[t];
@@ -741,39 +737,32 @@ __device__ __forceinline__ float shadow_texel(const DevScene& S, const int4* __r
 }
 
 // The shadow pass's fine raster with the shadow-map resolve fused in. The setup
-// and medium passes ran before, and no other CTA touches this tile, so each
-// thread reads its texel's key once up front and resolves it at once (the
-// winner among the small and medium triangles: its vertex gathers overlap the
-// tile's staging), keeps the minimum with the tile's binned triangles in a
-// register and writes it back with a plain store. A texel won by a binned
-// triangle takes its shadow value from the weights of the winning evaluation
-// (the bary() the resolve would repeat) and the vertices' NDC z staged beside
-// the triangle.
+// and medium passes ran before, and no other CTA touches these tiles, so each
+// thread reads its texels' keys once, resolves them at once (the winner among the
+// small and medium triangles) and keeps the minimum with the large triangles in a
+// register. A texel won by a large triangle takes its shadow value from the weights
+// of the winning evaluation (the bary() the resolve would repeat) and the vertices'
+// NDC z staged beside the triangle. The keys are not needed after this.
+// A CTA takes kShadowTiles tiles: with few large triangles (large_direct) they are
+// staged once and the texels' keys, then their records, load together; one texel a
+// thread waited through three dependent loads a tile (63 us for a 2048^2 map, now 50; with
+// four tiles, at four CTAs per SM, 59).
+constexpr int kShadowTiles = 2;
+
 __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, RasterScratch rs, DevScene S,
-                                                            const int4* __restrict__ scrL, float* __restrict__ shadow)
+                                                            const int4* __restrict__ scrL, float* __restrict__ shadow,
+                                                            int tiles)
 {
     __shared__ frx::RTri sh[kTileBatch];
     __shared__ int shIdx[kTileBatch];
     __shared__ int4 shBox[kTileBatch];
     __shared__ float4 shZ[kTileBatch];
     __shared__ int4 shE[2 * kDirectLarge];
-    const int tile = blockIdx.x;
     const int ntx = (rp.W + kTile - 1) / kTile;
-    const int px = (tile % ntx) * kTile + (threadIdx.x & 15);
-    const int py = (tile / ntx) * kTile + (threadIdx.x >> 4);
-    const bool inside = px < rp.W && py < rp.H;
-    const size_t p = inside ? (size_t)py * rp.W + px : 0;
-    const unsigned long long k0 = inside ? __ldcg(rs.keys + p) : frx::kEmptyKey;
-    const float out0 = shadow_texel(S, scrL, rs.triRec, k0, px, py);
-    unsigned long long best = k0;
-    float w0 = 0.f, w1 = 0.f, w2 = 0.f;
-    float4 wz = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int tile0 = blockIdx.x * kShadowTiles;
     const bool direct = large_direct(rs);
-    const long long start = direct ? 0 : rs.tileStart[tile];
-    const long long end = direct ? min(rs.counters[1], rs.triCap) : min((long long)rs.tileStart[tile + 1], rs.binCap);
-    for (long long base = start; base < end; base += kTileBatch)
-    {
-        const int cnt = (int)min((long long)kTileBatch, end - base);
+    // stages cnt triangles from list position `base` (bin entries unless direct)
+    auto stage = [&](long long base, int cnt) {
         for (int i = threadIdx.x; i < cnt; i += blockDim.x)
         {
             const int li = direct ? (int)(base + i) : rs.binTri[base + i];
@@ -786,8 +775,10 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
             bbox(r, rp.W, rp.H, x0, x1, y0, y1);
             shBox[i] = make_int4(x0, x1, y0, y1);
         }
-        __syncthreads();
-        for (int j = 0; inside && j < cnt; ++j)
+    };
+    // the smaller of `best` and the staged triangles' keys at a texel, its value in `out`
+    auto nearest = [&](int cnt, int px, int py, unsigned long long& best, float& out) {
+        for (int j = 0; j < cnt; ++j)
         {
             float b0, b1, b2;
             if (!large_fragment(sh[j], direct ? shE + 2 * j : nullptr, shBox[j], px, py, b0, b1, b2)) continue;
@@ -797,20 +788,70 @@ __global__ void __launch_bounds__(256, 5) k_tile_raster_shadow(RasterParams rp, 
             if (key < best)
             {
                 best = key;
-                w0 = b0, w1 = b1, w2 = b2;
-                wz = shZ[j];
+                out = interp(shZ[j].x, shZ[j].y, shZ[j].z, b0, b1, b2) * 0.5f + 0.5f;
             }
         }
-        __syncthreads();
-    }
-    if (!inside) return;
-    if (best != k0)
+    };
+    int px[kShadowTiles], py[kShadowTiles];
+    unsigned long long k0[kShadowTiles];
+    int4 ra[kShadowTiles], rb[kShadowTiles];
+#pragma unroll
+    for (int k = 0; k < kShadowTiles; ++k)
     {
-        rs.keys[p] = best;
-        shadow[p] = interp(wz.x, wz.y, wz.z, w0, w1, w2) * 0.5f + 0.5f;
+        const int tile = tile0 + k;
+        px[k] = (tile % ntx) * kTile + (threadIdx.x & 15);
+        py[k] = (tile / ntx) * kTile + (threadIdx.x >> 4);
+        const bool in = tile < tiles && px[k] < rp.W && py[k] < rp.H;
+        if (!in) px[k] = -1;
+        k0[k] = in ? __ldcg(rs.keys + (size_t)py[k] * rp.W + px[k]) : frx::kEmptyKey;
     }
-    else
-        shadow[p] = out0;
+    if (direct) stage(0, min(rs.counters[1], rs.triCap));
+#pragma unroll
+    for (int k = 0; k < kShadowTiles; ++k)
+    {
+        const bool has = rs.triRec && k0[k] != frx::kEmptyKey;
+        const int4* r = rs.triRec + 2 * (size_t)(has ? (unsigned)k0[k] : 0u);
+        ra[k] = has ? __ldg(r) : make_int4(0, 0, 0, 0);
+        rb[k] = has ? __ldg(r + 1) : make_int4(0, 0, 0, 0);
+    }
+    if (direct)
+    {
+        __syncthreads();
+        const int cnt = min(rs.counters[1], rs.triCap);
+#pragma unroll
+        for (int k = 0; k < kShadowTiles; ++k)
+        {
+            if (px[k] < 0) continue;
+            float out = shadow_texel(S, scrL, ra[k], rb[k], k0[k], px[k], py[k]);
+            nearest(cnt, px[k], py[k], k0[k], out);
+            shadow[(size_t)py[k] * rp.W + px[k]] = out;
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int k = 0; k < kShadowTiles && tile0 + k < tiles; ++k)
+    {
+        const int tile = tile0 + k, x = (tile % ntx) * kTile + (threadIdx.x & 15), y = (tile / ntx) * kTile + (threadIdx.x >> 4);
+        const bool in = x < rp.W && y < rp.H;
+        unsigned long long best = in ? __ldcg(rs.keys + (size_t)y * rp.W + x) : frx::kEmptyKey;
+        int4 a = make_int4(0, 0, 0, 0), b = a;
+        if (rs.triRec && best != frx::kEmptyKey)
+        {
+            a = __ldg(rs.triRec + 2 * (size_t)(unsigned)best);
+            b = __ldg(rs.triRec + 2 * (size_t)(unsigned)best + 1);
+        }
+        float out = in ? shadow_texel(S, scrL, a, b, best, x, y) : 0.f;
+        const long long end = min((long long)rs.tileStart[tile + 1], rs.binCap);
+        for (long long base = rs.tileStart[tile]; base < end; base += kTileBatch)
+        {
+            const int cnt = (int)min((long long)kTileBatch, end - base);
+            stage(base, cnt);
+            __syncthreads();
+            if (in) nearest(cnt, x, y, best, out);
+            __syncthreads();
+        }
+        if (in) shadow[(size_t)y * rp.W + x] = out;
+    }
 }
 
 // Shared-memory bytes of CAP staged triangles.
@@ -970,11 +1011,13 @@ __device__ __forceinline__ unsigned pack_rgb(unsigned r, unsigned g, unsigned b)
 
 // DepthShader::ProcessFragment (depthshader.h:30-36) of the surviving triangle.
 __global__ void k_resolve_shadow(DevScene S, const int4* __restrict__ scrL, const unsigned long long* __restrict__ keys,
-                                 int SW, int SH, float* __restrict__ shadow)
+                                 const int4* __restrict__ rec, int SW, int SH, float* __restrict__ shadow)
 {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= SW * SH) return;
-    shadow[p] = shadow_texel(S, scrL, nullptr, keys[p], p % SW, p / SW);
+    const unsigned long long key = keys[p];
+    const size_t t = key != frx::kEmptyKey ? (unsigned)key : 0u;
+    shadow[p] = shadow_texel(S, scrL, __ldg(rec + 2 * t), __ldg(rec + 2 * t + 1), key, p % SW, p / SW);
 }
 
 // GShader::ProcessFragment (gshader.h:95-202) of the surviving triangle, into the
@@ -2343,7 +2386,8 @@ void launch_raster(const DevScene& S, const int4* scr, const RasterParams& rp, R
     int sms = 152;
     k_raster_medium<<<sms * 8, kMediumThreads, 0, st>>>(rp, rs, tiles);
     k_bin<<<sms * 4, 256, 0, st>>>(rp, rs);
-    if (tileRaster && shadowOut) k_tile_raster_shadow<<<tiles, 256, 0, st>>>(rp, rs, S, scr, shadowOut);
+    if (tileRaster && shadowOut) 
+        k_tile_raster_shadow<<<blocks(tiles, kShadowTiles), 256, 0, st>>>(rp, rs, S, scr, shadowOut, tiles);
     else if (tileRaster) k_tile_raster<<<tiles, 256, 0, st>>>(rp, rs);
     launches += tileRaster ? 4 : 3;
 }
@@ -2387,10 +2431,10 @@ void launch_lighting_views(const DevScene& S, const ViewShade* views, const int*
         launch_lighting_views_t<false>(S, views, itemStart, nViews, total, lights, nLights, queue, T, grid, st);
 }
 
-void launch_resolve_shadow(const DevScene& S, const int4* scrL, const unsigned long long* keys, int SW, int SH,
-                           float* shadow, cudaStream_t st)
+void launch_resolve_shadow(const DevScene& S, const int4* scrL, const RasterScratch& rs, int SW, int SH, float* shadow,
+                           cudaStream_t st)
 {
-    k_resolve_shadow<<<blocks((long long)SW * SH, 256), 256, 0, st>>>(S, scrL, keys, SW, SH, shadow);
+    k_resolve_shadow<<<blocks((long long)SW * SH, 256), 256, 0, st>>>(S, scrL, rs.keys, rs.triRec, SW, SH, shadow);
 }
 
 void launch_resolve_gbuffer(const DevScene& S, const FrameConst& F, VertexOut vo, const unsigned long long* keys,

@@ -102,8 +102,9 @@ void launch_lighting_views(const frd::DevScene& S, const ViewShade* views, const
                            const BatchLight* lights, int nLights, int* queue, int T, int grid, cudaStream_t st);
 
 // Resolves.
-void launch_resolve_shadow(const frd::DevScene& S, const int4* scrL, const unsigned long long* keys, int SW,
-                           int SH, float* shadow, cudaStream_t st);
+// (rs.triRec holds the pass' resolve records)
+void launch_resolve_shadow(const frd::DevScene& S, const int4* scrL, const RasterScratch& rs, int SW, int SH,
+                           float* shadow, cudaStream_t st);
 void launch_resolve_gbuffer(const frd::DevScene& S, const frd::FrameConst& F, frd::VertexOut vo,
                             const unsigned long long* keys, frd::GBuffer gb, cudaStream_t st);
 // counters / statusOut (optional): block 0 copies the 8 raster counters to statusOut
