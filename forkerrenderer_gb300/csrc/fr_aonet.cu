@@ -75,6 +75,7 @@ __global__ void k_pool_fwd(const uint4* __restrict__ in, uint4* __restrict__ out
 __global__ void k_pool_bwd_add_mask(const uint4* __restrict__ gc, const uint4* __restrict__ gp,
                                     const uint4* __restrict__ mask, uint4* __restrict__ out, int BC8, int H, int W)
 {
+    griddep_wait();
     const int n = BC8 * H * W;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -113,43 +114,57 @@ __device__ __forceinline__ float up_weight(int o, int j, int n)
 
 // Transpose of k_up_fwd, then the ReLU mask of the low-resolution activation:
 // g(j,i) = (sum_oy w(oy) * sum_ox w(ox) * G(oy,ox)) * (mask(j,i) > 0), outputs in ascending order.
-__global__ void k_up_bwd_mask(const uint4* __restrict__ G, const uint4* __restrict__ mask, uint4* __restrict__ out,
-                              int BC8, int h, int w)
+// Eight threads an output: thread r sums the row oy = 4j - 2 + r, then thread e adds up
+// the rows of channel e in order (one thread an output walked 64 vectors: 17 us at
+// level 0 -> 1 of a 16 x 256 x 256 batch, 15 us with 8,192 threads at level 1 -> 2).
+constexpr int kUpBwdThreads = 256;
+__global__ void __launch_bounds__(kUpBwdThreads) k_up_bwd_mask(const uint4* __restrict__ G, const uint4* __restrict__ mask,
+                                                               __nv_bfloat16* __restrict__ out, int BC8, int h, int w)
 {
+    static_assert(kScale == 4, "eight output rows and columns reach an input pixel");
+    __shared__ float rows[kUpBwdThreads][9];  // [output * 8 + row][channel], padded
+    griddep_wait();
     const int H = kScale * h, W = kScale * w;
     const int n = BC8 * h * w;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
+    const int idx = (blockIdx.x * kUpBwdThreads + threadIdx.x) >> 3, k = threadIdx.x & 7;
     const int i = idx % w;
     const int r = idx / w;
     const int j = r % h;
     const int bc = r / h;
-    const uint4* src = G + static_cast<size_t>(bc) * H * W;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int oy = kScale * j - kScale / 2; oy < kScale * j + kScale + kScale / 2; ++oy)
+    const int oy = kScale * j - kScale / 2 + k;
+    float row[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (idx < n && oy >= 0 && oy < H)
     {
-        if (oy < 0 || oy >= H) continue;
-        const float wy = up_weight(oy, j, h);
-        if (wy == 0.f) continue;
-        float row[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int ox = kScale * i - kScale / 2; ox < kScale * i + kScale + kScale / 2; ++ox)
+        const uint4* src = G + (static_cast<size_t>(bc) * H + oy) * W;
+#pragma unroll
+        for (int d = 0; d < 2 * kScale; ++d)
         {
+            const int ox = kScale * i - kScale / 2 + d;
             if (ox < 0 || ox >= W) continue;
             const float wx = up_weight(ox, i, w);
             if (wx == 0.f) continue;
             float g[8];
-            unpack8(src[oy * W + ox], g);
+            unpack8(src[ox], g);
 #pragma unroll
             for (int e = 0; e < 8; ++e) row[e] += wx * g[e];
         }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += wy * row[e];
     }
-    float m[8];
-    unpack8(mask[idx], m);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = m[e] > 0.f ? acc[e] : 0.f;
-    out[idx] = pack8(acc);
+    for (int e = 0; e < 8; ++e) rows[threadIdx.x][e] = row[e];
+    __syncthreads();
+    if (idx >= n) return;
+    float acc = 0.f;
+#pragma unroll
+    for (int q = 0; q < 2 * kScale; ++q)
+    {
+        const int y = kScale * j - kScale / 2 + q;
+        if (y < 0 || y >= H) continue;
+        const float wy = up_weight(y, j, h);
+        if (wy == 0.f) continue;
+        acc += wy * rows[(threadIdx.x & ~7) + q][k];
+    }
+    const float m = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(mask)[static_cast<size_t>(idx) * 8 + k]);
+    out[static_cast<size_t>(idx) * 8 + k] = __float2bfloat16_rn(m > 0.f ? acc : 0.f);
 }
 
 // ---- input rearrangement, head backward + loss ---------------------------------
@@ -183,6 +198,7 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_bwd(const float* __restri
                                                            int h, int w, float invN)
 {
     __shared__ float red[kHeadSums][kHeadThreads / 32];
+    griddep_wait();
     const int HW = h * w;
     const int n = B * HW;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -223,12 +239,37 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_bwd(const float* __restri
         }
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // The warp's sums. The 64 head weights as a reduce-scatter: in the step of distance o
+    // each lane hands half of its values over and adds the other half, 62 exchanges
+    // instead of 5 for each value, in the same tree of additions.
+    constexpr int kW = kHeadOut * 16;
+    static_assert(kW == 64, "two values a lane after five halvings");
+    float v[kW];
+#pragma unroll
+    for (int k = 0; k < kW; ++k) v[k] = s[1 + k];
+#pragma unroll
+    for (int o = 16, half = kW / 2; o > 0; o >>= 1, half >>= 1)
+    {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < half; ++k)
+        {
+            const float give = upper ? v[k] : v[k + half], keep = upper ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    // lane bits 4..0 chose the halves: values 2 * bit-reversed order of the halvings
+    const int first = ((lane >> 4) & 1) * 32 + ((lane >> 3) & 1) * 16 + ((lane >> 2) & 1) * 8 + ((lane >> 1) & 1) * 4 +
+                      (lane & 1) * 2;
+    red[1 + first][wid] = v[0];
+    red[2 + first][wid] = v[1];
 #pragma unroll
     for (int k = 0; k < kHeadSums; ++k)
     {
-        float v = s[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[k][wid] = v;
+        if (k >= 1 && k <= kW) continue;  // the loss and the head's biases
+        float x = s[k];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) red[k][wid] = x;
     }
     __syncthreads();
     for (int k = threadIdx.x; k < kHeadSums; k += blockDim.x)
@@ -301,6 +342,7 @@ __device__ __forceinline__ void two_sum_add(float& hi, float& lo, float x)
 // over 120 thousand gradients), the last of a row for the bias.
 __global__ void __launch_bounds__(kReduceThreads) k_grad_reduce(const __grid_constant__ ReduceArgs R)
 {
+    griddep_wait();
     if (blockIdx.x < kHeadSums) return reduce_head(R, blockIdx.x);
     int L = 0;
     while (L + 1 < kNumLayers && static_cast<int>(blockIdx.x) >= R.layer[L + 1].block0) ++L;
@@ -339,11 +381,47 @@ __global__ void __launch_bounds__(kReduceThreads) k_grad_reduce(const __grid_con
         a.db[co] = total;
 }
 
+// The layers' places in the parameter vector and their packed BF16 weights.
+struct PackLayer
+{
+    int off, cin, cout;    // W[cout][cin][9] at params + off
+    __nv_bfloat16 *fwd, *bwd;
+};
+struct PackArgs
+{
+    PackLayer layer[kNumLayers];
+};
+
+// Parameter i in the BF16 shared-memory layouts of k_conv3x3, if it is a 3x3 weight:
+// forward  [tap][cin/8][cout][8]
+// backward [tap'][cout/8][cin][8] with W'[ci][co][t'] = W[co][ci][8 - t'] (a 3x3
+//          convolution of the output gradient gives the input gradient).
+__device__ __forceinline__ void pack_weight(const PackArgs& P, int i, float w)
+{
+    int L = kNumLayers - 1;
+    while (L > 0 && i < P.layer[L].off) --L;
+    const PackLayer& a = P.layer[L];
+    const int k = i - a.off;
+    if (k >= a.cout * a.cin * 9) return;  // a bias, or the head
+    const int t = k % 9, q = k / 9, ci = q % a.cin, co = q / a.cin;
+    const __nv_bfloat16 v = __float2bfloat16_rn(w);
+    a.fwd[((t * (a.cin / 8) + ci / 8) * a.cout + co) * 8 + ci % 8] = v;
+    if (a.bwd) a.bwd[(((8 - t) * (a.cout / 8) + co / 8) * a.cin + ci) * 8 + co % 8] = v;
+}
+
+__global__ void k_pack(const float* __restrict__ p, int n, const __grid_constant__ PackArgs P)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) pack_weight(P, i, p[i]);
+}
+
 // PyTorch's Adam: m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2;
 // p -= step * m / (sqrt(v) / bc2sqrt + eps), step = lr / (1 - b1^t), bc2sqrt = sqrt(1 - b2^t).
+// The thread packs its new weight too (a launch a layer took 30 us of a training step).
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int n, float b1, float b2, float eps, float step, float bc2sqrt)
+                       int n, float b1, float b2, float eps, float step, float bc2sqrt, const __grid_constant__ PackArgs P)
 {
+    griddep_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -351,54 +429,9 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
     const float vi = b2 * v[i] + (1.f - b2) * (gi * gi);
     m[i] = mi;
     v[i] = vi;
-    p[i] -= step * (mi / (sqrtf(vi) / bc2sqrt + eps));
-}
-
-__constant__ int c_pairA[5] = {0, 2, 4, 6, 7};
-__constant__ int c_pairB[5] = {1, 3, 5, 7, 8};
-
-// Packs FP32 W[cout][cinReal][9] into the BF16 shared-memory layouts of k_conv3x3:
-// forward  [tap][cin/8][cout][8]           (paired input layer: [pair][2][cout][8])
-// backward [tap'][cout/8][cin][8] with W'[ci][co][t'] = W[co][ci][8 - t'] (a 3x3
-//          convolution of the output gradient gives the input gradient).
-__global__ void k_pack(const float* __restrict__ W, int cin, int cinReal, int cout, int paired,
-                       __nv_bfloat16* __restrict__ fwd, __nv_bfloat16* __restrict__ bwd)
-{
-    const int nf = paired ? 5 * 2 * cout * 8 : 9 * cin * cout;
-    const int nb = bwd ? 9 * cin * cout : 0;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nf)
-    {
-        const int e = i & 7;
-        const int r = i >> 3;
-        const int co = r % cout;
-        const int q = r / cout;  // tap * (cin/8) + chunk, or pair * 2 + which
-        float val = 0.f;
-        if (paired)
-        {
-            const int pr = q >> 1, which = q & 1;
-            const int t = which ? c_pairB[pr] : c_pairA[pr];
-            if (e < cinReal && !(pr == 4 && which == 0)) val = W[(co * cinReal + e) * 9 + t];
-        }
-        else
-        {
-            const int t = q / (cin / 8), cc = q % (cin / 8);
-            const int ci = cc * 8 + e;
-            if (ci < cinReal) val = W[(co * cinReal + ci) * 9 + t];
-        }
-        fwd[i] = __float2bfloat16_rn(val);
-    }
-    else if (i < nf + nb)
-    {
-        const int k = i - nf;
-        const int e = k & 7;
-        const int r = k >> 3;
-        const int ci = r % cin;  // output channel of the backward convolution
-        const int q = r / cin;   // tap' * (cout/8) + chunk
-        const int tp = q / (cout / 8), cc = q % (cout / 8);
-        const int co = cc * 8 + e;
-        bwd[k] = __float2bfloat16_rn(W[(co * cinReal + ci) * 9 + (8 - tp)]);
-    }
+    const float w = p[i] - step * (mi / (sqrtf(vi) / bc2sqrt + eps));
+    p[i] = w;
+    pack_weight(P, i, w);
 }
 
 // ---- tensor maps ------------------------------------------------------------------
@@ -613,18 +646,18 @@ int ensure_bwd(fr_aonet* n, long long pix)
     return FR_OK;
 }
 
+PackArgs pack_args(const fr_aonet* n)
+{
+    PackArgs P{};
+    for (int L = 0; L < kNumLayers; ++L)
+        P.layer[L] = PackLayer{n->paramOff[L], kLayers[L].c0 + kLayers[L].c1, kLayers[L].cout, n->packFwd[L],
+                               L > 0 ? n->packBwd[L] : nullptr};
+    return P;
+}
+
 int pack_all(fr_aonet* n, cudaStream_t st)
 {
-    for (int L = 0; L < kNumLayers; ++L)
-    {
-        const LayerSpec& s = kLayers[L];
-        const int cin = s.c0 + s.c1;
-        const int paired = cin == 8;
-        const int nf = paired ? 5 * 2 * s.cout * 8 : 9 * cin * s.cout;
-        const int nb = L > 0 ? 9 * cin * s.cout : 0;
-        k_pack<<<blocks_for(nf + nb, 256), 256, 0, st>>>(n->params + n->paramOff[L], cin, s.cinReal, s.cout, paired,
-                                                          n->packFwd[L], L > 0 ? n->packBwd[L] : nullptr);
-    }
+    k_pack<<<blocks_for(kNumParams, 256), 256, 0, st>>>(n->params, kNumParams, pack_args(n));
     NET_CUDA(n, cudaGetLastError());
     return FR_OK;
 }
@@ -817,7 +850,7 @@ int wgrad_all(fr_aonet* n, const WgradLayer* layers, int headBlocks, float invN,
     R.gradsHead = n->grads + n->paramOff[kNumLayers];
     R.loss = n->lossDev, R.invN = invN;
     launch_wgrad(U, grid, st);
-    k_grad_reduce<<<rblocks, kReduceThreads, 0, st>>>(R);
+    launch_pdl(k_grad_reduce, rblocks, kReduceThreads, st, R);
     n->launches += 2;
     return FR_OK;
 }
@@ -948,13 +981,13 @@ int backward_impl(fr_aonet* n, const uint16_t* in, const float* label, const Sha
         const LayerSpec& s = kLayers[L];
         // backward data: input channels = the layer's cout, output channels = its cin
         return conv(n, S, s.level, dy, s.cout, nullptr, 0, s.c0 + s.c1, n->packBwd[L],
-                    9u * (s.c0 + s.c1) * s.cout * 2u, nullptr, true, out0, co0, out1, mask, nullptr, nullptr, st);
+                    9u * (s.c0 + s.c1) * s.cout * 2u, nullptr, true, out0, co0, out1, mask, nullptr, nullptr, st, true);
     };
     const float invN = 1.f / static_cast<float>(pix * kHeadOut);  // full-resolution pixels
     const int hb = blocks_for(pix, kHeadThreads);
-    k_head_bwd<<<hb, kHeadThreads, 0, st>>>(n->aoTmp, label, reinterpret_cast<const uint4*>(n->a7),
-                                            n->params + n->paramOff[kNumLayers], reinterpret_cast<uint4*>(n->g7),
-                                            n->headPart, S.B, S.H, S.W, invN);
+    launch_pdl(k_head_bwd, hb, kHeadThreads, st, static_cast<const float*>(n->aoTmp), label,
+               reinterpret_cast<const uint4*>(n->a7), static_cast<const float*>(n->params + n->paramOff[kNumLayers]),
+               reinterpret_cast<uint4*>(n->g7), n->headPart, S.B, S.H, S.W, invN);
     n->launches++;
     WgradLayer wg[kNumLayers];
     auto WG = [&](int L, const uint16_t* x0, const uint16_t* x1, const uint16_t* dy) {
@@ -965,23 +998,23 @@ int backward_impl(fr_aonet* n, const uint16_t* in, const float* label, const Sha
     NET_TRY(DG(9, n->g7, n->g6, 16, nullptr, n->a6));
     NET_TRY(WG(8, n->u0, n->s0, n->g6));
     NET_TRY(DG(8, n->g6, n->gu0, 32, n->gs0c, nullptr));
-    k_up_bwd_mask<<<blocks_for((long long)S.B * 4 * S.h(1) * S.w(1), 256), 256, 0, st>>>(
-        reinterpret_cast<const uint4*>(n->gu0), reinterpret_cast<const uint4*>(n->a5), reinterpret_cast<uint4*>(n->g5),
-        S.B * 4, S.h(1), S.w(1));
+    launch_pdl(k_up_bwd_mask, blocks_for(8LL * S.B * 4 * S.h(1) * S.w(1), kUpBwdThreads), kUpBwdThreads, st,
+               reinterpret_cast<const uint4*>(n->gu0), reinterpret_cast<const uint4*>(n->a5),
+               reinterpret_cast<__nv_bfloat16*>(n->g5), S.B * 4, S.h(1), S.w(1));
     // level 1 decoder
     NET_TRY(WG(7, n->a4, nullptr, n->g5));
     NET_TRY(DG(7, n->g5, n->g4, 32, nullptr, n->a4));
     NET_TRY(WG(6, n->u1, n->s1, n->g4));
     NET_TRY(DG(6, n->g4, n->gu1, 64, n->gs1c, nullptr));
-    k_up_bwd_mask<<<blocks_for((long long)S.B * 8 * S.h(2) * S.w(2), 256), 256, 0, st>>>(
-        reinterpret_cast<const uint4*>(n->gu1), reinterpret_cast<const uint4*>(n->a3), reinterpret_cast<uint4*>(n->g3),
-        S.B * 8, S.h(2), S.w(2));
+    launch_pdl(k_up_bwd_mask, blocks_for(8LL * S.B * 8 * S.h(2) * S.w(2), kUpBwdThreads), kUpBwdThreads, st,
+               reinterpret_cast<const uint4*>(n->gu1), reinterpret_cast<const uint4*>(n->a3),
+               reinterpret_cast<__nv_bfloat16*>(n->g3), S.B * 8, S.h(2), S.w(2));
     // bottleneck
     NET_TRY(WG(5, n->a2, nullptr, n->g3));
     NET_TRY(DG(5, n->g3, n->g2, 64, nullptr, n->a2));
     NET_TRY(WG(4, n->p1, nullptr, n->g2));
     NET_TRY(DG(4, n->g2, n->gp1, 32, nullptr, nullptr));
-    k_pool_bwd_add_mask<<<blocks_for((long long)S.B * 4 * S.h(1) * S.w(1), 256), 256, 0, st>>>(
+    launch_pdl(k_pool_bwd_add_mask, blocks_for((long long)S.B * 4 * S.h(1) * S.w(1), 256), 256, st,
         reinterpret_cast<const uint4*>(n->gs1c), reinterpret_cast<const uint4*>(n->gp1),
         reinterpret_cast<const uint4*>(n->s1), reinterpret_cast<uint4*>(n->gS1), S.B * 4, S.h(1), S.w(1));
     // level 1 encoder
@@ -989,7 +1022,7 @@ int backward_impl(fr_aonet* n, const uint16_t* in, const float* label, const Sha
     NET_TRY(DG(3, n->gS1, n->g1, 32, nullptr, n->a1));
     NET_TRY(WG(2, n->p0, nullptr, n->g1));
     NET_TRY(DG(2, n->g1, n->gp0, 16, nullptr, nullptr));
-    k_pool_bwd_add_mask<<<blocks_for((long long)S.B * 2 * S.H * S.W, 256), 256, 0, st>>>(
+    launch_pdl(k_pool_bwd_add_mask, blocks_for((long long)S.B * 2 * S.H * S.W, 256), 256, st,
         reinterpret_cast<const uint4*>(n->gs0c), reinterpret_cast<const uint4*>(n->gp0),
         reinterpret_cast<const uint4*>(n->s0), reinterpret_cast<uint4*>(n->gS0), S.B * 2, S.H, S.W);
     // level 0 encoder
@@ -1115,7 +1148,7 @@ fr_aonet* fr_aonet_create(int32_t device, uint64_t seed, char* err, size_t errle
     {
         const LayerSpec& sp = kLayers[L];
         const int cin = sp.c0 + sp.c1;
-        n->packFwdBytes[L] = cin == 8 ? 5u * 2u * 8u * sp.cout * 2u : 9u * cin * sp.cout * 2u;
+        n->packFwdBytes[L] = 9u * cin * sp.cout * 2u;
         ok = cudaMalloc(&n->packFwd[L], n->packFwdBytes[L]) == cudaSuccess;
         if (ok && L > 0) ok = cudaMalloc(&n->packBwd[L], 9u * cin * sp.cout * 2u) == cudaSuccess;
     }
@@ -1229,12 +1262,10 @@ int fr_aonet_adam_step(fr_aonet* n, float lr, float beta1, float beta2, float ep
     n->adamT++;
     const double bc1 = 1.0 - std::pow(static_cast<double>(beta1), static_cast<double>(n->adamT));
     const double bc2 = 1.0 - std::pow(static_cast<double>(beta2), static_cast<double>(n->adamT));
-    k_adam<<<blocks_for(kNumParams, 256), 256, 0, st>>>(n->params, n->grads, n->adamM, n->adamV, kNumParams, beta1,
-                                                        beta2, eps, static_cast<float>(lr / bc1),
-                                                        static_cast<float>(std::sqrt(bc2)));
+    launch_pdl(k_adam, blocks_for(kNumParams, 256), 256, st, n->params, static_cast<const float*>(n->grads), n->adamM,
+               n->adamV, static_cast<int>(kNumParams), beta1, beta2, eps, static_cast<float>(lr / bc1),
+               static_cast<float>(std::sqrt(bc2)), pack_args(n));
     n->launches++;
-    NET_TRY(pack_all(n, st));
-    n->launches += kNumLayers;
     NET_CUDA(n, cudaGetLastError());
     return FR_OK;
 }

@@ -589,6 +589,7 @@ __global__ void __launch_bounds__(192) k_wgrad(const __grid_constant__ WgradArgs
     frtc::tc_fence_after();
     const uint32_t tmem = sy.tmem;
     volatile int* abortp = &sy.abort;
+    griddep_wait();
     // this CTA's chains k0, k0 + ctas, ... in groups of `sets`; a group's tiles go
     // round by round (one tile of each chain), which every role walks alike
     const int mine = (nch - 1 - k0) / ctas + 1;
@@ -821,7 +822,17 @@ void launch_wgrad(const WgradArgs& a, int grid, cudaStream_t st)
         cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
         attr = true;
     }
-    k_wgrad<<<grid, 192, kWgradSmem, st>>>(a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = kWgradSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_wgrad, a);
 }
 
 }  // namespace fra
