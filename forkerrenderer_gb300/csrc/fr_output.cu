@@ -63,13 +63,16 @@ enum SrcKind : int
     kSrcF1 = 2,     // float: Buffer1f::GenerateImage
     kSrcF3 = 3,     // float3: Buffer3f::GenerateImage
     kSrcGVec = 4,   // float4 plane of the packed G-buffer (normal or world position), as a Buffer3f
-    kSrcGMat = 5,   // material field of the packed G-buffer (albedo, param: Buffer3f; shading type: Buffer1f)
-    kSrcGMatLinear = 6  // the same of a bilinear-filtered frame (the G-buffer holds texture coordinates)
+    // material fields of the packed G-buffer (albedo, param: Buffer3f; shading type: Buffer1f),
+    // and of a bilinear-filtered frame's (its G-buffer holds texture coordinates)
+    kSrcAlbedo = 5, kSrcParam = 6, kSrcType = 7,
+    kSrcLinear = 8,  // kinds from here on sample textures
+    kSrcAlbedoLinear = 8, kSrcParamLinear = 9, kSrcTypeLinear = 10
 };
 
 struct PixelSrc
 {
-    int kind, bpp, which;  // which (kSrcGMat): 3 albedo, 5 param, 6 shading type
+    int kind, bpp;
     const void* p;
     GBuffer gb;
     DevScene S;
@@ -88,10 +91,19 @@ __device__ __forceinline__ uint32_t bgr3(F3 c)
     return ref_u8(c.z * 254.99f) | (ref_u8(c.y * 254.99f) << 8) | (ref_u8(c.x * 254.99f) << 16);
 }
 
-// Pixel i's bytes in TGA order, packed little-endian into 32 bits. The kind is
-// a template argument so unrolled loops keep all their loads in flight.
+// What a pixel is read as, and its bytes in TGA order, packed little-endian into 32
+// bits, from that. The kind is a template argument and the two are apart so that
+// unrolled loops keep all their loads in flight.
+template <int K> struct RawOf { using T = uint4; };  // a G-buffer word
+template <> struct RawOf<kSrcBytes> { using T = uint32_t; };
+template <> struct RawOf<kSrcRgbx> { using T = uint32_t; };
+template <> struct RawOf<kSrcF1> { using T = float; };
+template <> struct RawOf<kSrcF3> { using T = F3; };
+template <> struct RawOf<kSrcGVec> { using T = float4; };
+template <int K> using Raw = typename RawOf<K>::T;
+
 template <int K>
-__device__ __forceinline__ uint32_t pix(const PixelSrc& s, long long i)
+__device__ __forceinline__ Raw<K> load_pixel(const PixelSrc& s, long long i)
 {
     if constexpr (K == kSrcBytes)
     {
@@ -101,43 +113,54 @@ __device__ __forceinline__ uint32_t pix(const PixelSrc& s, long long i)
         if (s.bpp == 4) v |= (uint32_t)p[3] << 24;
         return v;
     }
-    else if constexpr (K == kSrcRgbx)
-    {
-        const uint32_t c = static_cast<const uint32_t*>(s.p)[i];
-        return ((c >> 16) & 0xffu) | (c & 0xff00u) | ((c & 0xffu) << 16);
-    }
-    else if constexpr (K == kSrcF1)
-        return ref_u8(static_cast<const float*>(s.p)[i] * 255);
+    else if constexpr (K == kSrcRgbx || K == kSrcF1 || K == kSrcGVec)
+        return static_cast<const Raw<K>*>(s.p)[i];
     else if constexpr (K == kSrcF3)
     {
         const float* f = static_cast<const float*>(s.p) + 3 * i;
-        return bgr3(F3{f[0], f[1], f[2]});
-    }
-    else if constexpr (K == kSrcGVec)
-    {
-        const float4 v = static_cast<const float4*>(s.p)[i];
-        return bgr3(F3{v.x, v.y, v.z});
+        return F3{f[0], f[1], f[2]};
     }
     else
+        return s.gb.c[i];
+}
+
+template <int K>
+__device__ __forceinline__ uint32_t tga_pixel(const PixelSrc& s, const Raw<K>& v)
+{
+    if constexpr (K == kSrcBytes) return v;
+    else if constexpr (K == kSrcRgbx) return ((v >> 16) & 0xffu) | (v & 0xff00u) | ((v & 0xffu) << 16);
+    else if constexpr (K == kSrcF1) return ref_u8(v * 255);
+    else if constexpr (K == kSrcF3) return bgr3(v);
+    else if constexpr (K == kSrcGVec) return bgr3(F3{v.x, v.y, v.z});
+    else
     {
-        const GDecoded g = decode_gbuffer_t<K == kSrcGMatLinear>(s.S, s.gb.c[i]);
-        if (s.which == 6) return ref_u8(g.type * 255);
-        return bgr3(s.which == 3 ? g.albedo : g.param);
+        const GDecoded g = decode_gbuffer_t<(K >= kSrcLinear)>(s.S, v);
+        if constexpr (K == kSrcType || K == kSrcTypeLinear) return ref_u8(g.type * 255);
+        else if constexpr (K == kSrcAlbedo || K == kSrcAlbedoLinear) return bgr3(g.albedo);
+        else return bgr3(g.param);
     }
+}
+
+template <int K>
+__device__ __forceinline__ uint32_t pix(const PixelSrc& s, long long i)
+{
+    return tga_pixel<K>(s, load_pixel<K>(s, i));
 }
 
 // Calls BODY<K>(args...) for the source kind k (uniform across a CTA). LIN: the
 // kernel is instantiated for bilinear G-buffers (a compile-time flag), so the
 // nearest-filtered instantiations carry none of the texture sampling code.
-#define FRO_BY_KIND(LIN, k, BODY, ...)                                      \
-    switch (k)                                                              \
-    {                                                                       \
-        case kSrcBytes: BODY<kSrcBytes>(__VA_ARGS__); break;                \
-        case kSrcRgbx: BODY<kSrcRgbx>(__VA_ARGS__); break;                  \
-        case kSrcF1: BODY<kSrcF1>(__VA_ARGS__); break;                      \
-        case kSrcF3: BODY<kSrcF3>(__VA_ARGS__); break;                      \
-        case kSrcGVec: BODY<kSrcGVec>(__VA_ARGS__); break;                  \
-        default: BODY<(LIN) ? kSrcGMatLinear : kSrcGMat>(__VA_ARGS__); break; \
+#define FRO_BY_KIND(LIN, k, BODY, ...)                                                        \
+    switch (k)                                                                                \
+    {                                                                                         \
+        case kSrcBytes: BODY<kSrcBytes>(__VA_ARGS__); break;                                  \
+        case kSrcRgbx: BODY<kSrcRgbx>(__VA_ARGS__); break;                                    \
+        case kSrcF1: BODY<kSrcF1>(__VA_ARGS__); break;                                        \
+        case kSrcF3: BODY<kSrcF3>(__VA_ARGS__); break;                                        \
+        case kSrcGVec: BODY<kSrcGVec>(__VA_ARGS__); break;                                    \
+        case kSrcAlbedo: case kSrcAlbedoLinear: BODY<(LIN) ? kSrcAlbedoLinear : kSrcAlbedo>(__VA_ARGS__); break; \
+        case kSrcParam: case kSrcParamLinear: BODY<(LIN) ? kSrcParamLinear : kSrcParam>(__VA_ARGS__); break; \
+        default: BODY<(LIN) ? kSrcTypeLinear : kSrcType>(__VA_ARGS__); break;                 \
     }
 
 __device__ void put_header(uint8_t* o, int w, int h, int bpp, int rle, int vflip)
@@ -211,30 +234,79 @@ __device__ __forceinline__ int job_of_group(const Jobs& J, int blk)
     return ji;
 }
 
-// Bit r of eqw: pixel seg0 + r equals its successor (r < kWinWords * 32). Warp w
-// handles words w * kPer .. w * kPer + kPer - 1, every load issued before the
-// first comparison; a word's last pixel finds its successor in the next word.
+// Bit r of eqw: pixel seg0 + r equals its successor (r < kWinWords * 32). Every load
+// of a warp is issued before its first comparison. Kinds of four bytes a pixel go four
+// pixels a lane, where the source is aligned for it: warp w takes the 128-pixel groups
+// w, w + kParseWarps, ...; a lane's four bits join into words by three shuffles. The
+// others go a lane a pixel: warp w takes the words w * kPer .. w * kPer + kPer - 1.
 template <int K>
 __device__ __forceinline__ void equality_bits(const Job& jb, long long seg0, uint32_t* eqw)
 {
-    constexpr int kPer = (kWinWords + kParseWarps - 1) / kParseWarps;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int left = (int)min(jb.n - seg0, (long long)(32 * kWinWords + 1));  // pixels that matter here
+    if constexpr (K == kSrcRgbx || K == kSrcF1)
+    {
+        if ((reinterpret_cast<uintptr_t>(jb.src.p) & 15) == 0)
+        {
+            constexpr int kGroups = kWinWords / 4, kPer = (kGroups + kParseWarps - 1) / kParseWarps;
+            static_assert(kSeg % 4 == 0 && kWinWords % 4 == 0, "whole groups, 16-byte loads");
+            const Raw<K>* src = static_cast<const Raw<K>*>(jb.src.p) + seg0;
+            Raw<K> v[kPer][5];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+            {
+                const int r = 128 * (warp + i * kParseWarps) + 4 * lane;
+#pragma unroll
+                for (int e = 0; e < 5; ++e) v[i][e] = 0;
+                if (warp + i * kParseWarps >= kGroups) continue;
+                if (r + 4 <= left)
+                {
+                    const uint4 q = *reinterpret_cast<const uint4*>(src + r);
+                    memcpy(&v[i][0], &q, 16);
+                }
+                else
+                    for (int e = 0; e < 4; ++e)
+                        if (r + e < left) v[i][e] = src[r + e];
+                if (lane == 31 && r + 4 < left) v[i][4] = src[r + 4];
+            }
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+            {
+                const int grp = warp + i * kParseWarps, r = 128 * grp + 4 * lane;
+                if (grp >= kGroups) break;
+                uint32_t px[5];
+#pragma unroll
+                for (int e = 0; e < 5; ++e) px[e] = tga_pixel<K>(jb.src, v[i][e]);
+                const uint32_t next = __shfl_down_sync(0xffffffffu, px[0], 1);
+                if (lane < 31) px[4] = next;
+                uint32_t m = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m |= (uint32_t)(px[e] == px[e + 1] && r + e + 1 < left) << e;
+                m <<= 4 * (lane & 7);
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+                if ((lane & 7) == 0) eqw[4 * grp + (lane >> 3)] = m;
+            }
+            return;
+        }
+    }
+    constexpr int kPer = (kWinWords + kParseWarps - 1) / kParseWarps;
     const int w0 = warp * kPer;
     uint32_t av[kPer + 1];
 #pragma unroll
     for (int i = 0; i <= kPer; ++i)
     {
-        const long long g = seg0 + (long long)(w0 + i) * 32 + lane;
-        av[i] = (i < kPer || lane == 0) && w0 + i <= kWinWords && g < jb.n ? pix<K>(jb.src, g) : 0u;
+        const int r = 32 * (w0 + i) + lane;
+        av[i] = (i < kPer || lane == 0) && r < left ? pix<K>(jb.src, seg0 + r) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < kPer; ++i)
     {
-        const long long g = seg0 + (long long)(w0 + i) * 32 + lane;
+        const int r = 32 * (w0 + i) + lane;
         uint32_t b = __shfl_down_sync(0xffffffffu, av[i], 1);
         const uint32_t next = __shfl_sync(0xffffffffu, av[i + 1], 0);
         if (lane == 31) b = next;
-        const unsigned m = __ballot_sync(0xffffffffu, g + 1 < jb.n && av[i] == b);
+        const unsigned m = __ballot_sync(0xffffffffu, r + 1 < left && av[i] == b);
         if (lane == 0 && w0 + i < kWinWords) eqw[w0 + i] = m;
     }
 }
@@ -243,19 +315,21 @@ __device__ __forceinline__ void equality_bits(const Job& jb, long long seg0, uin
 // each 128-pixel sub-block (carrying the packets' file bytes) the sub-block transfer
 // functions, stored for k_tga_write; composed over the 32 sub-blocks, the
 // segment's transfer function and its byte counts.
-// Bound by instruction issue. A warp owns a sub-block: its eight equality words (own and
-// look-ahead) sit in the lanes, so the end of every packet is one bit scan of the
-// position's own word or a shuffle from the first later word that has such a bit. Its
-// doubling needs no CTA barrier and ends when every path has left the sub-block (mostly
-// after one to three of the seven rounds). Scanning words in shared memory at each
-// position and seven CTA-wide rounds took 111 us for the ten images of a 1280 x 800 frame.
+// Bound by instruction issue. A warp owns a sub-block, a lane four neighbouring
+// positions: its eight equality words (own and look-ahead) sit in the lanes, so the
+// first later pixel with such a bit is one bit scan or shuffle for the last of the four
+// and a select for each one before. The doubling needs no CTA barrier and ends when
+// every path has left the sub-block (mostly after one to three of seven rounds); a
+// sub-block inside one run, the background's case, needs none of it. Scanning words in
+// shared memory at each position and seven CTA-wide rounds took 111 us for the nine
+// images of a 1280 x 800 frame (12.4 million pixels); this form takes 57 us.
 template <bool kLin>
 __global__ void __launch_bounds__(kParseThreads, 4) k_tga_parse(const __grid_constant__ Jobs J)
 {
     constexpr int kQuarter = kSubBlocks / 4;
     static_assert(kParseThreads == 4 * 128, "a quarter of the sub-blocks per 128 threads");
     __shared__ uint32_t eqw[kWinWords];
-    __shared__ uint32_t F[kSeg];  // next packet start, from the sub-block's first position | file bytes << 16
+    __shared__ __align__(16) uint32_t F[kSeg];  // next packet start, from the sub-block's first position | file bytes << 16
     __shared__ uint32_t Q[4][128];
     const Job& jb = J.j[job_of(J, blockIdx.x)];
     const int k = blockIdx.x - jb.segBase, bpp = jb.bpp;
@@ -268,55 +342,72 @@ __global__ void __launch_bounds__(kParseThreads, 4) k_tga_parse(const __grid_con
         const long long pos0 = seg0 + 128 * sb;
         const int left = (int)max(0ll, min(n - pos0, 4096ll));  // pixels of the image from here
         uint32_t* P = F + 128 * sb;
+        const int r0 = 4 * lane;
         const uint32_t v = eqw[4 * sb + (lane & 7)];
         const unsigned hasZero = __ballot_sync(0xffffffffu, v != ~0u) & 0xffu;
         const unsigned hasOne = __ballot_sync(0xffffffffu, v != 0u) & 0xffu;
-        const int firstZero = 32 * (lane & 7) + __ffs(~v) - 1, firstOne = 32 * (lane & 7) + __ffs(v) - 1;
+        uint32_t* info = reinterpret_cast<uint32_t*>(jb.info + pos0 + r0);  // slices are padded to 256 bytes
         uint32_t x[4];
-        bool more = false;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
+        if (hasZero == 0)  // 256 equal pixels and one more: a full run packet at every position
         {
-            const uint32_t w = __shfl_sync(0xffffffffu, v, i);
-            const unsigned zs = hasZero >> (i + 1), os = hasOne >> (i + 1);
-            const int z = __shfl_sync(0xffffffffu, firstZero, (i + __ffs(zs)) & 7);
-            const int o = __shfl_sync(0xffffffffu, firstOne, (i + __ffs(os)) & 7);
-            const int r = 32 * i + lane;
-            const bool run = (w >> lane) & 1u;
-            // a run ends at the first pixel unequal to its successor, a raw packet before
-            // the first later pixel equal to its successor
-            const uint32_t t = run ? ~w & (~0u << lane) : w & (~1u << lane);
-            const int later = run ? (zs ? z : 256) : (os ? o : 256);
-            const int p = t ? 32 * i + __ffs(t) - 1 : later;
-            const int L = run ? min(128, p - r + 1) : p <= r + 126 ? p - r : min(128, left - r);
-            x[i] = 128u;  // past the image: terminal
-            if (r < left)
-            {
-                jb.info[pos0 + r] = (uint8_t)((L - 1) | (run ? 0x80 : 0));
-                x[i] = (uint32_t)(r + L) | (uint32_t)(run ? 1 + bpp : 1 + L * bpp) << 16;
-            }
-            more = more || (x[i] & 0xffffu) < 128u;
-            P[r] = x[i];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = (uint32_t)(r0 + j + 128) | (uint32_t)(1 + bpp) << 16;
+            *info = 0xffffffffu;
+            *reinterpret_cast<uint4*>(P + r0) = make_uint4(x[0], x[1], x[2], x[3]);
         }
-        __syncwarp();
-        while (__any_sync(0xffffffffu, more))
+        else
         {
-            more = false;
+            const int wi = lane >> 3, b0 = r0 & 31;
+            const uint32_t w = __shfl_sync(0xffffffffu, v, wi);
+            const unsigned zs = hasZero >> (wi + 1), os = hasOne >> (wi + 1);
+            // first zero and first one of the words after this lane's
+            const int fz = 32 * (lane & 7) + __ffs(~v) - 1, fo = 32 * (lane & 7) + __ffs(v) - 1;
+            int z = __shfl_sync(0xffffffffu, fz, (wi + __ffs(zs)) & 7);
+            int o = __shfl_sync(0xffffffffu, fo, (wi + __ffs(os)) & 7);
+            if (!zs) z = 256;
+            if (!os) o = 256;
+            // first zero and first one after position r0 + 3
+            const uint32_t above = ~1u << (b0 + 3);
+            if (~w & above) z = 32 * wi + __ffs(~w & above) - 1;
+            if (w & above) o = 32 * wi + __ffs(w & above) - 1;
+            uint32_t bytes4 = 0;
+            bool more = false;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if ((x[i] & 0xffffu) < 128u)
-                {
-                    x[i] = P[x[i] & 0xffffu] + (x[i] & 0xffff0000u);  // at most 255 pixels * 5 bytes in all
-                    more = more || (x[i] & 0xffffu) < 128u;
-                }
+            for (int j = 3; j >= 0; --j)
+            {
+                const int r = r0 + j;
+                const bool run = (w >> (b0 + j)) & 1u;
+                // a run ends at the first pixel unequal to its successor, a raw packet
+                // before the first later pixel equal to its successor
+                const int L = run ? min(128, z - r + 1) : o <= r + 126 ? o - r : min(128, left - r);
+                if (run) o = r;
+                else z = r;
+                bytes4 = bytes4 << 8 | ((uint32_t)(L - 1) & 0x7fu) | (run ? 0x80u : 0u);
+                x[j] = r < left ? (uint32_t)(r + L) | (uint32_t)(run ? 1 + bpp : 1 + L * bpp) << 16
+                                : 128u;  // past the image: terminal
+                more = more || (x[j] & 0xffffu) < 128u;
+            }
+            if (r0 < left) *info = bytes4;
+            *reinterpret_cast<uint4*>(P + r0) = make_uint4(x[0], x[1], x[2], x[3]);
             __syncwarp();
+            while (__any_sync(0xffffffffu, more))
+            {
+                more = false;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) P[32 * i + lane] = x[i];
-            __syncwarp();
+                for (int j = 0; j < 4; ++j)
+                    if ((x[j] & 0xffffu) < 128u)
+                    {
+                        x[j] = P[x[j] & 0xffffu] + (x[j] & 0xffff0000u);  // at most 255 pixels * 5 bytes in all
+                        more = more || (x[j] & 0xffffu) < 128u;
+                    }
+                __syncwarp();
+                *reinterpret_cast<uint4*>(P + r0) = make_uint4(x[0], x[1], x[2], x[3]);
+                __syncwarp();
+            }
         }
         // sub-block function: offset of the first packet start in the next sub-block
-#pragma unroll
-        for (int i = 0; i < 4; ++i) jb.sub[(size_t)k * kSeg + 128 * sb + 32 * i + lane] = (uint8_t)(x[i] & 127u);
+        *reinterpret_cast<uint32_t*>(jb.sub + (size_t)k * kSeg + 128 * sb + r0) =
+            (x[0] & 127u) | (x[1] & 127u) << 8 | (x[2] & 127u) << 16 | (x[3] & 127u) << 24;
     }
     __syncthreads();
     // the segment's function: each quarter's 8 sub-blocks in a chain, then the 4 quarters
@@ -349,11 +440,37 @@ __global__ void __launch_bounds__(kParseThreads, 4) k_tga_parse(const __grid_con
 // Waits for the kernel before (programmatic launch).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// bytes (a multiple of 8, at most kMost) from the scratch buffer to shared memory, both
+// 8-byte aligned, by a compose CTA; past L1, for what other CTAs of the launch wrote.
+template <int kMost>
+__device__ __forceinline__ void copy8(void* dst, const void* src, int bytes)
+{
+    constexpr int kPer = (kMost / 8 + kComposeThreads - 1) / kComposeThreads, kBatch = kPer < 8 ? kPer : 8;
+    for (int i0 = 0; i0 < bytes / 8; i0 += kBatch * kComposeThreads)
+    {
+        uint2 v[kBatch];
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+        {
+            const int i = i0 + j * kComposeThreads + threadIdx.x;
+            v[j] = i < bytes / 8 ? __ldcg(static_cast<const uint2*>(src) + i) : make_uint2(0, 0);
+        }
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+        {
+            const int i = i0 + j * kComposeThreads + threadIdx.x;
+            if (i < bytes / 8) static_cast<uint2*>(dst)[i] = v[j];
+        }
+    }
+}
+
 // CTA per group of gsz segments: composes the group's transfer function (and
 // byte counts) segment by segment, keeping for every segment the map from the
 // group's entry offset to its own (pre, preB). The last CTA of an image to
 // finish chains its <= kMaxGroups group functions from offset 0 and gives every
-// segment its entry offset and file offset; it writes header, footer and size.
+// segment its entry offset and file offset; it writes header, footer and size. A chain of
+// latencies: the maps come in 8-byte loads, all of a batch in flight (18 -> 13 us for nine
+// images).
 __global__ void __launch_bounds__(kComposeThreads) k_tga_compose(const __grid_constant__ Jobs J)
 {
     __shared__ __align__(16) uint8_t buf[kMaxGroups * 128 * 5];  // staged maps, then group maps
@@ -372,11 +489,8 @@ __global__ void __launch_bounds__(kComposeThreads) k_tga_compose(const __grid_co
     for (int c0 = k0; c0 < k1; c0 += kComposeChunk)
     {
         const int c1 = min(k1, c0 + kComposeChunk);
-        for (int i = tid; i < (c1 - c0) * 128; i += kComposeThreads)
-        {
-            fs[i >> 7][i & 127] = jb.func[(size_t)c0 * 128 + i];
-            fb[i >> 7][i & 127] = jb.fbytes[(size_t)c0 * 128 + i];
-        }
+        copy8<kComposeChunk * 128>(fs, jb.func + (size_t)c0 * 128, (c1 - c0) * 128);
+        copy8<kComposeChunk * 256>(fb, jb.fbytes + (size_t)c0 * 128, (c1 - c0) * 256);
         __syncthreads();
         if (tid < 128)
             for (int k = c0; k < c1; ++k)
@@ -401,11 +515,8 @@ __global__ void __launch_bounds__(kComposeThreads) k_tga_compose(const __grid_co
     __threadfence();
     uint8_t(*gf)[128] = reinterpret_cast<uint8_t(*)[128]>(buf);
     uint32_t(*gb)[128] = reinterpret_cast<uint32_t(*)[128]>(buf + kMaxGroups * 128);
-    for (int i = tid; i < jb.G * 128; i += kComposeThreads)
-    {
-        gf[i >> 7][i & 127] = __ldcg(jb.gfun + i);
-        gb[i >> 7][i & 127] = __ldcg(jb.gbytes + i);
-    }
+    copy8<kMaxGroups * 128>(gf, jb.gfun, jb.G * 128);
+    copy8<kMaxGroups * 512>(gb, jb.gbytes, jb.G * 512);
     __syncthreads();
     if (tid == 0)
     {
@@ -442,51 +553,46 @@ __global__ void __launch_bounds__(kComposeThreads) k_tga_compose(const __grid_co
 
 constexpr int kWriteWarps = kWriteThreads / 32;
 constexpr int kWriteWords = (kWinWords + kWriteWarps - 1) / kWriteWarps;  // 32-pixel words per warp
+constexpr int kWriteBatch = 3;  // words whose pixels are loaded together
 constexpr int kStageBytes = ((kSeg + 128) * 5 + 16 + 15) & ~15;          // a segment's packets + alignment
-
-// The pixels of the warp's words, a lane a pixel, loaded together (issued before the
-// packet walk, so their latency hides behind it).
-template <int K>
-__device__ __forceinline__ void prefetch_pixels(const Job& jb, long long seg0, uint32_t (&px)[kWriteWords])
-{
-    const int w0 = (threadIdx.x >> 5) * kWriteWords;
-#pragma unroll
-    for (int i = 0; i < kWriteWords; ++i)
-    {
-        const long long g = seg0 + 32 * (w0 + i) + (threadIdx.x & 31);
-        px[i] = w0 + i < kWinWords && g < jb.n ? pix<K>(jb.src, g) : 0u;
-    }
-}
 
 // Bytes of the packets that start in the segment, which are those of its pixels
 // [a, b), into the staging buffer (stg[s0 + i] is the file byte at base + i,
 // s0 = base & 15). A packet start has a header byte, and a pixel is stored unless a run
 // packet that began before it covers it: it starts no packet and equals its predecessor.
-// So two bit masks a word of 32 pixels give every pixel's place by population counts, and
-// a warp's sum needs no shuffles. Returns the bytes staged.
-__device__ __forceinline__ int stage_segment(int bpp, int a, int b, int s0, const uint32_t (&px)[kWriteWords],
-                                             const uint8_t* inf, const uint32_t* starts, uint32_t* stored, uint8_t* stg,
-                                             int* warpSum)
+// So two bit masks a word of 32 pixels give every pixel's place by population counts. Only stored pixels are read. total: the bytes staged.
+template <int K>
+__device__ __forceinline__ void stage_segment(const Job& jb, long long seg0, int a, int b, int s0, const uint8_t* inf,
+                                              const uint32_t* starts, uint2* stored, uint8_t* stg, int* warpSum,
+                                              int& total)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * kWriteWords;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * kWriteWords, bpp = jb.bpp;
     const unsigned below = (1u << lane) - 1u;
-    int sum = 0;
-    uint32_t carry = warp > 0 ? inf[32 * w0 - 1] >> 7 : 0u;
+    // the run bits of the warp's words, a word a lane; then every word's masks and place at once
+    uint32_t run = 0;
 #pragma unroll
     for (int i = 0; i < kWriteWords; ++i)
     {
-        const int w = w0 + i;
-        if (w >= kWinWords) break;
-        const uint32_t run = __ballot_sync(0xffffffffu, inf[32 * w + lane] & 0x80);
-        const uint32_t st = w < kSegWords ? starts[w] : 0u;
-        const int lo = min(max(a - 32 * w, 0), 32), hi = min(max(b - 32 * w, 0), 32);
-        const uint32_t inside = (hi == 32 ? ~0u : (1u << hi) - 1u) & (lo == 32 ? 0u : ~0u << lo);
-        const uint32_t keep = (st | ~(run << 1 | carry)) & inside;
-        carry = run >> 31;
-        if (lane == 0) stored[w] = keep;
-        sum += __popc(st) + bpp * __popc(keep);
+        const uint32_t m = w0 + i < kWinWords ? __ballot_sync(0xffffffffu, inf[32 * (w0 + i) + lane] & 0x80) : 0u;
+        if (lane == i) run = m;
     }
-    if (lane == 0) warpSum[warp] = sum;
+    const int wl = w0 + lane;
+    const bool own = lane < kWriteWords && wl < kWinWords;
+    uint32_t carry = __shfl_up_sync(0xffffffffu, run, 1) >> 31;
+    if (lane == 0) carry = warp > 0 ? inf[32 * w0 - 1] >> 7 : 0u;
+    const uint32_t stw = own && wl < kSegWords ? starts[wl] : 0u;
+    const int lo = min(max(a - 32 * wl, 0), 32), hi = min(max(b - 32 * wl, 0), 32);
+    const uint32_t inside = (hi == 32 ? ~0u : (1u << hi) - 1u) & (lo == 32 ? 0u : ~0u << lo);
+    const uint32_t keepw = own ? (stw | ~(run << 1 | carry)) & inside : 0u;
+    const int mine = __popc(stw) + bpp * __popc(keepw);
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
+    {
+        const int u = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += u;
+    }
+    if (lane == 31) warpSum[warp] = incl;
     __syncthreads();
     int o = s0, all = 0;
 #pragma unroll
@@ -495,27 +601,44 @@ __device__ __forceinline__ int stage_segment(int bpp, int a, int b, int s0, cons
         o += w < warp ? warpSum[w] : 0;
         all += warpSum[w];
     }
-#pragma unroll
-    for (int i = 0; i < kWriteWords; ++i)
+    total = all;
+    if (own) stored[wl] = make_uint2(keepw, (uint32_t)(o + incl - mine));
+    __syncwarp();
+    // a batch of words: the kept pixels' loads, then their bytes
+    for (int i0 = 0; i0 < kWriteWords; i0 += kWriteBatch)
     {
-        const int w = w0 + i;
-        if (w >= kWinWords) break;
-        const uint32_t st = w < kSegWords ? starts[w] : 0u, keep = stored[w];
-        uint8_t* d = stg + o + __popc(st & below) + bpp * __popc(keep & below);
-        if ((st >> lane) & 1u)
+        Raw<K> v[kWriteBatch];
+#pragma unroll
+        for (int i = 0; i < kWriteBatch; ++i)
         {
-            const int v = inf[32 * w + lane], L = (v & 127) + 1;
-            *d++ = (uint8_t)((v & 0x80) ? L + 127 : L - 1);
+            const int w = w0 + i0 + i;
+            v[i] = Raw<K>{};
+            if (i0 + i < kWriteWords && w < kWinWords && ((stored[w].x >> lane) & 1u))
+                v[i] = load_pixel<K>(jb.src, seg0 + 32 * w + lane);
         }
-        if ((keep >> lane) & 1u)
+#pragma unroll
+        for (int i = 0; i < kWriteBatch; ++i)
         {
-            d[0] = (uint8_t)px[i];
-            if (bpp >= 3) d[1] = (uint8_t)(px[i] >> 8), d[2] = (uint8_t)(px[i] >> 16);
-            if (bpp == 4) d[3] = (uint8_t)(px[i] >> 24);
+            const int w = w0 + i0 + i;
+            if (i0 + i >= kWriteWords || w >= kWinWords) break;
+            const uint32_t keep = stored[w].x;
+            if (!keep) continue;  // all of it inside run packets that began before
+            const uint32_t st = w < kSegWords ? starts[w] : 0u;
+            uint8_t* d = stg + stored[w].y + __popc(st & below) + bpp * __popc(keep & below);
+            if ((st >> lane) & 1u)
+            {
+                const int f = inf[32 * w + lane], L = (f & 127) + 1;
+                *d++ = (uint8_t)((f & 0x80) ? L + 127 : L - 1);
+            }
+            if ((keep >> lane) & 1u)
+            {
+                const uint32_t px = tga_pixel<K>(jb.src, v[i]);
+                d[0] = (uint8_t)px;
+                if (bpp >= 3) d[1] = (uint8_t)(px >> 8), d[2] = (uint8_t)(px >> 16);
+                if (bpp == 4) d[3] = (uint8_t)(px >> 24);
+            }
         }
-        o += __popc(st) + bpp * __popc(keep);
     }
-    return all;
 }
 
 // Per segment: its packet starts (the segment's entry through the 32 sub-block
@@ -523,13 +646,17 @@ __device__ __forceinline__ int stage_segment(int bpp, int a, int b, int s0, cons
 // packets), then the packets' bytes, staged in shared memory and copied out in
 // 16-byte stores. Lanes hold neighbouring pixels: a run of 17 pixels a thread, each
 // with its own scan of the packet state, made every load touch 32 lines and took 107 us
-// for the ten images of a 1280 x 800 frame.
+// for the nine images of a 1280 x 800 frame; this form takes 51 us. Three words' loads at a time and eight CTAs
+// an SM: the walk and the loads are latency, so more CTAs hide more of it (6 words and
+// four CTAs: 77 us, 9 and five 72, 6 and six 64, 3 and eight 55, before the masks of a
+// warp's words were formed a word a lane).
 template <bool kLin>
-__global__ void __launch_bounds__(kWriteThreads, 4) k_tga_write(const __grid_constant__ Jobs J)
+__global__ void __launch_bounds__(kWriteThreads, 8) k_tga_write(const __grid_constant__ Jobs J)
 {
     __shared__ __align__(16) uint8_t inf[kSeg + 128];
     __shared__ __align__(16) uint8_t work[kStageBytes];  // sub-block maps, then the staged bytes
-    __shared__ uint32_t bits[kSegWords], stored[kWinWords];
+    __shared__ uint32_t bits[kSegWords];
+    __shared__ uint2 stored[kWinWords];  // a word's stored pixels, and where its bytes begin
     __shared__ uint8_t xs[kSubBlocks];
     __shared__ int warpSum[kWriteThreads / 32];
     const Job& jb = J.j[job_of(J, blockIdx.x)];
@@ -537,8 +664,6 @@ __global__ void __launch_bounds__(kWriteThreads, 4) k_tga_write(const __grid_con
     const long long n = jb.n, seg0 = (long long)kk * kSeg;
     const int segLen = (int)min((long long)kSeg, n - seg0);
     const int avail = (int)min((long long)kSeg + 128, n - seg0);
-    uint32_t px[kWriteWords];
-    FRO_BY_KIND(kLin, jb.src.kind, prefetch_pixels, jb, seg0, px)
     griddep_wait();
     {
         // info and sub-block map words (scratch slices are 256-byte aligned and padded)
@@ -589,7 +714,8 @@ __global__ void __launch_bounds__(kWriteThreads, 4) k_tga_write(const __grid_con
     __syncthreads();  // the sub-block maps are done with: the buffer becomes the staging buffer
     const long long base = kHeaderBytes + jb.segOff[kk];
     const int s0 = (int)(base & 15);
-    const int total = stage_segment(jb.bpp, a, bEnd, s0, px, inf, bits, stored, work, warpSum);
+    int total = 0;
+    FRO_BY_KIND(kLin, jb.src.kind, stage_segment, jb, seg0, a, bEnd, s0, inf, bits, stored, work, warpSum, total)
     __syncthreads();
     // stg[i] -> out[(base & ~15) + i] for i in [s0, s0 + total); bytes past cap - 26 are dropped
     const long long g0 = base - s0;
@@ -698,7 +824,7 @@ int encode_batch(const EncodeJob* list, int count, void* scratch, cudaStream_t s
         if (!jb.rle || jb.n == 0)
         {
             const long long threads = jb.n > 0 && !jb.rle ? jb.n : 1;
-            if (jb.src.kind == kSrcGMatLinear)
+            if (jb.src.kind >= kSrcLinear)
                 k_tga_plain<true><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(jb);
             else
                 k_tga_plain<false><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(jb);
@@ -713,7 +839,7 @@ int encode_batch(const EncodeJob* list, int count, void* scratch, cudaStream_t s
     {
         cudaMemsetAsync(counters, 0, kCounterBytes, st);
         bool lin = false;
-        for (int i = 0; i < J.count; ++i) lin = lin || J.j[i].src.kind == kSrcGMatLinear;
+        for (int i = 0; i < J.count; ++i) lin = lin || J.j[i].src.kind >= kSrcLinear;
         if (lin) k_tga_parse<true><<<seg, kParseThreads, 0, st>>>(J);
         else k_tga_parse<false><<<seg, kParseThreads, 0, st>>>(J);
         launch_after(k_tga_compose, groups, kComposeThreads, st, J);
@@ -760,9 +886,9 @@ bool image_source(fr_ctx* ctx, int image, PixelSrc& src, int& w, int& h)
         default:
         {
             if (!ctx->info.deferred) return false;
-            src.kind = ctx->S.texLinear ? kSrcGMatLinear : kSrcGMat;
+            src.kind = (image == FR_OUT_GB_ALBEDO ? kSrcAlbedo : image == FR_OUT_GB_PARAM ? kSrcParam : kSrcType) +
+                       (ctx->S.texLinear ? kSrcAlbedoLinear - kSrcAlbedo : 0);
             src.bpp = image == FR_OUT_GB_SHADING_TYPE ? 1 : 3;
-            src.which = image == FR_OUT_GB_ALBEDO ? 3 : image == FR_OUT_GB_PARAM ? 5 : 6;
             return true;
         }
     }

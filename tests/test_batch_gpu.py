@@ -152,3 +152,68 @@ def test_multi_light_views_match_oracle(shadow_mode, mixed):
                 got_s = b.download(-1 - k, N.FR_BUF_SHADOW).reshape(s.shape)
                 assert np.array_equal(got_s.view(np.uint32), s.view(np.uint32)), k
     b.close()
+
+
+@pytest.mark.parametrize("areas", [(4, 8), (0, 0), (4, 4096)], ids=["binned", "all_binned", "medium"])
+@pytest.mark.parametrize("name", ["def_stress", "def_ao_128"])
+def test_raster_paths_match_render_frame(name, areas):
+    """Area thresholds that send nearly every triangle through the bins (or the medium
+    raster) of a batch, over an odd-sized shadow map: the same bits as the single frame."""
+    if not gpu_available():
+        pytest.skip("no CUDA GPU")
+    import forkerrenderer_gb300 as fr
+    from forkerrenderer_gb300 import _native as N
+    from forkerrenderer_gb300.batch import Batch, point_light, view
+    from scenes import render_config, scene_path
+
+    scene = fr.Scene(scene_path(name))
+    cfg = render_config(name, shadow_size=127)
+    r = fr.Renderer(**cfg)
+    r.Preconfigure(scene)
+    r.Render()
+    s = fr.Renderer(**cfg, small_tri_area=areas[0], medium_tri_area=areas[1])
+    s.Preconfigure(scene)
+    info, m = scene.info, scene.frame_matrices(127)
+    b = Batch(s, [view(m, info.eye)] * 3, [point_light(info.light_pos, info.light_color, 127)])
+    b.render()
+    b.timings()
+    for i in range(3):
+        assert np.array_equal(b.download(i, N.FR_BUF_DEPTH).view(np.uint32), r.depth().view(np.uint32))
+        assert np.array_equal(b.download(i, N.FR_BUF_FRAME_U8), r.frame8())
+    assert np.array_equal(b.download(-1, N.FR_BUF_SHADOW).view(np.uint32), r.shadow_map().view(np.uint32))
+    b.close()
+
+
+@pytest.mark.parametrize("size", [(1, 1), (3, 5), (85, 41), (701, 601)])
+def test_downloads_to_pinned_and_pageable_memory(size):
+    """A packed frame into pinned memory, pageable memory at an odd address and through
+    Batch.download: the same bytes (odd byte counts; above 1 MB several threads copy), and
+    nothing past the frame is written."""
+    fr, scene, cfg, r = _setup()
+    import ctypes as C
+
+    import torch
+
+    from forkerrenderer_gb300 import _native as N
+    from forkerrenderer_gb300.batch import Batch, view
+
+    views, lights = _views_and_lights(scene, fr)
+    w, h = size
+    m = scene.view_matrices((0.0, 6.0, 9.0), (0, 0, 0), 256)
+    vm = fr.FrameMatrices()
+    C.memmove(C.byref(vm), C.byref(m), C.sizeof(m))
+    vm.width, vm.height = w, h
+    vp = np.array([[w / 2, 0, 0, w / 2], [0, h / 2, 0, h / 2], [0, 0, 0.5, 0.5], [0, 0, 0, 1]], np.float32)
+    vm.viewport[:] = list(vp.reshape(-1))
+    b = Batch(r, [views[0], view(vm, (0.0, 6.0, 9.0))], lights)
+    b.render()
+    b.timings()
+    want = b.download(1, N.FR_BUF_FRAME_U8).reshape(-1)
+    n = want.size
+    pinned = torch.full((n + 8,), 77, dtype=torch.uint8).pin_memory().numpy()
+    plain = np.full(n + 9, 77, np.uint8)
+    for buf in (pinned, plain[1:]):
+        assert N.lib().fr_batch_download(b._h, 1, N.FR_BUF_FRAME_U8, buf.ctypes.data_as(C.c_void_p), n) >= 0
+        assert np.array_equal(buf[:n], want) and (buf[n:] == 77).all()
+    assert plain[0] == 77
+    b.close()

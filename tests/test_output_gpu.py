@@ -82,6 +82,48 @@ def test_random_images_match_oracle_across_segments(bpp):
                 assert _gpu_tga(img, rle) == OB.oracle_tga(img, rle), (h, w, bpp, mode, rle)
 
 
+# lengths at the ends of a lane's four positions, a word, a sub-block of 128 and its
+# look-ahead, a segment of 4096 and its look-ahead
+EDGE_LENGTHS = [1, 2, 3, 4, 5, 31, 32, 33, 127, 128, 129, 130, 255, 256, 257, 258, 383, 384, 385, 4095, 4096, 4097, 4223,
+                4224, 4225, 4353, 8191, 8192, 8193]
+
+
+@pytest.mark.parametrize("bpp", [1, 3, 4])
+def test_edge_lengths_match_oracle(bpp):
+    """Constant images, the same with one pixel changed around the last edges, and raw
+    ones, at every edge length: byte-identical to the oracle's files."""
+    rng = np.random.default_rng(40 + bpp)
+    for n in EDGE_LENGTHS:
+        images = [np.full((n, bpp), 9, np.uint8), rng.integers(0, 256, (n, bpp)).astype(np.uint8)]
+        for at in {n - 1, n // 2, max(0, n - 129), max(0, n - 128), max(0, n - 257)}:
+            one = images[0].copy()
+            one[at] = 10
+            images.append(one)
+        for i, img in enumerate(images):
+            img = img.reshape(1, n, bpp) if bpp > 1 else img.reshape(1, n)
+            assert _gpu_tga(img) == OB.oracle_tga(img), (n, bpp, i)
+
+
+@pytest.mark.parametrize("width,height", [(37, 23), (61, 67), (64, 64), (241, 17), (131, 97)])
+def test_odd_frames_match_oracle(width, height):
+    """Frames whose pixel counts leave every remainder of four and cross a segment by one,
+    so the four-pixel loads meet the image's end everywhere."""
+    _torch()
+    from forkerrenderer_gb300 import output
+
+    with tempfile.TemporaryDirectory() as d:
+        scene = Scene(scenes.stress_scene(d, width=width, height=height))
+        r = Renderer(**scenes.render_config("def_stress", shadow_size=63))
+        r.Preconfigure(scene)
+        r.Render()
+        bufs = _gpu_buffers(scene, r)
+        files, _ = output.encode_all(r)
+        for fn, key, kind in T.OUTPUTS:
+            if fn in files:
+                assert files[fn] == OB.oracle_tga(T.reference_image(key, kind, bufs)), fn
+        r.close()
+
+
 def test_large_images_round_trip_and_match_oracle():
     rng = np.random.default_rng(7)
     # a 2048 x 2048 gray image: constant background, noise blocks and stripes
