@@ -184,7 +184,7 @@ typedef struct fr_config
                                  pixels are dealt to the lanes of its setup warp        */
     int32_t medium_tri_area;  /* raster: bbox area (px, 0..2^20) up to which a triangle is
                                  drawn by one warp, or by several where there are few;
-                                 larger ones go through 16x16 tile bins                                                   */
+                                 larger ones go through 16x16 tile bins */
     int64_t bin_capacity;     /* max (triangle, tile) pairs per pass; 0 = automatic    */
     int32_t device;           /* CUDA device ordinal                                    */
     float ao_probe_threshold; /* learned AO: mean squared difference to plain SSAO on the
