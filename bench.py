@@ -182,8 +182,8 @@ def algorithmic_bytes(W: int, H: int, S: int) -> dict:
 #       python bench.py --steps 3 --warmup 3 --no-cpu-baseline --no-learned --batch-views 0
 # Both kernels are bound by instruction issue, not DRAM: the issue roofline is the
 # instruction count over the pass time against 4 warp instructions per SM per cycle.
-NCU_DRAM_TRAFFIC = {"ssao": 20_000_512 + 768, "lighting": 48_232_448 + 62_464}
-NCU_WARP_INSTRUCTIONS = {"ssao": 86_896_404, "lighting": 22_027_953}
+NCU_DRAM_TRAFFIC = {"ssao": 19_979_008, "lighting": 48_232_704 + 75_264}
+NCU_WARP_INSTRUCTIONS = {"ssao": 79_949_892, "lighting": 22_379_953}
 
 
 def replica_ms_per_frame(dev_ms: float, steps: int, ws: int, device: str) -> tuple[float, float]:
@@ -573,7 +573,7 @@ UNET_LAYERS = [(16, 16, 0), (16, 16, 0), (16, 32, 1), (32, 32, 1), (32, 64, 2), 
                (32, 32, 1), (48, 16, 0), (16, 16, 0)]
 # ncu --set full capture of the level-0 16 -> 16 convolution (k_conv3x3, 760 CTAs) in
 # the 1280x800 learned frame: sm__pipe_tensor_cycles_active.avg.pct_of_peak_sustained_active
-NCU_TENSOR_PIPE_LEVEL0 = 0.050
+NCU_TENSOR_PIPE_LEVEL0 = 0.058
 
 
 def network_flops(W: int, H: int) -> int:

@@ -4,8 +4,8 @@
 // strict-less depth test (forkergl.cpp:165-234) would leave it, but in parallel:
 // every covered fragment forms a 64-bit key (order-preserving depth bits, draw
 // index) and the per-pixel unsigned minimum survives (frx::make_key). Triangles
-// are drawn by one thread (tiny bounding boxes), one warp (medium) or through
-// 16 x 16 tile bins with one CTA per tile (large), all feeding the same keys.
+// are drawn by their setup warp (small bounding boxes), one or several warps
+// (medium) or through 16 x 16 tile bins (large), all feeding the same keys.
 // Shading then runs once per pixel on the surviving triangle, which is what the
 // reference's overwrite-on-pass leaves in its buffers.
 #include <cuda_bf16.h>

@@ -14,7 +14,7 @@ constexpr int kTile = 16;  // screen tile edge for the binned raster path
 struct RasterScratch
 {
     unsigned long long* keys;  // [W*H] visibility keys
-    frx::RTri* mediumTris;     // [cap] triangles drawn one warp each
+    frx::RTri* mediumTris;     // [cap] triangles drawn by one or several warps each
     int* mediumIdx;
     frx::RTri* largeTris;      // [cap] triangles drawn through tile bins
     int* largeIdx;
@@ -40,7 +40,7 @@ struct RasterParams
 {
     int W, H;              // raster target size
     int smallArea;         // bbox area drawn by one thread
-    int mediumArea;        // bbox area drawn by one warp (larger: tile bins)
+    int mediumArea;        // bbox area drawn by one or several warps (larger: tile bins)
 };
 
 // ---- batched multi-view rendering (fr_batch.h) -------------------------------------------
