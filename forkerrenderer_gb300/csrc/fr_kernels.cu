@@ -1974,7 +1974,8 @@ __device__ __forceinline__ int blur_sidx(int l, int i, int rowStride, int L)
 }
 
 // The same index split into a base (position s, a multiple of 32) and an offset of
-// position s + tt, so that with tt a compile-time constant the offset is one too.
+// position s + tt (tt from -4 to 36), so that with tt a compile-time constant the
+// offset is one too.
 template <bool VERT>
 __device__ __forceinline__ int blur_base(int l, int s, int rowStride, int L)
 {
@@ -1984,6 +1985,11 @@ template <bool VERT, int LV>
 __device__ __forceinline__ constexpr int blur_off(int tt)
 {
     return VERT ? (tt >> 5) * (32 * (LV + 1) + LV) + (tt & 31) * (LV + 1) : tt + (tt >> 5);
+}
+// Floats a line's chunks take: whole chunks and the four positions after them.
+__host__ __device__ __forceinline__ int blur_line_floats(int nch, int L, bool vert)
+{
+    return vert ? nch * (32 * (L + 1) + L) + 5 * (L + 1) : nch * 33 + 5;
 }
 
 // VERT: LV columns per CTA (a compile-time constant); horizontal: L rows per CTA.
@@ -2000,9 +2006,9 @@ __global__ void __launch_bounds__(512) k_blur_spec(float* a, int W, int H, int L
     const int first = blockIdx.x * L;
     const int cnt = min(L, lines - first);
     const int nch = (n + kBlurChunk - 1) / kBlurChunk;
-    const int rowStride = n + nch + 1;
+    const int rowStride = blur_line_floats(nch, L, false);
     const int items = L * nch;
-    const int smLine = VERT ? nch * (32 * (L + 1) + L) : L * rowStride;
+    const int smLine = VERT ? blur_line_floats(nch, L, true) : L * rowStride;
     float4* chk = reinterpret_cast<float4*>(sm + ((smLine + 3) & ~3));
     int* bad = reinterpret_cast<int*>(chk + items);
     auto gidx = [&](int l, int i) -> size_t {
@@ -2031,60 +2037,56 @@ __global__ void __launch_bounds__(512) k_blur_spec(float* a, int W, int H, int L
             {
                 const int i = i0 + u * rstep;
                 if (i < n) sm[blur_sidx<VERT>(l, i, rowStride, L)] = v[u];
+                if (i == n - 1)  // positions past the line read its last original
+                    for (int k = 1; k <= 4; ++k) sm[blur_sidx<VERT>(l, n - 1 + k, rowStride, L)] = v[u];
             }
         }
     __syncthreads();
 
-    // Work items: the interior chunks (those the unrolled path takes at the default
-    // warm-up, jlo <= j <= jlo + nInt - 1) on consecutive threads first, the chunks at
-    // the two ends of the lines after them, so that a warp runs one of the two paths.
-    // Vertical: the L columns of a chunk index are adjacent threads.
-    const int jlo = (kBlurWarmDefault + 4 + kBlurChunk - 1) / kBlurChunk;
-    const int nInt = warm == kBlurWarmDefault ? max(0, min(nch, (n - kBlurChunk - 5) / kBlurChunk + 1) - jlo) : 0;
-    const int nEdge = nch - nInt;
+    // Work items: horizontal a line's chunks on consecutive threads, vertical the L
+    // columns of a chunk on adjacent threads.
     const int t = threadIdx.x;
-    int l, j;
-    {
-        int q, k;
-        if (VERT)
-        {
-            l = t % L;
-            q = t / L;
-        }
-        else
-        {
-            const bool in = t < L * nInt;
-            const int e2 = in ? t : t - L * nInt;
-            const int per = in ? nInt : nEdge;
-            l = per > 0 ? e2 / per : 0;
-            q = in ? e2 % max(per, 1) : nInt + e2 % max(per, 1);
-        }
-        k = q - nInt;
-        j = q < nInt ? jlo + q : (k < jlo ? k : k + nInt);
-    }
+    const int l = VERT ? t % L : t / nch, j = VERT ? t / L : t % nch;
     const bool active = t < items && l < cnt;
     const int b = j * kBlurChunk, e = min(b + kBlurChunk, n);
     float res[kBlurChunk];
     float c1 = 0.f, c2 = 0.f, c3 = 0.f, c4 = 0.f;
-    const bool fast = active && warm == kBlurWarmDefault && b - warm >= 4 && b + kBlurChunk + 4 < n;
-    if (fast)
+    if (active && warm == kBlurWarmDefault)
     {
-        // An interior chunk at the default warm-up: its first position is a multiple
-        // of 32, so every read is a fixed offset from one base and the 96 steps unroll
-        // into straight-line code.
-        const float* base = sm + blur_base<VERT>(l, b - kBlurWarmDefault, rowStride, L);
-        float l1 = base[blur_off<VERT, LV>(-1)], l2 = base[blur_off<VERT, LV>(-2)];
-        float l3 = base[blur_off<VERT, LV>(-3)], l4 = base[blur_off<VERT, LV>(-4)];
+        // The default warm-up: up to two chunks, then the thread's own, all from one
+        // body of 32 steps with fixed offsets (a warm-up's results are overwritten). The
+        // code runs once a thread, so its length is instruction fetches: 96 steps in a
+        // line, and a second form for the ends of the lines, took 15.2 us a pass.
+        const int s0 = max(b - kBlurWarmDefault, 0);
+        const float* base = sm + blur_base<VERT>(l, s0, rowStride, L);
+        constexpr int kStride = VERT ? 32 * (LV + 1) + LV : 33;  // to the next chunk
         float x0 = base[blur_off<VERT, LV>(0)], x1 = base[blur_off<VERT, LV>(1)], x2 = base[blur_off<VERT, LV>(2)];
         float x3 = base[blur_off<VERT, LV>(3)], x4 = base[blur_off<VERT, LV>(4)];
-#pragma unroll
-        for (int u = 0; u < kBlurWarmDefault + kBlurChunk; ++u)
+        // at the line's start position 0's left reads are itself, original, and position
+        // 1's are all position 0's result: the true state
+        bool start = s0 == 0;
+        float l1 = x0, l2 = x0, l3 = x0, l4 = x0;
+        if (!start)
         {
-            if (u == kBlurWarmDefault) c1 = l1, c2 = l2, c3 = l3, c4 = l4;
-            const float r = blur_step(x0, x1, x2, x3, x4, l1, l2, l3, l4, w);
-            if (u >= kBlurWarmDefault) res[u - kBlurWarmDefault] = r;
-            l4 = l3, l3 = l2, l2 = l1, l1 = r;
-            x0 = x1, x1 = x2, x2 = x3, x3 = x4, x4 = base[blur_off<VERT, LV>(u + 5)];
+            l1 = base[blur_off<VERT, LV>(-1)], l2 = base[blur_off<VERT, LV>(-2)];
+            l3 = base[blur_off<VERT, LV>(-3)], l4 = base[blur_off<VERT, LV>(-4)];
+        }
+#pragma unroll 1
+        for (int s = s0; s <= b; s += kBlurChunk)
+        {
+            c1 = l1, c2 = l2, c3 = l3, c4 = l4;
+#pragma unroll
+            for (int u = 0; u < kBlurChunk; ++u)
+            {
+                const float r = blur_step(x0, x1, x2, x3, x4, l1, l2, l3, l4, w);
+                res[u] = r;
+                l4 = l3, l3 = l2, l2 = l1, l1 = r;
+                if (u == 0 && start) l2 = l3 = l4 = r;
+                x0 = x1, x1 = x2, x2 = x3, x3 = x4;
+                x4 = base[blur_off<VERT, LV>(u + 5)];
+            }
+            start = false;
+            base += kStride;
         }
     }
     else if (active)
@@ -2156,10 +2158,7 @@ __global__ void __launch_bounds__(512) k_blur_spec(float* a, int W, int H, int L
             for (int c = 1; c < nch; ++c)
             {
                 const int cb = c * kBlurChunk, ce = min(cb + kBlurChunk, n);
-                // the work item of chunk c of this line (the inverse of the mapping above)
-                const bool inner = c >= jlo && c < jlo + nInt;
-                const int qq = inner ? c - jlo : nInt + (c < jlo ? c : c - nInt);
-                const int it = VERT ? qq * L + l : (inner ? l * nInt + qq : L * nInt + l * nEdge + (qq - nInt));
+                const int it = VERT ? c * L + l : l * nch + c;  // the work item of chunk c of this line
                 float l1 = S(cb - 1), l2 = S(cb - 2), l3 = S(cb - 3), l4 = S(cb - 4);
                 bool ok;
                 if (prevRedone)
@@ -2195,7 +2194,7 @@ __global__ void __launch_bounds__(512) k_blur_spec(float* a, int W, int H, int L
 size_t blur_spec_smem(int n, int L, bool vert)
 {
     const int nch = (n + kBlurChunk - 1) / kBlurChunk;
-    const size_t line = vert ? (size_t)nch * (32 * (L + 1) + L) : (size_t)L * (n + nch + 1);
+    const size_t line = (size_t)blur_line_floats(nch, L, vert) * (vert ? 1 : L);
     const size_t items = (size_t)L * nch;
     if (items > 512) return 0;
     const size_t bytes = ((line + 3) & ~(size_t)3) * sizeof(float) + items * (sizeof(float4) + sizeof(int));
