@@ -312,3 +312,39 @@ def test_shadow_pass_after_another_light_matches_oracle():
         assert np.array_equal(r.shadow_map().view(np.uint32), want["shadow"].view(np.uint32))
         assert np.array_equal(r.depth().view(np.uint32), want["depth"].view(np.uint32))
     r.close()
+
+
+def _inplace_blur(x):
+    """One in-place pass along the rows in the reference's order, in float32."""
+    w = np.array([0.227027, 0.1945946, 0.1216216, 0.054054, 0.016216], np.float32)
+    x = x.copy()
+    n = x.shape[1]
+    for i in range(n):
+        r = x[:, i] * w[0]
+        for k in range(1, 5):
+            r = r + x[:, min(i + k, n - 1)] * w[k]
+            r = r + x[:, max(i - k, 0)] * w[k]
+        x[:, i] = r
+    return x
+
+
+@pytest.mark.parametrize("width,height", [(1, 33), (4, 31), (5, 32), (31, 5), (32, 36), (33, 64), (36, 65), (37, 96),
+                                          (64, 97), (65, 100), (97, 128), (129, 132), (133, 1)])
+def test_inplace_blur_at_chunk_edges(width, height):
+    """Lines that end at, just before and just after a chunk of 32 positions and its four
+    look-ahead positions, with one to five chunks: the sequential recurrence's bits."""
+    import tempfile
+
+    import forkerrenderer_gb300._native as N
+
+    with tempfile.TemporaryDirectory() as d:
+        scene = Scene(scenes.stress_scene(d, width=width, height=height))
+        out = []
+        for mode in (N.FR_BLUR_NONE, N.FR_BLUR_REFERENCE):
+            r = Renderer(**scenes.render_config("def_stress", shadow_size=64, blur_mode=mode))
+            r.Preconfigure(scene)
+            r.Render()
+            out.append(r.ambient_occlusion().reshape(height, width).copy())
+            r.close()
+    want = _inplace_blur(_inplace_blur(out[0]).T).T
+    np.testing.assert_array_equal(out[1].view(np.uint32), np.ascontiguousarray(want).view(np.uint32))
