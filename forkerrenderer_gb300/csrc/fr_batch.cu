@@ -9,14 +9,13 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "fr_aonet.h"
 #include "fr_aonet_internal.h"
 #include "fr_batch.h"
 #include "fr_context_internal.h"
+#include "fr_hostcopy.h"
 #include "fr_hostmath.h"
 #include "fr_kernels.cuh"
 
@@ -47,32 +46,6 @@ struct Alloc
         for (void* p : ptrs) cudaFree(p);
     }
 };
-
-// dst = src, large copies by up to four threads (a fresh destination's page faults are
-// most of its time).
-void copy_bytes(unsigned char* dst, const unsigned char* src, size_t n)
-{
-    const size_t parts = std::min<size_t>(4, n >> 20);
-    if (parts < 2)
-    {
-        std::memcpy(dst, src, n);
-        return;
-    }
-    std::vector<std::thread> ts;
-    const size_t step = ((n / parts) + 65535) & ~(size_t)65535;
-    size_t at = step;
-    try
-    {
-        for (; at < n; at += step)
-            ts.emplace_back([=] { std::memcpy(dst + at, src + at, std::min(step, n - at)); });
-    }
-    catch (const std::system_error&)  // no thread to be had: the rest here
-    {
-        std::memcpy(dst + at, src + at, n - at);
-    }
-    std::memcpy(dst, src, std::min(step, n));
-    for (auto& t : ts) t.join();
-}
 
 int tiles_of(int w, int h, int t) { return ((w + t - 1) / t) * ((h + t - 1) / t); }
 
@@ -699,7 +672,7 @@ int64_t fr_batch_download(fr_batch* b, int32_t view, int32_t id, void* dst, size
         frk::launch_pack_rgb(rgba, b->rgbDev, n, st);
         B_CUDA(b, cudaGetLastError());
         B_CUDA(b, cudaStreamSynchronize(st));
-        copy_bytes(static_cast<unsigned char*>(dst), b->rgb, need);
+        fr::copy_bytes(static_cast<unsigned char*>(dst), b->rgb, need);
         return FR_OK;
     }
     B_CUDA(b, cudaGetLastError());
