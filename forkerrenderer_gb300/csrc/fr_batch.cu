@@ -8,6 +8,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -120,7 +122,7 @@ struct fr_batch
     frk::BatchLight* dLights = nullptr;
     int* dQueues = nullptr;
     float4* ssaoTblGlobal = nullptr;
-    uint8_t *rgb = nullptr, *rgbDev = nullptr;  // pinned: a packed 8-bit frame of any view, for downloads
+    uint8_t *rgb = nullptr, *rgbDev = nullptr;  // pinned: a packed 8-bit frame of any view (pinned_frame)
 
     fr_batch_tuning tuning{16, 64, 2};
     cudaStream_t br[kBranches] = {};
@@ -301,6 +303,30 @@ int capture(fr_batch* b)
     return FR_OK;
 }
 
+// The batch's pinned buffer for packed frames, allocated by the first download that
+// needs it (a batch whose frames are never read as bytes takes none). False where no
+// pinned memory is to be had.
+bool pinned_frame(fr_batch* b)
+{
+    if (b->rgb) return true;
+    size_t most = 0;
+    for (auto& X : b->views) most = std::max(most, (size_t)X.F.W * X.F.H);
+    void *host = nullptr, *dev = nullptr;
+    if (cudaHostAlloc(&host, 3 * most, cudaHostAllocMapped) != cudaSuccess)
+    {
+        cudaGetLastError();  // this call's own error
+        return false;
+    }
+    if (cudaHostGetDevicePointer(&dev, host, 0) != cudaSuccess)
+    {
+        cudaGetLastError();
+        cudaFreeHost(host);
+        return false;
+    }
+    b->rgb = static_cast<uint8_t*>(host), b->rgbDev = static_cast<uint8_t*>(dev);
+    return true;
+}
+
 bool valid_tuning(const fr_batch_tuning& t)
 {
     return (t.light_tile == 8 || t.light_tile == 16 || t.light_tile == 32) &&
@@ -476,14 +502,6 @@ fr_batch* fr_batch_create(fr_ctx* ctx, const fr_view_desc* views, int32_t n_view
     b->dShadeStart = A.get<int>(n_views + 1);
     b->dLights = A.get<frk::BatchLight>(bl.size());
     b->dQueues = A.get<int>(2);
-    size_t maxPix = 0;
-    for (auto& X : b->views) maxPix = std::max(maxPix, (size_t)X.F.W * X.F.H);
-    if (cudaHostAlloc(reinterpret_cast<void**>(&b->rgb), 3 * maxPix, cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->rgbDev), b->rgb, 0) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return fr_batch_destroy(b), bail("out of pinned host memory");
-    }
     if (A.err != cudaSuccess) return fr_batch_destroy(b), bail("out of device memory");
     cudaMemcpy(b->dRaster, vr.data(), sizeof(frk::ViewRaster) * vr.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(b->dRasterStart, rstart.data(), sizeof(int) * rstart.size(), cudaMemcpyHostToDevice);
@@ -662,21 +680,31 @@ int64_t fr_batch_download(fr_batch* b, int32_t view, int32_t id, void* dst, size
     // costs milliseconds a pass when the caller's buffers come fresh from the system.)
     const int n = (int)(need / 3);
     cudaStream_t st = b->ctx->stream;
+    unsigned char* out = static_cast<unsigned char*>(dst);
     cudaPointerAttributes pa{};
     const cudaError_t ae = cudaPointerGetAttributes(&pa, dst);
     if (ae != cudaSuccess) cudaGetLastError();  // this call's own error: copy below
-    if (ae == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer && pa.device == b->ctx->cfg.device)
-        frk::launch_pack_rgb(rgba, static_cast<uint8_t*>(pa.devicePointer), n, st);
-    else
+    const bool direct =
+        ae == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer && pa.device == b->ctx->cfg.device;
+    if (direct || pinned_frame(b))
     {
-        frk::launch_pack_rgb(rgba, b->rgbDev, n, st);
+        frk::launch_pack_rgb(rgba, direct ? static_cast<uint8_t*>(pa.devicePointer) : b->rgbDev, n, st);
         B_CUDA(b, cudaGetLastError());
         B_CUDA(b, cudaStreamSynchronize(st));
-        fr::copy_bytes(static_cast<unsigned char*>(dst), b->rgb, need);
+        if (!direct) fr::copy_bytes(out, b->rgb, need);
         return FR_OK;
     }
-    B_CUDA(b, cudaGetLastError());
+    // no pinned memory to be had: packed r | g << 8 | b << 16 -> RGB8 on the host
     B_CUDA(b, cudaStreamSynchronize(st));
+    const std::unique_ptr<unsigned[]> tmp(new (std::nothrow) unsigned[n]);
+    if (!tmp) return bfail(b, FR_ERR_OOM, "out of host memory");
+    B_CUDA(b, cudaMemcpy(tmp.get(), rgba, sizeof(unsigned) * n, cudaMemcpyDeviceToHost));
+    for (int i = 0; i < n; ++i)
+    {
+        out[3 * (size_t)i] = tmp[i] & 0xff;
+        out[3 * (size_t)i + 1] = (tmp[i] >> 8) & 0xff;
+        out[3 * (size_t)i + 2] = (tmp[i] >> 16) & 0xff;
+    }
     return FR_OK;
 }
 

@@ -59,7 +59,9 @@ typedef struct fr_batch_tuning
 typedef struct fr_batch fr_batch;
 
 /* The context's scene and configuration (shadow mode, sample counts, SSAO
- * parameters, blur) apply to every view. At most 4 lights. */
+ * parameters, blur) apply to every view. At most 4 lights. Device memory, beside the
+ * maps and G-buffers: raster scratch of every view and light as a context's pass has it
+ * (for a light with 32 bytes a scene triangle for its shadow map's resolve). */
 fr_batch* fr_batch_create(fr_ctx* ctx, const fr_view_desc* views, int32_t n_views, const fr_light_desc* lights,
                           int32_t n_lights, char* err, size_t errlen);
 void fr_batch_destroy(fr_batch* batch);
@@ -87,7 +89,9 @@ int fr_batch_work(const fr_batch* batch, int64_t* triangles, int64_t* pixels, in
 
 /* Reads one buffer of view `view` (FR_BUF_FRAME_U8, FR_BUF_DEPTH, FR_BUF_AO) or,
  * with view = -1 - k, light k's shadow map (FR_BUF_SHADOW). Same layouts and
- * return convention as fr_download. */
+ * return convention as fr_download. The first FR_BUF_FRAME_U8 download into memory the
+ * device does not write itself allocates 3 bytes of pinned host memory per pixel of the
+ * largest view; without any the download is slower but succeeds. */
 int64_t fr_batch_download(fr_batch* batch, int32_t view, int32_t buffer_id, void* dst, size_t bytes);
 
 #ifdef __cplusplus
