@@ -674,21 +674,17 @@ int64_t fr_batch_download(fr_batch* b, int32_t view, int32_t id, void* dst, size
         return FR_OK;
     }
     // Packed to R, G, B bytes by the device, into the caller's pinned memory where the
-    // device can address it, else into the batch's pinned buffer and copied from there. (A
+    // device can write all of it, else into the batch's pinned buffer and copied from there. (A
     // 4-byte copy and a scalar loop on the host took as long as rendering the views; the
     // device writing pageable memory itself is faster while its pages stay mapped, but
     // costs milliseconds a pass when the caller's buffers come fresh from the system.)
     const int n = (int)(need / 3);
     cudaStream_t st = b->ctx->stream;
     unsigned char* out = static_cast<unsigned char*>(dst);
-    cudaPointerAttributes pa{};
-    const cudaError_t ae = cudaPointerGetAttributes(&pa, dst);
-    if (ae != cudaSuccess) cudaGetLastError();  // this call's own error: copy below
-    const bool direct =
-        ae == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer && pa.device == b->ctx->cfg.device;
+    void* direct = frctx_pinned_destination(b->ctx->cfg.device, dst, need);
     if (direct || pinned_frame(b))
     {
-        frk::launch_pack_rgb(rgba, direct ? static_cast<uint8_t*>(pa.devicePointer) : b->rgbDev, n, st);
+        frk::launch_pack_rgb(rgba, direct ? static_cast<uint8_t*>(direct) : b->rgbDev, n, st);
         B_CUDA(b, cudaGetLastError());
         B_CUDA(b, cudaStreamSynchronize(st));
         if (!direct) fr::copy_bytes(out, b->rgb, need);

@@ -1,11 +1,15 @@
 // C ABI of include/forkerrenderer.h: render context, scene upload, the frame's
 // pass sequence (Render::Render, src/render.cpp:40-58) and read-back in the
 // reference's buffer layouts.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -979,15 +983,11 @@ int64_t fr_download(fr_ctx* ctx, int32_t id, void* dst, size_t bytes)
     {
         // pinned host memory the device can address: the packing kernel writes it
         // directly, queued behind the frame's last event, and one wait covers both
-        cudaPointerAttributes pa{};
-        const cudaError_t ae = cudaPointerGetAttributes(&pa, dst);
-        if (ae != cudaSuccess) cudaGetLastError();  // this call's own error: take the copy below
-        if (ae == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer && pa.device == ctx->cfg.device)
+        if (void* out = frctx_pinned_destination(ctx->cfg.device, dst, need))
         {
             const size_t n = id == FR_BUF_FRAME_U8 ? P : (size_t)(ctx->W / k) * (ctx->H / k);
             if (ctx->statusPending) FR_CUDA(cudaStreamWaitEvent(st, ctx->ev[6], 0));
-            frk::launch_pack_rgb(id == FR_BUF_FRAME_U8 ? ctx->frame8 : ctx->ssaa,
-                                 static_cast<uint8_t*>(pa.devicePointer), (int)n, st);
+            frk::launch_pack_rgb(id == FR_BUF_FRAME_U8 ? ctx->frame8 : ctx->ssaa, static_cast<uint8_t*>(out), (int)n, st);
             FR_CUDA(cudaGetLastError());
             FR_CUDA(cudaStreamSynchronize(st));
             return check_status(ctx);
@@ -1022,8 +1022,8 @@ int64_t fr_download(fr_ctx* ctx, int32_t id, void* dst, size_t bytes)
         case FR_BUF_FRAME_U8:
         case FR_BUF_SSAA_U8:
         {
-            // packed to R, G, B on the device, then one copy into dst (pinned,
-            // device-addressable destinations took the direct path above)
+            // packed to R, G, B on the device, then one copy into dst (destinations
+            // that the device can write took the direct path above)
             const size_t n = id == FR_BUF_FRAME_U8 ? P : (size_t)(ctx->W / k) * (ctx->H / k);
             if (ctx->rgbCap < 3 * n)
             {
@@ -1033,7 +1033,20 @@ int64_t fr_download(fr_ctx* ctx, int32_t id, void* dst, size_t bytes)
                 ctx->rgbCap = 3 * n;
             }
             frk::launch_pack_rgb(id == FR_BUF_FRAME_U8 ? ctx->frame8 : ctx->ssaa, ctx->rgbBuf, (int)n, st);
-            rc = d2h(ctx->rgbBuf, need);
+            const cudaError_t ce = cudaMemcpyAsync(dst, ctx->rgbBuf, need, cudaMemcpyDeviceToHost, st);
+            if (ce == cudaErrorInvalidValue)
+            {
+                // a destination pinned in part is none to CUDA's copies: by way of the heap
+                cudaGetLastError();
+                const std::unique_ptr<unsigned char[]> host(new (std::nothrow) unsigned char[need]);
+                if (!host) return fail(ctx, FR_ERR_OOM, "out of host memory");
+                FR_CUDA(cudaMemcpyAsync(host.get(), ctx->rgbBuf, need, cudaMemcpyDeviceToHost, st));
+                FR_CUDA(cudaStreamSynchronize(st));
+                std::memcpy(dst, host.get(), need);
+                break;
+            }
+            FR_CUDA(ce);
+            FR_CUDA(cudaStreamSynchronize(st));
             break;
         }
         default:
@@ -1096,6 +1109,40 @@ int fr_ao_probe_result(fr_ctx* ctx, float* mean_sq_diff, int32_t* fell_back)
 }
 
 }  // extern "C"
+
+// ---- where the device may write host memory itself (fr_context_internal.h) ----------
+
+// dst alone says nothing about its last byte: a buffer may be registered in part, and two
+// registrations have adjacent device addresses with or without a hole between them. So
+// the range that dst belongs to decides, as the driver keeps it. cuPointerGetAttributes
+// leaves a value 0 that it does not have (a pageable dst has none).
+void* frctx_pinned_destination(int32_t device, void* dst, size_t bytes)
+{
+    using Fn = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static std::once_flag once;
+    static Fn fn = nullptr;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<Fn>(p);
+    });
+    if (!fn || !dst || bytes == 0) return nullptr;
+    unsigned long long type = 0, dev = 0, managed = 0, ordinal = ~0ull, start = 0, size = 0, access = 0;
+    CUpointer_attribute want[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_IS_MANAGED,       CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                  CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void* got[] = {&type, &dev, &managed, &ordinal, &start, &size, &access};
+    if (fn(7, want, got, reinterpret_cast<CUdeviceptr>(dst)) != CUDA_SUCCESS) return nullptr;
+    if ((type & 0xffffffffu) != CU_MEMORYTYPE_HOST || !dev || (managed & 0xffu) ||
+        (ordinal & 0xffffffffu) != static_cast<unsigned>(device) ||
+        (access & 0xffffffffu) != CU_MEM_ACCESS_FLAGS_PROT_READWRITE)
+        return nullptr;
+    if (dev < start || dev - start >= size || size - (dev - start) < bytes) return nullptr;
+    return reinterpret_cast<void*>(dev);
+}
 
 // ---- accessors for the learned-AO trainer (fr_context_internal.h) -------------------
 

@@ -123,6 +123,9 @@ void frctx_refresh_background(frd::FrameConst& F);
 float* frctx_ao(fr_ctx* ctx);           // AO plane of the last SSAO pass, W * H floats
 const float* frctx_depth(fr_ctx* ctx);  // depth buffer, FLT_MAX where no triangle
 cudaStream_t frctx_stream(fr_ctx* ctx);
+// The device's address of dst where the device can write all of [dst, dst + bytes): pinned
+// host memory of one allocation or registration, of this device. Else null.
+extern "C" void* frctx_pinned_destination(int32_t device, void* dst, size_t bytes);
 void frout_free(fr_ctx* ctx);  // releases ctx->output
 void frctx_size(const fr_ctx* ctx, int* W, int* H);
 // Model::generateTangents on the device into ctx->S.tan for the models flagged in
