@@ -642,6 +642,16 @@ int ensure_bwd(fr_aonet* n, long long pix)
         NET_CUDA(n, cudaMalloc(&n->headPart, sizeof(float) * kHeadSums * hb));
         n->headPartCap = hb;
     }
+    if (!n->partial)
+    {
+        // the weight gradients' chains of any shape (at most one per SM and layer: 73 MB),
+        // once: a step that was captured keeps its address, and one of another shape with
+        // no more pixels allocates nothing
+        size_t floats = 0;
+        for (const LayerSpec& s : kLayers) floats += n->numSMs * wgrad_partial_floats(s.c0 + s.c1, s.cout);
+        NET_CUDA(n, cudaMalloc(&n->partial, sizeof(float) * floats));
+        n->partialCap = floats;
+    }
     n->capBwd = pix;
     return FR_OK;
 }
@@ -838,13 +848,7 @@ int wgrad_all(fr_aonet* n, const WgradLayer* layers, int headBlocks, float invN,
                                  n->grads + n->paramOff[L] + w_count(L)};
         rblocks += blocks_for(static_cast<long long>(wgrad_partial_floats(cin, w.cout)), kReduceThreads);
     }
-    if (need > n->partialCap)
-    {
-        cudaFree(n->partial);  // waits for earlier steps
-        n->partial = nullptr, n->partialCap = 0;
-        NET_CUDA(n, cudaMalloc(&n->partial, sizeof(float) * need));
-        n->partialCap = need;
-    }
+    if (need > n->partialCap) return net_fail(n, FR_ERR_INVALID, "wgrad partial buffer too small");
     for (int L = 0; L < kNumLayers; ++L) R.layer[L].partial = U.layer[L].partial = n->partial + at[L];
     R.headPart = n->headPart, R.headBlocks = headBlocks;
     R.gradsHead = n->grads + n->paramOff[kNumLayers];

@@ -355,3 +355,46 @@ def test_fused_forward_grid_barrier_times_out_and_recovers():
     net.check()
     r.close()
     net.close()
+
+
+def test_captured_backward_at_another_shape():
+    """A backward pass captured at a shape with fewer pixels but more tiles a level than
+    any step before it (many small images: 60 chains of level 2 where there were 4), and
+    replayed after eager steps of shapes with more tiles still: the eager gradients' bits."""
+    _need_gpu()
+    import torch
+    from forkerrenderer_gb300 import _native as N
+    from forkerrenderer_gb300.aonet import AONet
+
+    rng = np.random.default_rng(5)
+    dev = {}
+    for shape in [(4, 128, 128), (60, 32, 32), (64, 32, 32)]:
+        bits, _ = _batch(rng, *shape)
+        dev[shape] = (_dev(bits.view(np.int16)), _dev(rng.uniform(0.1, 0.95, shape).astype(np.float32)))
+
+    def backward(net, shape, stream):
+        x, label = dev[shape]
+        assert N.lib().fr_aonet_backward(net.handle, x.data_ptr(), label.data_ptr(), *shape, None, stream) == N.FR_OK
+
+    eager = AONet(0, seed=9)
+    backward(eager, (60, 32, 32), 0)
+    torch.cuda.synchronize()
+    want = eager.get_grads()
+    net = AONet(0, seed=9)
+    s = torch.cuda.Stream()
+    backward(net, (4, 128, 128), s.cuda_stream)
+    s.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        backward(net, (60, 32, 32), s.cuda_stream)
+    for other in [None, (64, 32, 32), (4, 128, 128)]:
+        if other:
+            backward(net, other, s.cuda_stream)
+            s.synchronize()
+        with torch.cuda.stream(s):
+            g.replay()
+        s.synchronize()
+        assert np.array_equal(net.get_grads().view(np.uint32), want.view(np.uint32)), other
+    net.check(s)
+    net.close()
+    eager.close()
