@@ -19,6 +19,7 @@
 #include "fr_aonet_conv.cuh"
 #include "fr_aonet_ew.cuh"
 #include "fr_aonet_internal.h"
+#include "fr_sum.cuh"
 
 namespace fra
 {
@@ -282,11 +283,7 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_bwd(const float* __restri
 
 // The gradient from its partial sums, one launch: the first kHeadSums CTAs sum the
 // head's per-block partials (loss -> out_loss, head gradients), the others the
-// layers' weight-gradient chains. FP64 is slow on this GPU (a convert and an add per
-// partial made this kernel 91 us of a 16 x 256 x 256 step), so a weight's sum is
-// compensated FP32: every add's exact rounding error (Knuth's TwoSum) goes into a
-// second float, and the pair rounds to the result, within 2^-40 of the FP64 sum of
-// these at most 152 terms before that rounding.
+// layers' weight-gradient chains (frx::sum_terms).
 constexpr int kReduceThreads = 256;
 
 struct ReduceLayer
@@ -327,16 +324,6 @@ __device__ __forceinline__ void reduce_head(const ReduceArgs& R, int k)
         R.gradsHead[k - 1] = static_cast<float>(sum[0]);  // w[4][16], then b[4]
 }
 
-// (hi, lo) += x: hi the rounded running sum, lo the sum of its rounding errors.
-__device__ __forceinline__ void two_sum_add(float& hi, float& lo, float x)
-{
-    const float s = __fadd_rn(hi, x);
-    const float b = __fsub_rn(s, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b));
-    hi = s;
-    lo = __fadd_rn(lo, e);
-}
-
 // One thread per (kx, co, ky, ci) of a layer, ci fastest as in the partials (a warp
 // reads whole lines of every chain; the scattered 4-byte writes are a single pass
 // over 120 thousand gradients), the last of a row for the bias.
@@ -353,28 +340,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_grad_reduce(const __grid_con
     const int row = i % rows, q = i / rows;
     const int co = q % a.cout, kx = q / a.cout;
     if (row == 3 * a.cin && kx != 1) return;
-    const float* src = a.partial + i;
-    const size_t stride = static_cast<size_t>(n);
-    // chain c into sum c mod 4, combined pairwise at the end; 32 loads in flight
-    constexpr int kLoads = 32;
-    float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < a.chains; c += kLoads)
-    {
-        float v[kLoads];
-#pragma unroll
-        for (int j = 0; j < kLoads; ++j) v[j] = c + j < a.chains ? src[(c + j) * stride] : 0.f;
-#pragma unroll
-        for (int j = 0; j < kLoads; ++j) two_sum_add(hi[j & 3], lo[j & 3], v[j]);  // adding 0 is exact
-    }
-#pragma unroll
-    for (int j = 2; j > 0; j >>= 1)
-#pragma unroll
-        for (int k = 0; k < j; ++k)
-        {
-            two_sum_add(hi[k], lo[k], hi[k + j]);
-            two_sum_add(hi[k], lo[k], lo[k + j]);
-        }
-    const float total = __fadd_rn(hi[0], lo[0]);
+    const float total = frx::sum_terms(a.partial + i, static_cast<size_t>(n), a.chains);
     if (row < 3 * a.cin)
         a.dW[(co * a.cin + row % a.cin) * 9 + row / a.cin * 3 + kx] = total;
     else
