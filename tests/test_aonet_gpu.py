@@ -398,3 +398,32 @@ def test_captured_backward_at_another_shape():
     net.check(s)
     net.close()
     eager.close()
+
+
+def test_weight_gradients_over_chains_of_several_tiles():
+    """512 tiles of level 0 in chains of three and four. Against the oracle as in the other
+    gradient tests, and against the mean of the images' own gradients (the scale is a power
+    of two, so only FP32 accumulation differs): a chain's accumulator takes 8 adds a tile,
+    at most 32, each off by 2^-23 of what it holds, so 3.8e-6 of the sums of magnitudes;
+    1e-4 of the gradient leaves a factor 26 for cancellation."""
+    _need_gpu()
+    import aonet_ref as R
+    from forkerrenderer_gb300.aonet import AONet
+
+    B, H, W = 4, 256, 256
+    rng = np.random.default_rng(77)
+    net = AONet(0, seed=11)
+    bits, x4 = _batch(rng, B, H, W)
+    label = rng.uniform(0.1, 0.95, (B, H, W)).astype(np.float32)
+    net.backward(_dev(bits.view(np.int16)), _dev(label), B, H, W)
+    g = net.get_grads().astype(np.float64)
+    ref_net = R.Net(net.get_params())
+    ref_net.forward(x4)
+    _, gref = ref_net.backward(label)
+    mean = np.zeros(g.size)
+    for i in range(B):
+        net.backward(_dev(bits[i:i + 1].view(np.int16)), _dev(label[i:i + 1]), 1, H, W)
+        mean += net.get_grads().astype(np.float64) / B
+    for name, sl in _layer_slices():
+        assert np.linalg.norm(g[sl] - gref[sl]) < 3e-2 * max(np.linalg.norm(gref[sl]), 1e-12), name
+        assert np.linalg.norm(g[sl] - mean[sl]) < 1e-4 * max(np.linalg.norm(mean[sl]), 1e-12), name

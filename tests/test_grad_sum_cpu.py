@@ -59,3 +59,22 @@ def test_infinities_and_sums_beyond_the_range_of_fp32(sum_terms, n):
                     if 0 <= at + i * gap < n:
                         v[at + i * gap] = x
                 _check(sum_terms, v)
+
+
+@pytest.mark.parametrize("n", [2, 33, 128, 152])
+@pytest.mark.parametrize("spread", [0, 8, 20, 60])
+def test_terms_that_cancel(sum_terms, n, spread):
+    """Random terms over 2^spread whose last one cancels nearly all of the rest, sums of
+    signed pairs in a shuffled order, and long runs of one sign: no further off than FP64."""
+    rng = np.random.default_rng(100 * n + spread)
+    for _ in range(300):
+        v = (rng.standard_normal(n) * 2.0 ** rng.uniform(-spread, 0, n)).astype(np.float32)
+        _check(sum_terms, v)
+        _check(sum_terms, np.abs(v))
+        w = v.copy()
+        w[-1] = -math.fsum(v[:-1].astype(np.float64))
+        _check(sum_terms, w)
+        k = n // 2
+        w = v.copy()
+        w[k:2 * k] = -w[:k] * np.float32(1 + 2.0 ** -23)
+        _check(sum_terms, rng.permutation(w))
