@@ -22,9 +22,7 @@ namespace fra
 constexpr int kTileW = 8;
 constexpr int kTileH = 16;
 constexpr int kHaloW = kTileW + 2;
-constexpr int kHaloH = kTileH + 2;
-constexpr int kRowBytes = kHaloW * 16;               // 160
-constexpr int kPlaneBytes = kHaloW * kHaloH * 16;    // 2880
+constexpr int kRowBytes = kHaloW * 16;  // 160
 constexpr int kMaxStages = 4;
 
 struct ConvArgs

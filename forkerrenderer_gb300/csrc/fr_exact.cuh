@@ -422,14 +422,15 @@ FR_HD bool ref_edge_neg_zero32(int a1, int b1, int a2, int b2)
 
 FR_HD float signed_zero(bool negative) { return negative ? -0.f : 0.f; }
 
-// Cheap conservative pre-test for a fast-class triangle: false only if the
-// pixel is certainly rejected (a strict sign violation of an exact edge value);
-// pixels with c == 0 pass and are decided by bary().
 FR_HD bool small_pixel(int px, int py)
 {
     return px >= -kSmallLimit && px <= kSmallLimit && py >= -kSmallLimit && py <= kSmallLimit;
 }
 
+// Cheap conservative pre-test for a fast-class triangle: false only if the
+// pixel is certainly rejected (a strict sign violation of an exact edge value);
+// pixels with c == 0 pass and are decided by bary(). (This and pretest_kind: for
+// the host check of the exact forms; the raster kernels start from SmallEdges.)
 FR_HD bool maybe_covered(const RTri& t, int px, int py)
 {
     if (t.small && small_pixel(px, py))
@@ -449,9 +450,9 @@ FR_HD bool maybe_covered(const RTri& t, int px, int py)
     return c == 0 || ((c > 0) == pos);
 }
 
-// maybe_covered for the setup kernel's queues: 0 = certainly rejected, 1 =
-// maybe covered, 2 = maybe covered on edge BC (c == 0, small path): bary() of
-// kind 2 pixels takes the on-edge weight, of kind 1 pixels never does.
+// maybe_covered by the weight path: 0 = certainly rejected, 1 = maybe covered,
+// 2 = maybe covered on edge BC (c == 0, small path): bary() of kind 2 pixels
+// takes the on-edge weight, of kind 1 pixels never does.
 FR_HD int pretest_kind(const RTri& t, int px, int py)
 {
     if (t.small && small_pixel(px, py))
@@ -465,15 +466,13 @@ FR_HD int pretest_kind(const RTri& t, int px, int py)
     return maybe_covered(t, px, py) ? 1 : 0;
 }
 
-// Exact coverage + barycentric for one pixel, bit-identical to Barycentric()
-// including the sign of zero weights. Returns false if the reference rejects
-// the pixel.
 // bary() of a fast-class triangle (|bz| < 2^24) with every coordinate and the
 // pixel within +-kSmallLimit: the same values, with every edge value and test in
 // int32 (the common case of the raster and resolve kernels).
 // kOnly: 0 = any pixel, 1 = pixels off edge BC (c != 0), 2 = pixels on it (c == 0);
 // a pixel of the other kind is handed to the general form (it does not happen
 // when the kind comes from pretest_kind), so each form carries one weight path.
+// The kernels use 0; the host check runs all three.
 // kZeroSigns: reproduce the sign of zero weights too. Every consumer of the
 // weights (Dot from 0.f for depth and varyings, sign tests for coverage) gives the
 // same bits whatever the sign of a zero weight: a sum that starts at +0 stays +0
@@ -522,6 +521,9 @@ FR_HD bool bary_small(const RTri& t, int px, int py, float& b0, float& b1, float
     return true;
 }
 
+// Exact coverage + barycentric for one pixel, bit-identical to Barycentric()
+// including (kZeroSigns) the sign of zero weights. Returns false if the reference
+// rejects the pixel.
 template <int kOnly = 0, bool kZeroSigns = true>
 FR_HD bool bary(const RTri& t, int px, int py, float& b0, float& b1, float& b2)
 {
@@ -609,7 +611,8 @@ FR_HD int affine_wrapped(int a, int bx, int by, int lx, int ly)
 }
 
 // Row floor(l / w) of pixel l of a box of width w: rw = RN(1 / w), l < 2^22. (l + 0.5) / w
-// is at least 0.5 / w from an integer, the rounded product off by less than l 2^-22 / w.
+// is at least 0.5 / w from an integer, the rounded product off by less than
+// (l + 0.5)(2^-23 + 2^-48) / w.
 FR_HD int box_row(int l, float rw)
 {
 #ifdef __CUDA_ARCH__

@@ -78,12 +78,11 @@ __device__ __forceinline__ void bbox(const frx::RTri& r, int W, int H, int& x0, 
     y1 = clampi(max(r.y[0], max(r.y[1], r.y[2])), 0, H - 1);
 }
 
-template <int kOnly = 0>
 __device__ __forceinline__ void fragment_key(const frx::RTri& r, int t, int px, int py, int W,
                                              unsigned long long* __restrict__ keys)
 {
     float b0, b1, b2;
-    if (!frx::bary<kOnly, false>(r, px, py, b0, b1, b2)) return;
+    if (!frx::bary<0, false>(r, px, py, b0, b1, b2)) return;
     float d = frx::depth_of(r, b0, b1, b2);
     if (!frx::depth_passes_clear(d)) return;
     atomicMin(keys + (size_t)py * W + px, frx::make_key(d, (unsigned)t));  // result unused: RED.MIN
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(kSetupThreads, 5) k_setup(DevScene S, const in
 }
 
 // Medium triangles: the grid's warps are shared out among them, each triangle's box
-// dealt 32 pixels at a time to its warps (at most one step each). One warp a triangle
+// dealt 32 pixels at a time to its warps in turn. One warp a triangle
 // left a box of 8,192 pixels to 256 dependent steps: 61 us for the ground's two triangles
 // in a 161 x 97 frame (now 6 us), 86 us for the medium triangles of a 4096^2 shadow map
 // of 2.05 million (now 67 us).
@@ -2000,7 +1999,7 @@ __global__ void __launch_bounds__(512) k_blur_spec(float* a, int W, int H, int L
     extern __shared__ float sm[];
     const float* w = c_blurW;
     const int L = VERT ? LV : Lrows;
-    constexpr int lgL = LV == 16 ? 4 : LV == 8 ? 3 : LV == 4 ? 2 : 0;
+    constexpr int lgL = LV == 8 ? 3 : LV == 4 ? 2 : 0;
     const int n = VERT ? H : W;
     const int lines = VERT ? W : H;
     const int first = blockIdx.x * L;
@@ -2397,7 +2396,7 @@ void launch_raster(const DevScene& S, const int4* scr, const RasterParams& rp, R
     int sms = 152;
     k_raster_medium<<<sms * 8, kMediumThreads, 0, st>>>(rp, rs, tiles);
     k_bin<<<sms * 4, 256, 0, st>>>(rp, rs);
-    if (tileRaster && shadowOut) 
+    if (tileRaster && shadowOut)
         k_tile_raster_shadow<<<blocks(tiles, kShadowTiles), 256, 0, st>>>(rp, rs, S, scr, shadowOut, tiles);
     else if (tileRaster) k_tile_raster<<<tiles, 256, 0, st>>>(rp, rs);
     launches += tileRaster ? 4 : 3;
@@ -2494,12 +2493,6 @@ void launch_ssao(const FrameConst& F, GBuffer gb, const float* table, float* bg1
     cfg.attrs = at, cfg.numAttrs = withBackground ? 1 : 0;
     const float* bg = bg16;
     cudaLaunchKernelEx(&cfg, k_ssao, F, gb, table, bg, gate);
-}
-
-void launch_ssao_background(const FrameConst& F, const float* depth, const float* table, float* bg16, cudaStream_t st)
-{
-    ssao_attributes();
-    k_ssao_background<<<1, 1024, sizeof(float) * 16 * F.ssaoN, st>>>(F, depth, table, bg16, nullptr);
 }
 
 size_t ao_input_smem(int K) { return K > 0 ? sizeof(float4) * 16 * (size_t)ssao_q_stride(K) : 0; }

@@ -39,7 +39,7 @@ enum StatusBits : int
 struct RasterParams
 {
     int W, H;              // raster target size
-    int smallArea;         // bbox area drawn by one thread
+    int smallArea;         // bbox area drawn by the triangle's setup warp
     int mediumArea;        // bbox area drawn by one or several warps (larger: tile bins)
 };
 
@@ -135,14 +135,11 @@ int launch_blur(int mode, int W, int H, float* ao, float* tmp, cudaStream_t st, 
 // the 1-in-64 plain-SSAO probe: one warp per probe pixel; the last block sets
 // *gate = 1 when the network's AO differs by more than `threshold` (mean squared).
 // part: 2 * ao_probe_blocks floats; done: a zeroed counter (left zeroed).
-// The 16 per-noise-cell SSAO values of background pixels (k_ssao_background), ungated.
-void launch_ssao_background(const frd::FrameConst& F, const float* depth, const float* table, float* bg16,
-                            cudaStream_t st);
 // inputTable / K: K-sample SSAO table for channel 3 (K = 0: the normal's z instead).
 void launch_ao_features(const frd::FrameConst& F, frd::GBuffer gb, uint4* out, cudaStream_t st,
                         const float* inputTable, int K);
 // With bg16 the same launch also writes the 16 background values of the frame's
-// SSAO (launch_ssao_background's, from frameTable).
+// SSAO (those of k_ssao_background, from frameTable).
 void launch_ao_features_blocks(const frd::FrameConst& F, frd::GBuffer gb, uint4* out, cudaStream_t st,
                                const float* inputTable, int K, const float* frameTable = nullptr,
                                float* bg16 = nullptr);

@@ -51,7 +51,6 @@ constexpr int kSegWords = kSeg / 32;
 constexpr int kWinWords = kSeg / 32 + 4;  // + the 128-pixel look-ahead of a packet
 constexpr int kParseThreads = 512;
 constexpr int kParseWarps = kParseThreads / 32;
-constexpr int kWalkThreads = 256;
 constexpr int kWriteThreads = 256;
 constexpr int kHeaderBytes = 18;
 constexpr int kTailBytes = 26;          // two 4-byte area references + 18-byte footer
