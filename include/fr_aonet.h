@@ -71,7 +71,8 @@ int fr_aonet_forward(fr_aonet* net, const uint16_t* in, int32_t B, int32_t H, in
 /* Mean squared error against `label` (device FP32 [B][H][W]; pixels whose label
  * is negative are left out of the loss, the mean still divides by B*H*W) and the gradient
  * of every parameter (readable with fr_aonet_get_grads). `loss` (host) may be
- * NULL; when given, the call waits for the stream. */
+ * NULL; when given, the call waits for the stream. Device memory is allocated by
+ * the first call, and again only by one with more pixels than any before it. */
 int fr_aonet_backward(fr_aonet* net, const uint16_t* in, const float* label, int32_t B, int32_t H, int32_t W,
                       float* loss, void* stream);
 int fr_aonet_get_grads(fr_aonet* net, float* dst, int64_t count);
