@@ -782,6 +782,18 @@ int fr_ssaa_pass(fr_ctx* ctx, const fr_frame_params* p)
 namespace
 {
 
+// Whether p is host memory, pinned or not (a device's or managed memory is not).
+bool host_memory(const void* p)
+{
+    cudaPointerAttributes pa{};
+    if (cudaPointerGetAttributes(&pa, p) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return false;
+    }
+    return pa.type == cudaMemoryTypeHost || pa.type == cudaMemoryTypeUnregistered;
+}
+
 // The launches of one frame on `st` (captured into the frame graph, or run directly).
 // Concurrent deferred frames fork the camera chain (geometry, SSAO, blur) onto the
 // context's high-priority second stream while the shadow pass runs on `st`: the
@@ -1034,7 +1046,7 @@ int64_t fr_download(fr_ctx* ctx, int32_t id, void* dst, size_t bytes)
             }
             frk::launch_pack_rgb(id == FR_BUF_FRAME_U8 ? ctx->frame8 : ctx->ssaa, ctx->rgbBuf, (int)n, st);
             const cudaError_t ce = cudaMemcpyAsync(dst, ctx->rgbBuf, need, cudaMemcpyDeviceToHost, st);
-            if (ce == cudaErrorInvalidValue)
+            if (ce == cudaErrorInvalidValue && host_memory(dst) && host_memory(static_cast<char*>(dst) + need - 1))
             {
                 // a destination pinned in part is none to CUDA's copies: by way of the heap
                 cudaGetLastError();

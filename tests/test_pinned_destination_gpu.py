@@ -93,3 +93,25 @@ def test_downloads_into_partly_pinned_memory(memory, what, tmp_path):
     if b is not None:
         b.close()
     r.close()
+
+
+def test_device_memory_as_destination():
+    """fr_download into device memory copies there, as CUDA's copies do."""
+    if not gpu_available():
+        pytest.skip("no CUDA GPU")
+    import torch
+
+    import forkerrenderer_gb300 as fr
+    from forkerrenderer_gb300 import _native as N
+    from scenes import render_config, scene_path
+
+    r = fr.Renderer(**render_config("def_pcss", shadow_size=64))
+    r.Preconfigure(fr.Scene(scene_path("def_pcss")))
+    r.Render()
+    want = r.frame8()
+    there = torch.zeros(want.size, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    assert N.lib().fr_download(r._h, N.FR_BUF_FRAME_U8, C.c_void_p(there.data_ptr()), want.size) == N.FR_OK
+    assert np.array_equal(there.cpu().numpy(), want.reshape(-1))
+    assert np.array_equal(r.frame8(), want)
+    r.close()
