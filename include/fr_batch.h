@@ -76,7 +76,9 @@ int fr_batch_render(fr_batch* batch);
 
 /* Device milliseconds of the last render: [transforms + setup + binning,
  * persistent fine raster, resolves + ambient occlusion, persistent lighting,
- * total]. Waits for the batch. */
+ * total]. Waits for the batch. Returns FR_ERR_BIN_OVERFLOW where a view's or a map's
+ * tile bins were full (fr_config.bin_capacity): such an image lacks triangles, and which
+ * ones differs from render to render. fr_batch_download does not look at this. */
 int fr_batch_timings(fr_batch* batch, float* ms, int32_t n);
 
 /* Sweeps light_tile {8,16,32} x bin_batch {64,256,1024} x ctas_per_sm {1,2,4},
